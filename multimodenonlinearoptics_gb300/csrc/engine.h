@@ -198,6 +198,7 @@ inline void add_prop_key(GraphKey& k, const PropArgs& a) {
   k.add(a.out).add(a.outStride).add(a.tw).add(a.dstep).add(a.dlast).add(a.half).add(a.back).add(a.prop);
   k.add(a.pump).add(a.pumpStride).add(a.nPumps).add(a.coef).add(a.nCoef).add(a.gridF).add(a.gridT);
   k.add(a.ckpt).add(a.ckK).add(a.ckN).add(a.stages).add(a.raman).add(a.steep).add(a.relInt);
+  k.add(a.fx.tw).add(a.fx.tab).add(a.fx.et).add(a.fx.raman).add(a.fx.steep).add(a.fx.etRaman).add(a.fx.etSteep).add(a.fx.A0).add(a.fx.sh).add(a.fx.ls);
 }
 
 struct GraphCache {
@@ -300,6 +301,58 @@ struct TwiddleCache {
   }
 };
 inline TwiddleCache g_twiddles;
+
+// A value as a Q62 integer relative to 2^et, in balanced halves (nlm_fx.cuh): exact for a double of
+// at most 2^et that is no smaller than 2^(et - 9), rounded to 2^(et - 62) below.
+inline int4 fx_quantise(long double re, long double im, int et) {
+  auto halves = [et](long double v, int& h, int& l) {
+    const long long q = std::llrint(std::ldexp(v, 62 - et));
+    l = (int)(uint32_t)(unsigned long long)q;
+    h = (int)((q - l) >> 32);
+  };
+  int4 r;
+  halves(re, r.x, r.y);
+  halves(im, r.z, r.w);
+  return r;
+}
+
+// The twiddles of the block fixed-point transforms, one table per plan, per process: for every pass after
+// the first (radix r, L the product of the earlier radices) exp(-2 pi i q k / (L r)) at (q - 1) L + k.
+struct FxTwiddleCache {
+  std::mutex mu;
+  std::map<std::vector<int>, std::shared_ptr<DevBuf<int4>>> tables;
+  const int4* get(const FFTPlanH& p, cudaStream_t s) {
+    std::lock_guard<std::mutex> lock(mu);
+    const std::vector<int> key(p.radix, p.radix + p.nPass);
+    auto it = tables.find(key);
+    if (it != tables.end()) return it->second->p;
+    std::vector<int4> h;
+    int L = 1;
+    for (int i = 0; i < p.nPass; i++) {
+      const int r = p.radix[i];
+      for (int q = 1; i > 0 && q < r; q++)
+        for (int k = 0; k < L; k++) {
+          const int m = q * k, n = L * r;   // exp(-2 pi i m / n), exact at the quarter points
+          if (4LL * m % n == 0) {
+            const int c[4] = {1, 0, -1, 0}, sn[4] = {0, -1, 0, 1}, t = (int)(4LL * m / n) % 4;
+            h.push_back(fx_quantise(c[t], sn[t], 0));
+          } else {
+            const long double ang = -2.0L * 3.141592653589793238462643383279502884L * (long double)m / (long double)n;
+            h.push_back(fx_quantise(std::cos(ang), std::sin(ang), 0));
+          }
+        }
+      L *= r;
+    }
+    h.resize(p.N);   // the kernels stage N entries
+    auto buf = std::make_shared<DevBuf<int4>>();
+    buf->alloc(h.size());
+    ck(cudaMemcpyAsync(buf->p, h.data(), h.size() * sizeof(int4), cudaMemcpyHostToDevice, s), "twiddle upload");
+    ck(cudaStreamSynchronize(s), "twiddle upload");
+    tables[key] = buf;
+    return buf->p;
+  }
+};
+inline FxTwiddleCache g_fxTwiddles;
 
 inline bool is_pow2(int n) { return n > 0 && (n & (n - 1)) == 0; }
 
@@ -630,6 +683,10 @@ struct Medium {
   DevBuf<double2> pumpFreq, pumpTime, sigFreq, sigTime;
   DevBuf<double2> dstep, dlast, half, back, coef, ramanD, steepD;
   DevBuf<double> relIntD, dispPumpD, dispSignD, omegaD;
+  // block fixed-point tables (dispStep, last, half) and their exponent; empty on grids without them
+  DevBuf<int4> fxTab, fxRaman, fxSteep;
+  int fxEtRaman = 0, fxEtSteep = 0;
+  int fxEt = 0;
   DevBuf<double> prop;
   long long propVersion = -1, propBuilds = 0;
   // arithmetic of the single-mode propagator path: 0 FP64, 1 double-float on the FP32 units
@@ -820,6 +877,13 @@ struct Medium {
     upload(dlast, hl);
     upload(half, hh);
     upload(back, hb);
+    // a single z step has an infinite step length, and tables that are not finite: FP64 kernels
+    if (fxSize() && nZ > 1 && std::isfinite(dz)) {
+      std::vector<double2> all(hd);
+      all.insert(all.end(), hl.begin(), hl.end());
+      all.insert(all.end(), hh.begin(), hh.end());
+      uploadFx(fxTab, &fxEt, all);
+    }
     std::vector<double> hdp, hds;
     for (auto& v : dispPump) hdp.insert(hdp.end(), v.begin(), v.end());
     for (auto& v : dispSign) hds.insert(hds.end(), v.begin(), v.end());
@@ -844,6 +908,24 @@ struct Medium {
     d.alloc(h.size() + kTablePad);
     ck(cudaMemcpyAsync(d.p, h.data(), h.size() * sizeof(double2), cudaMemcpyHostToDevice, stream), "upload");
     ck(cudaMemsetAsync(d.p + h.size(), 0, kTablePad * sizeof(double2), stream), "upload");
+  }
+  // A table for the block fixed-point transforms, relative to the smallest power of two (*et) that no modulus
+  // exceeds by more than its rounding; left empty when a value is not finite (or all are zero).
+  void uploadFx(DevBuf<int4>& d, int* et, const std::vector<double2>& h) {
+    double big = 0;
+    for (const double2& v : h) {
+      if (!std::isfinite(v.x) || !std::isfinite(v.y)) return;
+      big = std::max(big, std::hypot(v.x, v.y));
+    }
+    if (!(big > 0) || !std::isfinite(big)) return;
+    std::frexp(big * (1 - 1e-15), et);
+    std::vector<int4> q;
+    q.reserve(h.size() + kTablePad);
+    for (const double2& v : h) q.push_back(fx_quantise(v.x, v.y, *et));
+    q.resize(h.size() + kTablePad);
+    d.alloc(q.size());
+    ck(cudaMemcpyAsync(d.p, q.data(), q.size() * sizeof(int4), cudaMemcpyHostToDevice, stream), "upload");
+    ck(cudaStreamSynchronize(stream), "upload");   // q goes out of scope
   }
   void uploadD(DevBuf<double>& d, const std::vector<double>& h) {
     if (h.empty()) {
@@ -1040,6 +1122,10 @@ struct Medium {
     }
     upload(ramanD, rs);
     upload(steepD, st);
+    if (fxTab.p) {
+      uploadFx(fxRaman, &fxEtRaman, rs);
+      uploadFx(fxSteep, &fxEtSteep, st);
+    }
     std::vector<double> rel((size_t)(nZ > 1 ? nZ - 1 : 0) * 3);
     for (uint i = 1; i < nZ; i++) {
       rel[(i - 1) * 3 + 0] = relativeIntensity((double)(i - 1));
@@ -1371,11 +1457,12 @@ struct Medium {
   // override or the occupancy maximum), grid = SMs x CTAs per SM, capped by the number of groups.
   Schedule schedule(const KernelEntry* k, long long nInst, int R, int cta = 0, int ipcMul = 1) {
     const int T = ((int)N + R - 1) / R;   // N / R on the register plan, ceil(N / R) on the general one
-    int ipc = (T >= 128 ? 1 : 128 / T) * ipcMul;
+    const bool fx = k->kind == kKindFxLinear || k->kind == kKindFxDirect || k->kind == kKindFxGnlse;
+    int ipc = fx ? 1 : (T >= 128 ? 1 : 128 / T) * ipcMul;
     if (ipc > nInst) ipc = (int)std::max<long long>(1, nInst);
     const int block = T * ipc;
     // exchange buffers of the ipc propagations, plus the staged twiddle table when R != 16
-    const size_t smem = (size_t)(ipc + (k->R != 16 ? 1 : 0)) * N * sizeof(double2);
+    const size_t smem = fx ? fx_smem((int)N) : (size_t)(ipc + (k->R != 16 ? 1 : 0)) * N * sizeof(double2);
     int dev = 0, sms = 1, optin = 0;
     ck(cudaGetDevice(&dev), "device");
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -1472,11 +1559,12 @@ struct Medium {
         if (kc->kind != kind || kc->key != key) continue;
         const int R = kc->R;
         if (!is_pow2((int)N) || (int)N < R || N / R > 512 || N > (uint)kMaxFFT) continue;
+        if ((kind == kKindFxLinear || kind == kKindFxDirect) && N / R < 32) continue;
         // the four-points-per-thread variant of the single-mode propagator serves latency-bound launches
         // (fewer propagations than SMs), which are not tuned; for two modes it is a candidate (the
         // eight-point variant spills)
         if (kind == kKindLinear && key == 1 && R == 4) continue;
-        for (int ipcMul = 1; ipcMul <= 2; ipcMul++) {
+        for (int ipcMul = 1; ipcMul <= (kind == kKindFxLinear || kind == kKindFxDirect ? 1 : 2); ipcMul++) {
           Schedule base;
           try {
             base = schedule(kc, nInst, R, 0, ipcMul);
@@ -1488,6 +1576,7 @@ struct Medium {
             PropArgs ta = a0;
             ta.plan = make_plan((int)N, R);
             ta.R = R;
+            if (kind == kKindFxLinear || kind == kKindFxDirect) ta.fx = fxArgs(ta.plan);
             ta.nZ = std::min<int>(a0.nZ, 17);
             ta.nInst = nInst;
             ta.ipc = sc.ipc;
@@ -1548,6 +1637,49 @@ struct Medium {
     a.steep = steepD.p;
     a.relInt = relIntD.p;
     return a;
+  }
+
+  // ---- block fixed-point transforms (nlm_fx.cuh) ----------------------------------------------
+  // Grids whose one-CTA kernels run them: whole warps of 4 or 8 points per thread, at most 512 threads.
+  static constexpr uint kFxMinN = 128, kFxMaxN = 4096;
+  bool fxSize() const { return is_pow2((int)N) && N >= kFxMinN && N <= kFxMaxN; }
+  bool fxGrid() const { return fxSize() && fxTab.p && (solver != kChi3GNLSE || (fxRaman.p && fxSteep.p)); }
+  int log2N() const { return (int)std::lround(std::log2((double)N)); }
+
+  // The arguments for a plan: A0 such that the norm peaks below 2^62, the shifts of one transform in all, and the
+  // shift that brings the table product back to at most 2^A0.
+  FxArgs fxArgs(const FFTPlanH& p) const {
+    FxArgs f{};
+    f.tw = g_fxTwiddles.get(p, stream);
+    f.tab = fxTab.p;
+    f.et = fxEt;
+    f.raman = fxRaman.p;
+    f.steep = fxSteep.p;
+    f.etRaman = fxEtRaman;
+    f.etSteep = fxEtSteep;
+    int level = 0;   // half bits
+    for (int i = 0; i < p.nPass; i++) {
+      const int s = i == 0 ? 0 : fx_pass_shift(level, p.radix[i]);
+      f.sh += s;
+      level += fx_log2(p.radix[i]) - 2 * s;
+    }
+    f.A0 = 60;
+    f.ls = 2 - (level + 1) / 2;
+    return f;
+  }
+
+  const KernelEntry* fxKernel(int kind, int key, int* R) const {
+    // one mode takes eight points per thread where that leaves whole warps; several modes, whose fields all stay
+    // in registers, four where 512 threads hold the grid
+    for (int q : {0, 1}) {
+      const int r = (nSignal == 1) == (q == 0) ? 8 : 4;
+      if (N / r < 32 || N / r > 512) continue;
+      if (const KernelEntry* k = findKernel(kind, key, r)) {
+        *R = r;
+        return k;
+      }
+    }
+    return nullptr;
   }
 
   // The propagator's device buffer at its size, allocated ahead of a graph capture (which may not
@@ -1883,11 +2015,20 @@ struct Medium {
     } else if (gnlse) {
       checkGridStrict(R);
       k = findKernel(kKindGnlse, solver, R);
+      const bool fx = fxGrid() && !plainOne;
+      const int fxKey = solver + 1000 * log2N();
+      if (fx) {
+        int Rx = R;
+        k = fxKernel(kKindFxGnlse, fxKey, &Rx);
+        a.plan = make_plan((int)N, Rx);
+        a.R = Rx;
+        a.fx = fxArgs(a.plan);
+      }
       // more rows than SMs (one row per thread group would take a second wave): two rows per thread
       // group, sharing their Raman transforms (k_propagate_gnlse_pair: 14 transforms per row and step
       // instead of 18, so a pair takes 1.56 rows' time)
       if (!plainOne && nInst > smCount() && !a.gridF && !a.gridT) {
-        if (const KernelEntry* kp = findKernel(kKindGnlse, solver + 400, R)) {
+        if (const KernelEntry* kp = fx ? findKernel(kKindFxGnlse, fxKey + 400, a.R) : findKernel(kKindGnlse, solver + 400, R)) {
           k = kp;
           paired = true;
         }
@@ -1896,7 +2037,12 @@ struct Medium {
       checkGridStrict(R);
       buildPropagator(R);
       a.prop = prop.p;
-      if (wantFF(R, a)) {
+      int Rx = R;
+      if (!plainOne && !wantFF(R, a) && fxGrid() && (k = fxKernel(kKindFxLinear, (int)nSignal + 1000 * log2N(), &Rx))) {
+        a.plan = make_plan((int)N, Rx);
+        a.R = Rx;
+        a.fx = fxArgs(a.plan);
+      } else if (wantFF(R, a)) {
         ff = true;
         ffT = prepareFF();
         k = findKernel(kKindLinearFF, 1 + 10 * shortRadix(a.plan), R);
@@ -1913,6 +2059,10 @@ struct Medium {
           }
         }
       }
+    } else if (int Rx = R; !plainOne && fxGrid() && (k = fxKernel(kKindFxDirect, solver, &Rx))) {
+      a.plan = make_plan((int)N, Rx);
+      a.R = Rx;
+      a.fx = fxArgs(a.plan);
     } else {
       checkGridStrict(R);
       k = findKernel(kKindDirect, solver, R);
@@ -1936,6 +2086,7 @@ struct Medium {
         k = findKernelFn(c.fn);
         a.plan = make_plan((int)N, c.R);
         a.R = c.R;
+        if (k->kind == kKindFxLinear || k->kind == kKindFxDirect) a.fx = fxArgs(a.plan);
         s = schedule(k, nInst, c.R, c.cta, c.ipcMul);
         lastTuned = 1;
       }
@@ -1955,7 +2106,8 @@ struct Medium {
       const long long fullPairs = units / wave * wave;
       const long long rest = nInst - 2 * fullPairs;
       if (fullPairs > 0 && rest > 0 && units % wave != 0) {
-        if (const KernelEntry* k1 = findKernel(kKindGnlse, solver, a.R)) {
+        if (const KernelEntry* k1 = k->kind == kKindFxGnlse ? findKernel(kKindFxGnlse, k->key - 400, a.R)
+                                                            : findKernel(kKindGnlse, solver, a.R)) {
           const Schedule s1 = schedule(k1, rest, a.R, ctaPerSM < 0 ? 0 : ctaPerSM);
           if ((long long)s1.grid * s1.ipc >= rest) {   // the rest in one wave
             kTail = k1;

@@ -17,6 +17,11 @@ void add_kernels_adjoint(std::vector<KernelEntry>& t);
 void add_kernels_ragged(std::vector<KernelEntry>& t);
 void add_kernels_adjoint_gnlse(std::vector<KernelEntry>& t);
 void add_kernels_ff(std::vector<KernelEntry>& t);
+void add_kernels_fx(std::vector<KernelEntry>& t);
+void add_kernels_fx_direct_a(std::vector<KernelEntry>& t);
+void add_kernels_fx_direct_b(std::vector<KernelEntry>& t);
+void add_kernels_fx_direct_c(std::vector<KernelEntry>& t);
+void add_kernels_fx_gnlse(std::vector<KernelEntry>& t);
 void add_kernels_direct_c(std::vector<KernelEntry>& t);
 void add_kernels_cluster(std::vector<KernelEntry>& t);
 void add_kernels_cluster_b(std::vector<KernelEntry>& t);
@@ -48,6 +53,11 @@ const KernelEntry* kernel_table(int* count) {
     add_kernels_ragged(table);
     add_kernels_adjoint_gnlse(table);
     add_kernels_ff(table);
+    add_kernels_fx(table);
+    add_kernels_fx_direct_a(table);
+    add_kernels_fx_direct_b(table);
+    add_kernels_fx_direct_c(table);
+    add_kernels_fx_gnlse(table);
     add_kernels_direct_c(table);
     add_kernels_cluster(table);
     add_kernels_cluster_b(table);

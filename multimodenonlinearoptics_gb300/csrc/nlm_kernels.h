@@ -23,6 +23,34 @@ struct FFTPlanH {
   int R;   // points per thread the plan was made for
 };
 
+// Block fixed-point transforms (nlm_fx.cuh): the twiddles and dispersion tables as Q62 integers, each complex
+// value as balanced 32-bit halves {re high, re low, im high, im low} with value (h 2^32 + l) 2^(et - 62).
+struct FxArgs {
+  const int4* tw;    // N twiddles exp(-2 pi i m / N), et = 0
+  const int4* tab;   // [dispStep, last, half][mode][N], each with its 1/N
+  int et;            // exponent of the tables: 2^et is at least their largest modulus
+  const int4* raman; // Chi3GNLSE: Raman response and self-steepening factors (1/N folded in), their exponents
+  const int4* steep;
+  int etRaman, etSteep;
+  int A0;            // log2 bound of the field's 2-norm on entry
+  int sh;            // places a transform shifts right in all
+  int ls;            // places the table product after a forward transform is shifted left
+};
+
+// Places a pass of radix r shifts its values right, in a block fixed-point transform whose 2-norm stands `level`
+// half bits above its entry: the fewest that keep it within kFxPeak half bits after the pass (each pass grows the
+// norm by sqrt(r)).  The higher the norm stands, the less a rounding weighs.  Updates level.
+constexpr int kFxPeak = 4;
+__host__ __device__ constexpr int fx_log2(int r) { return r >= 16 ? 4 : r >= 8 ? 3 : r >= 4 ? 2 : r >= 2 ? 1 : 0; }
+__host__ __device__ constexpr int fx_pass_shift(int level, int r) {
+  return level + fx_log2(r) <= kFxPeak ? 0 : (level + fx_log2(r) - kFxPeak + 1) / 2;
+}
+
+// Shared memory of a CTA of the block fixed-point kernels: the twiddles, two exchange buffers of
+// fx_buffer(N) values and one pair of words per warp (at most 16).
+__host__ __device__ constexpr int fx_buffer(int N) { return N + N / 8; }
+constexpr size_t fx_smem(int N) { return (size_t)(N + 2 * fx_buffer(N)) * 16 + 16 * 8; }
+
 // Arguments of every propagation kernel (batched impulses, dense rows, one full grid).
 struct PropArgs {
   FFTPlanH plan;          // mirrors nlm::FFTPlan
@@ -72,6 +100,7 @@ struct PropArgs {
   const double2* raman;   // ramanResponse / N
   const double2* steep;   // (nlStep0 + nlStep1 * omega) / N
   const double* relInt;   // [(nZ-1)][3] relative intensity at i-1, i-1/2, i
+  FxArgs fx;              // block fixed-point transforms
 };
 
 // Arguments of the reverse (adjoint) sweep.
@@ -99,7 +128,10 @@ enum KernelKind : int {
   kKindRagged = 5,     // k_propagate_ragged<Solver, R>      key = solver id; args (items, nItems, work)
   kKindLinearFF = 6,   // k_propagate_linear_ff<R, SMALL>    key = M + 10 SMALL; args (PropArgs, FFTables)
   kKindCluster = 7,    // k_propagate_cluster<Solver, C>     key = solver id, R = C; cluster launch
-  kKindSpreadFused = 8 // k_propagate_spread<Solver, C, M>   key as kKindCluster (R = 1): modes transformed together
+  kKindSpreadFused = 8, // k_propagate_spread<Solver, C, M>  key as kKindCluster (R = 1): modes transformed together
+  kKindFxLinear = 9,   // k_fx_linear<M, R, N>               key = modes + 1000 log2 N; args (PropArgs)
+  kKindFxDirect = 10,  // k_fx_direct<Solver, R>             key = solver id; args (PropArgs)
+  kKindFxGnlse = 11    // k_fx_gnlse<R, N>                   key = solver id (+ 400: pairs) + 1000 log2 N; extra arg: scratch
 };
 
 // Float-float copies (float4 {re.hi, re.lo, im.hi, im.lo} per complex value) of the tables of a
