@@ -18,7 +18,7 @@ __global__ void __launch_bounds__(C == 16 ? 256 : kMaxThreads) k_adjoint_gnlse_s
   SpreadFFT f;
   const int rank = (int)cl.block_rank();
   const int M = a.plan.N;
-  spread_init<C>(f, smem, a.tw, M, rank);
+  spread_init<C>(f, smem, a.fx.twN, M, rank);
   const int N = M * C;
   const int tn = rank + C * f.t, fk = f.j + M * rank;
   const double2 ram = __ldg(a.raman + fk), stp = __ldg(a.steep + fk);

@@ -20,7 +20,7 @@ __global__ void __launch_bounds__(kMaxThreads) k_adjoint_pdc_spread(const PropAr
   SpreadFFT f;
   const int rank = (int)cl.block_rank();
   const int M = a.plan.N;
-  spread_init(f, smem, a.tw, M, rank);
+  spread_init(f, smem, a.fx.twN, M, rank);
   const int N = M * kSpreadC;
   const int tn = rank + kSpreadC * f.t, fk = f.j + M * rank;
   const int K = d.K;
@@ -81,7 +81,7 @@ __global__ void __launch_bounds__(kMaxThreads) k_adjoint_pdc_spread_pipe(const P
   const int role = crank / kSpreadC;   // 0: reverse sweep, 1: recomputation
   SpreadFFT f;
   const int M = a.plan.N;
-  spread_init(f, smem, a.tw, M, crank - role * kSpreadC);
+  spread_init(f, smem, a.fx.twN, M, crank - role * kSpreadC);
   f.base = role * kSpreadC;
   const int N = M * kSpreadC;
   const int tn = f.rank + kSpreadC * f.t, fk = f.j + M * f.rank;
@@ -182,7 +182,7 @@ __global__ void __launch_bounds__(kMaxThreads) k_adjoint_pdc_spread_stage(const 
   const int N = M * kSpreadC;
   SpreadFFT f;
   if (role < 2) {
-    spread_init(f, smem, a.tw, M, lr);
+    spread_init(f, smem, a.fx.twN, M, lr);
     f.base = role * kSpreadC;
   }
   const int tn = lr + kSpreadC * spread_time_index((int)threadIdx.x, M), fk = (int)threadIdx.x + M * lr;

@@ -198,7 +198,7 @@ inline void add_prop_key(GraphKey& k, const PropArgs& a) {
   k.add(a.out).add(a.outStride).add(a.tw).add(a.dstep).add(a.dlast).add(a.half).add(a.back).add(a.prop);
   k.add(a.pump).add(a.pumpStride).add(a.nPumps).add(a.coef).add(a.nCoef).add(a.gridF).add(a.gridT);
   k.add(a.ckpt).add(a.ckK).add(a.ckN).add(a.stages).add(a.raman).add(a.steep).add(a.relInt);
-  k.add(a.fx.tw).add(a.fx.tab).add(a.fx.et).add(a.fx.raman).add(a.fx.steep).add(a.fx.etRaman).add(a.fx.etSteep).add(a.fx.A0).add(a.fx.sh).add(a.fx.ls);
+  k.add(a.fx.tw).add(a.fx.twN).add(a.fx.tab).add(a.fx.et).add(a.fx.raman).add(a.fx.steep).add(a.fx.etRaman).add(a.fx.etSteep).add(a.fx.A0).add(a.fx.sh).add(a.fx.ls);
 }
 
 struct GraphCache {
@@ -321,29 +321,41 @@ inline int4 fx_quantise(long double re, long double im, int et) {
 struct FxTwiddleCache {
   std::mutex mu;
   std::map<std::vector<int>, std::shared_ptr<DevBuf<int4>>> tables;
+  // exp(-2 pi i m / n), exact at the quarter points
+  static int4 root(int m, int n) {
+    if (4LL * m % n == 0) {
+      const int c[4] = {1, 0, -1, 0}, sn[4] = {0, -1, 0, 1}, t = (int)(4LL * m / n) % 4;
+      return fx_quantise(c[t], sn[t], 0);
+    }
+    const long double ang = -2.0L * 3.141592653589793238462643383279502884L * (long double)m / (long double)n;
+    return fx_quantise(std::cos(ang), std::sin(ang), 0);
+  }
   const int4* get(const FFTPlanH& p, cudaStream_t s) {
+    return find(std::vector<int>(p.radix, p.radix + p.nPass), s, [&](std::vector<int4>& h) {
+      int L = 1;
+      for (int i = 0; i < p.nPass; i++) {
+        const int r = p.radix[i];
+        for (int q = 1; i > 0 && q < r; q++)
+          for (int k = 0; k < L; k++) h.push_back(root(q * k, L * r));
+        L *= r;
+      }
+      h.resize(p.N);   // the kernels stage N entries
+    });
+  }
+  // exp(-2 pi i m / N) for m < N
+  const int4* natural(int N, cudaStream_t s) {
+    return find({-N}, s, [N](std::vector<int4>& h) {
+      for (int m = 0; m < N; m++) h.push_back(root(m, N));
+    });
+  }
+
+ private:
+  const int4* find(const std::vector<int>& key, cudaStream_t s, const std::function<void(std::vector<int4>&)>& fill) {
     std::lock_guard<std::mutex> lock(mu);
-    const std::vector<int> key(p.radix, p.radix + p.nPass);
     auto it = tables.find(key);
     if (it != tables.end()) return it->second->p;
     std::vector<int4> h;
-    int L = 1;
-    for (int i = 0; i < p.nPass; i++) {
-      const int r = p.radix[i];
-      for (int q = 1; i > 0 && q < r; q++)
-        for (int k = 0; k < L; k++) {
-          const int m = q * k, n = L * r;   // exp(-2 pi i m / n), exact at the quarter points
-          if (4LL * m % n == 0) {
-            const int c[4] = {1, 0, -1, 0}, sn[4] = {0, -1, 0, 1}, t = (int)(4LL * m / n) % 4;
-            h.push_back(fx_quantise(c[t], sn[t], 0));
-          } else {
-            const long double ang = -2.0L * 3.141592653589793238462643383279502884L * (long double)m / (long double)n;
-            h.push_back(fx_quantise(std::cos(ang), std::sin(ang), 0));
-          }
-        }
-      L *= r;
-    }
-    h.resize(p.N);   // the kernels stage N entries
+    fill(h);
     auto buf = std::make_shared<DevBuf<int4>>();
     buf->alloc(h.size());
     ck(cudaMemcpyAsync(buf->p, h.data(), h.size() * sizeof(int4), cudaMemcpyHostToDevice, s), "twiddle upload");
@@ -685,6 +697,7 @@ struct Medium {
   DevBuf<double> relIntD, dispPumpD, dispSignD, omegaD;
   // block fixed-point tables (dispStep, last, half) and their exponent; empty on grids without them
   DevBuf<int4> fxTab, fxRaman, fxSteep;
+  const int4* spreadTwD = nullptr;
   int fxEtRaman = 0, fxEtSteep = 0;
   int fxEt = 0;
   DevBuf<double> prop;
@@ -877,6 +890,7 @@ struct Medium {
     upload(dlast, hl);
     upload(half, hh);
     upload(back, hb);
+    if (fxSize()) spreadTwD = g_fxTwiddles.natural((int)N, stream);
     // a single z step has an infinite step length, and tables that are not finite: FP64 kernels
     if (fxSize() && nZ > 1 && std::isfinite(dz)) {
       std::vector<double2> all(hd);
@@ -1302,7 +1316,7 @@ struct Medium {
     upload(dr, rel);
     if (spreadGrid() || wideGrid()) {
       // the march on four (up to 1024 points) or eight SMs with one point per thread (prop_spread.cu)
-      ck(launch_pump_chi3_spread(pumpFreq.p, pumpTime.p, de.p, dh.p, dd.p, db.p, dr.p, (int)nZP, (int)N, tw, stream),
+      ck(launch_pump_chi3_spread(pumpFreq.p, pumpTime.p, de.p, dh.p, dd.p, db.p, dr.p, (int)nZP, (int)N, spreadTw(), stream),
          "chi3 pump (spread)");
     } else if (useCluster && is_pow2((int)N) && N >= 1024) {
       // 1024..8192 points: the march on four SMs (prop_cluster_pump.cu), four points per thread
@@ -1333,7 +1347,7 @@ struct Medium {
   void flushPump() {
     if (!deferredPump.pending) return;
     const PumpMarchArgs p = deferredPumpArgs();
-    ck(launch_pump_chi3_spread(p.pf, p.pt, p.env, p.halfP, p.dstepP, p.backP, p.rel, p.nRows, (int)N, tw, stream),
+    ck(launch_pump_chi3_spread(p.pf, p.pt, p.env, p.halfP, p.dstepP, p.backP, p.rel, p.nRows, (int)N, spreadTw(), stream),
        "chi3 pump (spread)");
     deferredPump.pending = false;
     launches++;
@@ -1624,6 +1638,7 @@ struct Medium {
     a.nModes = (int)nSignal;
     a.nZ = (int)nZ;
     a.tw = tw;
+    a.fx.twN = spreadTw();
     a.dstep = dstep.p;
     a.dlast = dlast.p;
     a.half = half.p;
@@ -1644,6 +1659,8 @@ struct Medium {
   static constexpr uint kFxMinN = 128, kFxMaxN = 4096;
   bool fxSize() const { return is_pow2((int)N) && N >= kFxMinN && N <= kFxMaxN; }
   bool fxGrid() const { return fxSize() && fxTab.p && (solver != kChi3GNLSE || (fxRaman.p && fxSteep.p)); }
+  // the N-point twiddles of the one-point-per-thread cluster kernels (null on grids without them)
+  const int4* spreadTw() const { return spreadTwD; }
   int log2N() const { return (int)std::lround(std::log2((double)N)); }
 
   // The arguments for a plan: A0 such that the norm peaks below 2^62, the shifts of one transform in all, and the
@@ -1651,6 +1668,7 @@ struct Medium {
   FxArgs fxArgs(const FFTPlanH& p) const {
     FxArgs f{};
     f.tw = g_fxTwiddles.get(p, stream);
+    f.twN = spreadTw();
     f.tab = fxTab.p;
     f.et = fxEt;
     f.raman = fxRaman.p;

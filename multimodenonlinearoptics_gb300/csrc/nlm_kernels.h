@@ -26,7 +26,8 @@ struct FFTPlanH {
 // Block fixed-point transforms (nlm_fx.cuh): the twiddles and dispersion tables as Q62 integers, each complex
 // value as balanced 32-bit halves {re high, re low, im high, im low} with value (h 2^32 + l) 2^(et - 62).
 struct FxArgs {
-  const int4* tw;    // N twiddles exp(-2 pi i m / N), et = 0
+  const int4* tw;    // the plan's twiddles, pass by pass (one-CTA kernels)
+  const int4* twN;   // exp(-2 pi i m / N), m < N (cluster kernels with one point per thread)
   const int4* tab;   // [dispStep, last, half][mode][N], each with its 1/N
   int et;            // exponent of the tables: 2^et is at least their largest modulus
   const int4* raman; // Chi3GNLSE: Raman response and self-steepening factors (1/N folded in), their exponents
@@ -187,7 +188,7 @@ constexpr int kSpreadW16Key = 900;
 // two from 32 to 1024.
 cudaError_t launch_pump_chi3_spread(double2* pumpFreq, double2* pumpTime, const double2* env, const double2* halfP,
                                     const double2* dstepP, const double2* backP, const double2* rel, int nRows, int N,
-                                    const double2* tw, cudaStream_t s);
+                                    const int4* tw, cudaStream_t s);
 
 // The Chi3 pump march's grids and per-point tables (k_pump_chi3_spread's arguments).
 struct PumpMarchArgs {

@@ -35,7 +35,7 @@ __global__ void __launch_bounds__(kMaxThreads) k_chi3_pump_signal_spread(const P
   const int role = crank / kSpreadC;   // 0: pump march, 1: signal
   SpreadFFT f;
   const int M = a.plan.N;
-  spread_init(f, smem, a.tw, M, crank - role * kSpreadC);
+  spread_init(f, smem, a.fx.twN, M, crank - role * kSpreadC);
   f.base = role * kSpreadC;
   const int N = M * kSpreadC;
   const int tn = f.rank + kSpreadC * f.t, fk = f.j + M * f.rank;

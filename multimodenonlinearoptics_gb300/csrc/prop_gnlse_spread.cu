@@ -13,7 +13,7 @@
 
 namespace nlm {
 
-// a.plan.N = M (N / C threads per CTA); a.tw: the N-point table.  Sixteen CTAs take grids up to 4096
+// a.plan.N = M (N / C threads per CTA); a.fx.twN: the N-point table.  Sixteen CTAs take grids up to 4096
 // points (at most 256 threads per CTA, a bound that leaves the 16-point combine its registers).
 template <int C>
 __global__ void __launch_bounds__(C == 16 ? 256 : kMaxThreads) k_propagate_gnlse_spread(const PropArgs a) {
@@ -22,7 +22,7 @@ __global__ void __launch_bounds__(C == 16 ? 256 : kMaxThreads) k_propagate_gnlse
   SpreadFFT f;
   const int rank = (int)cl.block_rank();
   const int M = a.plan.N;
-  spread_init<C>(f, smem, a.tw, M, rank);
+  spread_init<C>(f, smem, a.fx.twN, M, rank);
   const int N = M * C;
   const int tn = rank + C * f.t;   // time-domain point of this thread
   const int fk = f.j + M * rank;   // frequency bin of this thread

@@ -11,7 +11,7 @@ namespace nlm {
 
 cudaError_t launch_pump_chi3_spread(double2* pumpFreq, double2* pumpTime, const double2* env, const double2* halfP,
                                     const double2* dstepP, const double2* backP, const double2* rel, int nRows, int N,
-                                    const double2* tw, cudaStream_t s) {
+                                    const int4* tw, cudaStream_t s) {
   // four CTAs up to 1024 points, eight above (M = N / C threads per CTA)
   const int C = N <= 1024 ? 4 : 8;
   int M = N / C;

@@ -9,7 +9,7 @@
 
 namespace nlm {
 
-// tw: the N-point table; M = N / C threads per CTA.
+// tw: the N-point Q62 table; M = N / C threads per CTA.
 template <int C>
 __global__ void __launch_bounds__(kMaxThreads) k_pump_chi3_spread(double2* __restrict__ pf, double2* __restrict__ pt,
                                                                   const double2* __restrict__ env,
@@ -17,7 +17,7 @@ __global__ void __launch_bounds__(kMaxThreads) k_pump_chi3_spread(double2* __res
                                                                   const double2* __restrict__ dstepP,
                                                                   const double2* __restrict__ backP,
                                                                   const double2* __restrict__ rel, int nRows, int M,
-                                                                  const double2* __restrict__ tw) {
+                                                                  const int4* __restrict__ tw) {
   extern __shared__ double2 smem[];
   cg::cluster_group cl = cg::this_cluster();
   SpreadFFT f;
@@ -71,7 +71,7 @@ __device__ __forceinline__ void spread_inv_all(SpreadFFT& f, double2 (&x)[MD], c
   }
 }
 
-// One propagation per cluster (clusters take instances in turn); a.plan.N = M, a.tw the N-point table.
+// One propagation per cluster (clusters take instances in turn); a.plan.N = M, a.fx.twN the N-point table.
 // Point-wise work: the pump-driven solvers' RK4 matrices (a.prop) or the solver's DiffEq.  K = 1: the
 // modes' transforms one after another; K = the solver's mode count: all modes in each transform
 // together (spread_fwd_k, spread_inv_store_k: one barrier per stage and one cluster barrier per
@@ -86,7 +86,7 @@ __global__ void __launch_bounds__(kMaxThreads) k_propagate_spread(const PropArgs
   SpreadFFT f;
   const int rank = (int)cl.block_rank();
   const int M = a.plan.N;
-  spread_init<C, K>(f, smem, a.tw, M, rank);
+  spread_init<C, K>(f, smem, a.fx.twN, M, rank);
   const int N = M * C;
   const int tn = rank + C * f.t;
   const int fk = f.j + M * rank;
