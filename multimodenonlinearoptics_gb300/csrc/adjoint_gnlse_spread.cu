@@ -9,7 +9,7 @@
 
 namespace nlm {
 
-// a.plan.N = M (N / C threads per CTA); a.tw: the N-point table.  Sixteen CTAs: grids up to 4096 points.
+// a.plan.N = M (N / C threads per CTA); a.fx.twN: the N-point table.  Sixteen CTAs: grids up to 4096 points.
 template <int C>
 __global__ void __launch_bounds__(C == 16 ? 256 : kMaxThreads) k_adjoint_gnlse_stored_spread(const PropArgs a,
                                                                                              const AdjArgs d) {
@@ -18,10 +18,12 @@ __global__ void __launch_bounds__(C == 16 ? 256 : kMaxThreads) k_adjoint_gnlse_s
   SpreadFFT f;
   const int rank = (int)cl.block_rank();
   const int M = a.plan.N;
-  spread_init<C>(f, smem, a.fx.twN, M, rank);
+  spread_init<C>(f, smem, a.fx.twN, M, rank, a.fx.err);
+  cl.sync();
   const int N = M * C;
   const int tn = rank + C * f.t, fk = f.j + M * rank;
-  const double2 ram = __ldg(a.raman + fk), stp = __ldg(a.steep + fk);
+  const int4 ram = fx_conj(__ldg(a.fx.raman + fk));
+  const double2 stp = __ldg(a.steep + fk);
   const double2 dst = __ldg(a.dstep + fk), dla = __ldg(a.dlast + fk);
   const long long clusterId = blockIdx.x / C, nClusters = gridDim.x / C;
   for (long long local = clusterId; local < a.nInst; local += nClusters) {
@@ -44,20 +46,21 @@ __global__ void __launch_bounds__(C == 16 ? 256 : kMaxThreads) k_adjoint_gnlse_s
         const double ri = __ldg(rel + (s == 0 ? 0 : (s == 3 ? 2 : 1)));
         const double2 y = Yi[(long long)s * N + tn], u2 = Yi[(long long)(4 + s) * N + tn];
         // g_k_s (spectrum); the fourth stage's has no later stage's part
-        double2 u = s < 3 ? caxpy(spread_fwd<C>(f, gke, cl), w, h) : cscale(h, w);
-        u = spread_inv<C>(f, cmulc(u, stp), cl);                        // g_u3
+        double2 u = s < 3 ? caxpy(spread_fwd<C>(f, gke), w, h) : cscale(h, w);
+        u = spread_inv<C>(f, cmulc(u, stp));                            // g_u3
         double2 gy = cmulc(u, u2);                                    // conj(u2) g_u3
         u = cmulc(u, y);                                              // g_u2 = conj(y) g_u3
-        u = spread_inv<C>(f, cmulc(spread_fwd<C>(f, u, cl), ram), cl);   // g_u1 (real part)
+        u = spread_pair<C>(f, u, ram, a.fx.etRaman);                  // g_u1 (real part)
         gy = caxpy(gy, 2.0 * ri * u.x, y);
         gx = cadd(gx, gy);
         gke = cscale(gy, fac);
       }
-      g = cadd(spread_fwd<C>(f, gx, cl), h);
+      g = cadd(spread_fwd<C>(f, gx), h);
     }
     // g: the gradient of the input spectrum, times half a dispersion step
     d.gin[inst * (long long)N + fk] = cmulc(g, __ldg(a.half + fk));
   }
+  cl.sync();
 }
 
 void add_kernels_adjoint_gnlse_spread(std::vector<KernelEntry>& t) {

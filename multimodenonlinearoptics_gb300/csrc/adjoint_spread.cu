@@ -13,14 +13,22 @@
 
 namespace nlm {
 
-// a.plan.N = M (N / 4 threads per CTA); a.tw: the N-point table.  d.seg: [cluster][K][N] when d.K > 1.
+// The transpose of step i's dispersion: forward transform, conjugate factors, inverse transform; the last step's
+// gradient starts in the frequency domain.
+__device__ __forceinline__ double2 spread_adjoint_dispersion(const PropArgs& a, SpreadFFT& f, double2 g, int i, int fk) {
+  if (i < a.nZ - 1) return spread_pair(f, g, fx_conj(__ldg(a.fx.tab + fk)), a.fx.et);
+  return spread_inv(f, cmulc(g, __ldg(a.dlast + fk)));
+}
+
+// a.plan.N = M (N / 4 threads per CTA); a.fx.twN: the N-point table.  d.seg: [cluster][K][N] when d.K > 1.
 __global__ void __launch_bounds__(kMaxThreads) k_adjoint_pdc_spread(const PropArgs a, const AdjArgs d) {
   extern __shared__ double2 smem[];
   cg::cluster_group cl = cg::this_cluster();
   SpreadFFT f;
   const int rank = (int)cl.block_rank();
   const int M = a.plan.N;
-  spread_init(f, smem, a.fx.twN, M, rank);
+  spread_init(f, smem, a.fx.twN, M, rank, a.fx.err);
+  cl.sync();
   const int N = M * kSpreadC;
   const int tn = rank + kSpreadC * f.t, fk = f.j + M * rank;
   const int K = d.K;
@@ -40,15 +48,13 @@ __global__ void __launch_bounds__(kMaxThreads) k_adjoint_pdc_spread(const PropAr
         seg[tn] = x;
         for (int i = s0 + 1; i < segEnd; i++) {
           x = pdc_step_point(a, N, i, tn, x);
-          x = spread_inv(f, cmul(spread_fwd(f, x, cl), __ldg(a.dstep + fk)), cl);
+          x = spread_pair(f, x, __ldg(a.fx.tab + fk), a.fx.et);
           seg[(long long)(i - s0) * N + tn] = x;
         }
         states = seg;
       }
       for (int i = segEnd; i > s0; i--) {
-        if (i < a.nZ - 1) g = spread_fwd(f, g, cl);
-        const double2* tab = (i == a.nZ - 1) ? a.dlast : a.dstep;
-        g = spread_inv(f, cmulc(g, __ldg(tab + fk)), cl);
+        g = spread_adjoint_dispersion(a, f, g, i, fk);
         if (d.gp) {   // marching form: P^T per point, the stage-factor gradients afterwards in parallel
           g = pdc_march_point(a, d, N, i, tn, inst, g, true);
           continue;
@@ -60,20 +66,17 @@ __global__ void __launch_bounds__(kMaxThreads) k_adjoint_pdc_spread(const PropAr
       segEnd = s0;
     }
     // gradient of the input spectrum: s_0 = IFFT(half X_in)
-    g = spread_fwd(f, g, cl);
+    g = spread_fwd(f, g);
     d.gin[inst * (long long)N + fk] = cmulc(g, __ldg(a.half + fk));
   }
+  cl.sync();
 }
 
 // Pipelined form for checkpoint intervals K > 1 on clusters of eight CTAs (two groups of four, as in
 // k_adjoint_pdc_cluster_pipe): ranks 4..7 recompute the states of segment j-1 from its checkpoint into
-// one half of STG while ranks 0..3 reverse segment j from the other half.  Every spread transform ends
-// with one barrier of the whole cluster, so per segment iteration both groups run exactly K step slots
-// of 2 transforms (a recomputed step: the forward and inverse transform of the dispersion step; a
-// reverse step: the same pair, with a bare barrier in place of the forward transform for the last step,
-// whose gradient starts in the frequency domain) and then one barrier; a slot without a step passes 2
-// bare barriers.  The final forward transform of the input gradient is matched by one bare barrier in
-// the recomputing group.  d.seg: [cluster][2][K][N].
+// one half of STG while ranks 0..3 reverse segment j from the other half.  The groups' transforms only
+// wait for their own four CTAs; one barrier of the whole cluster ends each segment iteration and hands the
+// halves over.  d.seg: [cluster][2][K][N].
 __global__ void __launch_bounds__(kMaxThreads) k_adjoint_pdc_spread_pipe(const PropArgs a, const AdjArgs d) {
   extern __shared__ double2 smem[];
   cg::cluster_group cl = cg::this_cluster();
@@ -81,8 +84,9 @@ __global__ void __launch_bounds__(kMaxThreads) k_adjoint_pdc_spread_pipe(const P
   const int role = crank / kSpreadC;   // 0: reverse sweep, 1: recomputation
   SpreadFFT f;
   const int M = a.plan.N;
-  spread_init(f, smem, a.fx.twN, M, crank - role * kSpreadC);
+  spread_init(f, smem, a.fx.twN, M, crank - role * kSpreadC, a.fx.err);
   f.base = role * kSpreadC;
+  cl.sync();
   const int N = M * kSpreadC;
   const int tn = f.rank + kSpreadC * f.t, fk = f.j + M * f.rank;
   const int K = d.K;
@@ -106,14 +110,10 @@ __global__ void __launch_bounds__(kMaxThreads) k_adjoint_pdc_spread_pipe(const P
             const int i = s0 + q;
             if (i < segEnd) {
               x = pdc_step_point(a, N, i, tn, x);
-              x = spread_inv(f, cmul(spread_fwd(f, x, cl), __ldg(a.dstep + fk)), cl);
+              x = spread_pair(f, x, __ldg(a.fx.tab + fk), a.fx.et);
               stg[(long long)q * N + tn] = x;
-            } else {
-              spread_idle(cl, 2);
             }
           }
-        } else {
-          spread_idle(cl, 2 * K);
         }
       } else {
         if (it >= 1) {
@@ -123,29 +123,21 @@ __global__ void __launch_bounds__(kMaxThreads) k_adjoint_pdc_spread_pipe(const P
             const int i = segEnd - q;
             if (i > s0) {
               const double2* prev = stg + (long long)(i - 1 - s0) * N;
-              if (i < a.nZ - 1) g = spread_fwd(f, g, cl);
-              else cl.sync();
-              const double2* tab = (i == a.nZ - 1) ? a.dlast : a.dstep;
-              g = spread_inv(f, cmulc(g, __ldg(tab + fk)), cl);
+              g = spread_adjoint_dispersion(a, f, g, i, fk);
               const double2* c = a.coef + (long long)(i - 1) * 3 * a.nCoef;
               g = pdc_reverse_point(a, d, N, i, tn, c[0], c[1], c[2], prev[tn], g, true);
-            } else {
-              spread_idle(cl, 2);
             }
           }
-        } else {
-          spread_idle(cl, 2 * K);
         }
       }
       cl.sync();
     }
     if (role == 0) {
-      g = spread_fwd(f, g, cl);
+      g = spread_fwd(f, g);
       d.gin[inst * (long long)N + fk] = cmulc(g, __ldg(a.half + fk));
-    } else {
-      cl.sync();
     }
   }
+  cl.sync();
 }
 
 // Stage-factor gradient groups beside the pipelined sweep, on clusters of 4 (2 + G) CTAs, for
@@ -157,18 +149,11 @@ __global__ void __launch_bounds__(kMaxThreads) k_adjoint_pdc_spread_pipe(const P
 //     the gradient after each step's RK4 in GP;
 //   ranks 8.. (groups 2 .. 1 + G) compute the stage-factor gradients of segment j+1, reversed in the
 //     previous iteration, from its states (STG) and stored gradients (GP).  Group 2 + s takes the steps
-//     q = s mod G of the segment (q = 0 .. K-1): the loads and forward stages of step q in slot q, its
-//     transposed stages and stores in slot q + 1 (or after the last slot), both before the slot's
-//     first barrier.  That interval holds two local transforms in groups 0 and 1 (the inverse of the
-//     previous slot, the forward of this one); the one between the slot's two barriers holds only the
-//     cluster exchange.
-// Per slot a point costs about 76 FP64 instructions in groups 0 and 1 and 90 / G in each stage group;
-// the FP64 issue rate of an SM is fixed per scheduler, so G = 2 (sixteen CTAs) keeps the stage groups
-// off the critical path and G = 1 (twelve) is the form for GPUs without 16-CTA clusters.  STG holds
-// three segments (written by group 1 at iteration it, read by group 0 at it+1 and by the stage groups
-// at it+2) and GP two.  After the last iteration all groups share the stage-factor gradients of
-// segment 0, by steps.  Barriers per row: (nSeg + 1) (2K + 1) in the iterations, then one (the input
-// gradient's transform in group 0) and one after the shared work, in every group.
+//     q = s mod G of the segment (q = 0 .. K-1).
+// G = 2 (sixteen CTAs) halves the stage groups' work; G = 1 (twelve) is the form for GPUs without 16-CTA
+// clusters.  STG holds three segments (written by group 1 at iteration it, read by group 0 at it+1 and by the
+// stage groups at it+2) and GP two; one barrier of the whole cluster ends each iteration.  After the last
+// iteration all groups share the stage-factor gradients of segment 0, by steps.
 // d.seg: [cluster][3 + 2][K][N].
 template <int G>
 __global__ void __launch_bounds__(kMaxThreads) k_adjoint_pdc_spread_stage(const PropArgs a, const AdjArgs d) {
@@ -182,9 +167,10 @@ __global__ void __launch_bounds__(kMaxThreads) k_adjoint_pdc_spread_stage(const 
   const int N = M * kSpreadC;
   SpreadFFT f;
   if (role < 2) {
-    spread_init(f, smem, a.fx.twN, M, lr);
+    spread_init(f, smem, a.fx.twN, M, lr, a.fx.err);
     f.base = role * kSpreadC;
   }
+  cl.sync();
   const int tn = lr + kSpreadC * spread_time_index((int)threadIdx.x, M), fk = (int)threadIdx.x + M * lr;
   const int pc = lr * M + (int)threadIdx.x;   // the point of this thread's stage-factor gradients
   const int K = d.K;
@@ -227,14 +213,10 @@ __global__ void __launch_bounds__(kMaxThreads) k_adjoint_pdc_spread_stage(const 
             const int i = s0 + q;
             if (i < segEnd) {
               x = pdc_step_point(a, N, i, tn, x);
-              x = spread_inv(f, cmul(spread_fwd(f, x, cl), __ldg(a.dstep + fk)), cl);
+              x = spread_pair(f, x, __ldg(a.fx.tab + fk), a.fx.et);
               stg[(long long)q * N + tn] = x;
-            } else {
-              spread_idle(cl, 2);
             }
           }
-        } else {
-          spread_idle(cl, 2 * K);
         }
       } else if (role == 0) {
         if (it >= 1) {
@@ -243,18 +225,11 @@ __global__ void __launch_bounds__(kMaxThreads) k_adjoint_pdc_spread_stage(const 
           for (int q = 0; q < K; q++) {
             const int i = segEnd - q;
             if (i > s0) {
-              if (i < a.nZ - 1) g = spread_fwd(f, g, cl);
-              else cl.sync();
-              const double2* tab = (i == a.nZ - 1) ? a.dlast : a.dstep;
-              g = spread_inv(f, cmulc(g, __ldg(tab + fk)), cl);
+              g = spread_adjoint_dispersion(a, f, g, i, fk);
               gps[(long long)(i - 1 - s0) * N + tn] = g;
               g = pdc_transpose_point(a, N, i, tn, g);
-            } else {
-              spread_idle(cl, 2);
             }
           }
-        } else {
-          spread_idle(cl, 2 * K);
         }
       } else {
         if (it >= 2) {
@@ -266,20 +241,15 @@ __global__ void __launch_bounds__(kMaxThreads) k_adjoint_pdc_spread_stage(const 
             stageFinish();   // the step loaded in an earlier slot
             const int i = s0 + 1 + q;
             if (q % G == sub && i <= segEnd) stageLoad(stg, gps, i, s0);
-            spread_idle(cl, 2);
           }
           stageFinish();
-        } else {
-          spread_idle(cl, 2 * K);
         }
       }
       cl.sync();
     }
     if (role == 0) {
-      g = spread_fwd(f, g, cl);
+      g = spread_fwd(f, g);
       d.gin[inst * (long long)N + fk] = cmulc(g, __ldg(a.half + fk));
-    } else {
-      cl.sync();
     }
     // segment 0 (reversed in the last iteration): its steps shared by all groups
     {

@@ -366,6 +366,28 @@ struct FxTwiddleCache {
 };
 inline FxTwiddleCache g_fxTwiddles;
 
+// Host memory that a cluster kernel raises when an exchange between its CTAs does not arrive in time (nlm_spread.cuh);
+// read after every wait for a stream.
+struct ExchangeFlag {
+  std::mutex mu;
+  int* p = nullptr;
+  int* flag() {
+    std::lock_guard<std::mutex> lock(mu);
+    if (!p) {
+      ck(cudaHostAlloc((void**)&p, sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped), "exchange flag");
+      *p = 0;
+    }
+    return p;
+  }
+  void check() {
+    if (p && *(volatile int*)p) {
+      *(volatile int*)p = 0;
+      throw std::runtime_error("an exchange between the CTAs of a cluster did not arrive; the results are not valid");
+    }
+  }
+};
+inline ExchangeFlag g_exchange;
+
 inline bool is_pow2(int n) { return n > 0 && (n & (n - 1)) == 0; }
 
 // The general plan (FFTPlanH::gen == 1) of an N-point transform with R points per thread: T = ceil(N/R)
@@ -699,6 +721,7 @@ struct Medium {
   DevBuf<int4> fxTab, fxRaman, fxSteep;
   const int4* spreadTwD = nullptr;
   int fxEtRaman = 0, fxEtSteep = 0;
+  bool fxBad = false;   // a table has values that are not finite: only the FP64 kernels take this medium
   int fxEt = 0;
   DevBuf<double> prop;
   long long propVersion = -1, propBuilds = 0;
@@ -750,6 +773,12 @@ struct Medium {
     if (ev0) cudaEventDestroy(ev0);
     if (ev1) cudaEventDestroy(ev1);
     if (ownStream && stream) cudaStreamDestroy(stream);
+  }
+
+  // Waits for the medium's stream.
+  void sync(const char* what) {
+    ck(cudaStreamSynchronize(stream), what);
+    g_exchange.check();
   }
 
   // -- set-up, src/_NonlinearMedium.cpp:43-102 -------------------------------------------
@@ -897,6 +926,7 @@ struct Medium {
       all.insert(all.end(), hl.begin(), hl.end());
       all.insert(all.end(), hh.begin(), hh.end());
       uploadFx(fxTab, &fxEt, all);
+      fxBad = !fxTab.p;
     }
     std::vector<double> hdp, hds;
     for (auto& v : dispPump) hdp.insert(hdp.end(), v.begin(), v.end());
@@ -906,7 +936,7 @@ struct Medium {
     uploadD(omegaD, omega);
     buildCoefficients();
     if (solver == kChi3GNLSE) buildGnlse();
-    ck(cudaStreamSynchronize(stream), "device set-up");
+    sync("device set-up");
     devReady = true;
   }
 
@@ -939,7 +969,7 @@ struct Medium {
     q.resize(h.size() + kTablePad);
     d.alloc(q.size());
     ck(cudaMemcpyAsync(d.p, q.data(), q.size() * sizeof(int4), cudaMemcpyHostToDevice, stream), "upload");
-    ck(cudaStreamSynchronize(stream), "upload");   // q goes out of scope
+    sync("upload");   // q goes out of scope
   }
   void uploadD(DevBuf<double>& d, const std::vector<double>& h) {
     if (h.empty()) {
@@ -1124,7 +1154,7 @@ struct Medium {
     launches++;
     std::vector<double2> hr(N);
     ck(cudaMemcpyAsync(hr.data(), work.p, N * sizeof(double2), cudaMemcpyDeviceToHost, stream), "raman");
-    ck(cudaStreamSynchronize(stream), "raman");
+    sync("raman");
     raman.resize(N);
     std::vector<double2> rs(N), st(N);
     const double invN = 1.0 / N;
@@ -1139,6 +1169,7 @@ struct Medium {
     if (fxTab.p) {
       uploadFx(fxRaman, &fxEtRaman, rs);
       uploadFx(fxSteep, &fxEtSteep, st);
+      fxBad = !fxRaman.p || !fxSteep.p;
     }
     std::vector<double> rel((size_t)(nZ > 1 ? nZ - 1 : 0) * 3);
     for (uint i = 1; i < nZ; i++) {
@@ -1179,7 +1210,7 @@ struct Medium {
     ck(launch_fft_rows(spec.p, de.p, 1, plan, tw, true, 1.0 / N, nullptr, stream), "chirp ifft");
     launches += 2;
     ck(cudaMemcpyAsync(e.data(), de.p, N * sizeof(double2), cudaMemcpyDeviceToHost, stream), "chirp");
-    ck(cudaStreamSynchronize(stream), "chirp");
+    sync("chirp");
     for (uint k = 0; k < N; k++) envelope[idx][k] = cplx(e[k].x, e[k].y);
   }
 
@@ -1258,9 +1289,9 @@ struct Medium {
           ck(launch_scale_rows(pf, sd.p, (int)nZP, (int)N, stream), "pump profile");
           ck(launch_scale_rows(pt, sd.p, (int)nZP, (int)N, stream), "pump profile");
           launches += 2;
-          ck(cudaStreamSynchronize(stream), "pump");
+          sync("pump");
         }
-        ck(cudaStreamSynchronize(stream), "pump");
+        sync("pump");
       }
     }
     pumpVersion++;
@@ -1304,7 +1335,7 @@ struct Medium {
       upload(q.dstep, dP);
       upload(q.back, bP);
       upload(q.rel, rel);
-      ck(cudaStreamSynchronize(stream), "chi3 pump tables");
+      sync("chi3 pump tables");
       q.pending = true;
       return;
     }
@@ -1316,7 +1347,7 @@ struct Medium {
     upload(dr, rel);
     if (spreadGrid() || wideGrid()) {
       // the march on four (up to 1024 points) or eight SMs with one point per thread (prop_spread.cu)
-      ck(launch_pump_chi3_spread(pumpFreq.p, pumpTime.p, de.p, dh.p, dd.p, db.p, dr.p, (int)nZP, (int)N, spreadTw(), stream),
+      ck(launch_pump_chi3_spread(pumpFreq.p, pumpTime.p, de.p, dh.p, dd.p, db.p, dr.p, (int)nZP, (int)N, spreadTw(), g_exchange.flag(), stream),
          "chi3 pump (spread)");
     } else if (useCluster && is_pow2((int)N) && N >= 1024) {
       // 1024..8192 points: the march on four SMs (prop_cluster_pump.cu), four points per thread
@@ -1328,7 +1359,7 @@ struct Medium {
          "chi3 pump");
     }
     launches++;
-    ck(cudaStreamSynchronize(stream), "chi3 pump");
+    sync("chi3 pump");
   }
 
   // The Chi3 pump march runs beside the next signal propagation: cluster mode 1, 128..1024 points (the
@@ -1347,11 +1378,11 @@ struct Medium {
   void flushPump() {
     if (!deferredPump.pending) return;
     const PumpMarchArgs p = deferredPumpArgs();
-    ck(launch_pump_chi3_spread(p.pf, p.pt, p.env, p.halfP, p.dstepP, p.backP, p.rel, p.nRows, (int)N, spreadTw(), stream),
+    ck(launch_pump_chi3_spread(p.pf, p.pt, p.env, p.halfP, p.dstepP, p.backP, p.rel, p.nRows, (int)N, spreadTw(), g_exchange.flag(), stream),
        "chi3 pump (spread)");
     deferredPump.pending = false;
     launches++;
-    ck(cudaStreamSynchronize(stream), "chi3 pump");
+    sync("chi3 pump");
   }
 
   // src/_NonlinearMedium.cpp:506-534
@@ -1380,7 +1411,7 @@ struct Medium {
     // last time-domain row as it was (src/_NonlinearMedium.cpp:533)
     if (nZP > 1) ck(launch_fft_rows(pf, pt, nZP - 1, plan, tw, true, 1.0 / N, nullptr, stream), "pump from ifft");
     launches += 2;
-    ck(cudaStreamSynchronize(stream), "pump from");
+    sync("pump from");
     pumpVersion++;
   }
 
@@ -1639,6 +1670,13 @@ struct Medium {
     a.nZ = (int)nZ;
     a.tw = tw;
     a.fx.twN = spreadTw();
+    a.fx.tab = fxTab.p;
+    a.fx.et = fxEt;
+    a.fx.raman = fxRaman.p;
+    a.fx.steep = fxSteep.p;
+    a.fx.etRaman = fxEtRaman;
+    a.fx.etSteep = fxEtSteep;
+    a.fx.err = g_exchange.flag();
     a.dstep = dstep.p;
     a.dlast = dlast.p;
     a.half = half.p;
@@ -1675,6 +1713,7 @@ struct Medium {
     f.steep = fxSteep.p;
     f.etRaman = fxEtRaman;
     f.etSteep = fxEtSteep;
+    f.err = g_exchange.flag();
     int level = 0;   // half bits
     for (int i = 0; i < p.nPass; i++) {
       const int s = i == 0 ? 0 : fx_pass_shift(level, p.radix[i]);
@@ -1746,13 +1785,13 @@ struct Medium {
   // cluster mode 3 is mode 1 without the widest forms (sixteen CTAs on 2048 and 4096 points, eight on
   // 1024): four CTAs up to 1024 points and eight above, as a reference for them
   bool spreadGrid() const {
-    return (useCluster == 1 || useCluster == 3) && is_pow2((int)N) && N >= kSpreadMinN && N <= kSpreadMaxN;
+    return (useCluster == 1 || useCluster == 3) && !fxBad && is_pow2((int)N) && N >= kSpreadMinN && N <= kSpreadMaxN;
   }
   // 2048- and 4096-point grids: one point per thread on eight CTAs (prop_spread_b.cu), twice the SMs of
   // the four-points-per-thread cluster, for the launches that no reverse sweep pairs with (full grids,
   // the media of ragged batches marked by raggedWide) and the Chi3 pump march.
   bool wideGrid() const {
-    return (useCluster == 1 || useCluster == 3) && is_pow2((int)N) && N > kSpreadMaxN && N <= kWideMaxN;
+    return (useCluster == 1 || useCluster == 3) && !fxBad && is_pow2((int)N) && N > kSpreadMaxN && N <= kWideMaxN;
   }
   bool wideLaunch(const PropArgs& a) const {
     return wideGrid() && !a.ckpt && !a.stages && (a.gridF || a.gridT || raggedWide || raggedW16);
@@ -1813,7 +1852,7 @@ struct Medium {
   // least 128 threads per CTA (at most 256 on sixteen CTAs, 512 otherwise); 0 when none applies (then
   // four points per thread on four CTAs).  The stored-stage reverse sweep takes the same form.
   int gnlseSpreadC(long long rows) const {
-    if (solver != kChi3GNLSE || useCluster != 1 || !is_pow2((int)N)) return 0;
+    if (solver != kChi3GNLSE || useCluster != 1 || fxBad || !is_pow2((int)N)) return 0;
     for (int C : {16, 8, 4}) {
       const int M = (int)N / C;
       if (M < 128 || M > (C == 16 ? 256 : 512) || rows * C > smCount()) continue;
@@ -1830,6 +1869,7 @@ struct Medium {
     // checkpointed forwards (the adjoint's, Chi2PDC and Chi3GNLSE) run on clusters too: their reverse
     // sweeps have cluster forms that read the same checkpoints
     if (!useCluster || plainOne || a.inKind != 1) return nullptr;
+    if (fxBad) return nullptr;
     if (!is_pow2((int)N) || N > (uint)kMaxFFT) return nullptr;
     if (const int Cs = gnlseSpreadC(nInst))
       return Cs == 16 ? findKernel(kKindCluster, solver + kSpreadW16Key, 1)
@@ -2223,7 +2263,7 @@ struct Medium {
     poling.assign(d, d + n);
     if (devReady) {
       buildCoefficients();
-      ck(cudaStreamSynchronize(stream), "coefficients");
+      sync("coefficients");
     }
     propVersion = -1;
   }
@@ -2256,7 +2296,7 @@ struct Medium {
       a.outStride = (long long)N;
       a.stages = adjStages.p;
       propagate(a, (long long)rows, false);
-      ck(cudaStreamSynchronize(stream), "adjoint forward");
+      sync("adjoint forward");
       adjStored = true;
       adjRows = (long long)rows;
       adjK = 0;
@@ -2293,7 +2333,7 @@ struct Medium {
     a.ckK = K;
     a.ckN = nCk;
     propagate(a, (long long)rows, true);
-    ck(cudaStreamSynchronize(stream), "adjoint forward");
+    sync("adjoint forward");
     adjRows = (long long)rows;
     adjK = K;
     adjNCk = nCk;
@@ -2303,7 +2343,7 @@ struct Medium {
   // Stage values of every Chi3GNLSE step fit (at most a quarter of the free device memory and 64 GB),
   // and the forward of `rows` propagations runs on 4-CTA clusters (Medium::clusterKernel).
   bool storeStages(size_t rows) const {
-    if (solver != kChi3GNLSE || !useCluster || !is_pow2((int)N) || N < 1024 || N > (uint)kMaxFFT) return false;
+    if (solver != kChi3GNLSE || !useCluster || fxBad || !is_pow2((int)N) || N < 1024 || N > (uint)kMaxFFT) return false;
     if ((long long)rows * kClusterSize > smCount()) return false;
     if (!findKernel(kKindCluster, solver, kClusterSize) || !findKernel(kKindAdjoint, solver + 300, kClusterSize))
       return false;
@@ -2348,7 +2388,7 @@ struct Medium {
       lastRegs = fa.numRegs;
       ck(launch_clustered(k->fn, (int)(Cs * clusters), M, smem, stream, Cs, args), "adjoint (stored stages)");
       launches++;
-      ck(cudaStreamSynchronize(stream), "adjoint");
+      sync("adjoint");
       return;
     }
     constexpr int C = kClusterSize;
@@ -2377,7 +2417,7 @@ struct Medium {
     lastRegs = fa.numRegs;
     ck(launch_clustered(k->fn, (int)(C * clusters), a.plan.T, smem, stream, C, args), "adjoint (stored stages)");
     launches++;
-    ck(cudaStreamSynchronize(stream), "adjoint");
+    sync("adjoint");
   }
 
   // Chi3GNLSE on grids of 1024 to 8192 points with few rows: the pipelined sweep on clusters of eight
@@ -2385,7 +2425,7 @@ struct Medium {
   // such clusters fit on the device at once, or a grid outside its range).
   bool adjointCluster(const double2* gout, double2* gin) {
     constexpr int C = kClusterSize;
-    if (solver != kChi3GNLSE || !useCluster || !is_pow2((int)N) || N < 1024 || N > (uint)kMaxFFT) return false;
+    if (solver != kChi3GNLSE || !useCluster || fxBad || !is_pow2((int)N) || N < 1024 || N > (uint)kMaxFFT) return false;
     const KernelEntry* k = findKernel(kKindAdjoint, solver + 200, C);
     if (!k) return false;
     const int M = (int)N / C;
@@ -2422,7 +2462,7 @@ struct Medium {
     ck(launch_clustered(k->fn, (int)(2 * C * clusters), a.plan.T, smem, stream, 2 * C, args),
        "adjoint (cluster of eight)");
     launches++;
-    ck(cudaStreamSynchronize(stream), "adjoint");
+    sync("adjoint");
     return true;
   }
 
@@ -2712,7 +2752,7 @@ struct Medium {
       launches++;
       std::vector<double2> gc(steps * 3);
       ck(cudaMemcpyAsync(gc.data(), adjGc.p, gc.size() * sizeof(double2), cudaMemcpyDeviceToHost, stream), "gc");
-      ck(cudaStreamSynchronize(stream), "adjoint");
+      sync("adjoint");
       // c_s = pol_s q_s with q_s = nlStep * mismatch(z_s): dL/dpol_s = Re(g_c conj(q_s)),
       // pol_0 = d[i-1], pol_1 = (d[i-1] + d[i]) / 2, pol_2 = d[i]  (solvers/Chi2PDC.cpp:32-34)
       for (uint i = 0; i < nZ; i++) gpol[i] = 0;
@@ -2728,7 +2768,7 @@ struct Medium {
         gpol[i] += 0.5 * gs[1] + gs[2];
       }
     }
-    ck(cudaStreamSynchronize(stream), "adjoint");
+    sync("adjoint");
   }
 
   // ---- public operations ---------------------------------------------------------------------
@@ -2754,7 +2794,7 @@ struct Medium {
     a.gridT = sigTime.p;
     if (pipe) launchPumpSignal(a);
     else propagate(a, 1, true);
-    ck(cudaStreamSynchronize(stream), "signal simulation");
+    sync("signal simulation");
     signalVersion++;
   }
 
@@ -2889,7 +2929,7 @@ struct Medium {
       ck(cudaMemcpyAsync(Cdst, C, mat * sizeof(double2), cudaMemcpyDeviceToHost, stream), "C download");
       ck(cudaMemcpyAsync(Sdst, S, mat * sizeof(double2), cudaMemcpyDeviceToHost, stream), "S download");
     }
-    ck(cudaStreamSynchronize(stream), "green");
+    sync("green");
   }
 
   // Raw outputs of impulse propagations [first, first + count) of the Green's function over all modes
@@ -2920,7 +2960,7 @@ struct Medium {
     if (count > 0 && !device)
       ck(cudaMemcpyAsync(rawOut, raw.p, (size_t)count * outStride * sizeof(double2), cudaMemcpyDeviceToHost, stream),
          "rows download");
-    ck(cudaStreamSynchronize(stream), "green rows");
+    sync("green rows");
   }
 
   // C and S from the raw rows of all 2 N nSignal impulse propagations (the epilogue of green()).
@@ -2959,7 +2999,7 @@ struct Medium {
       ck(cudaMemcpyAsync(Cdst, cs.p, mat * sizeof(double2), cudaMemcpyDeviceToHost, stream), "C download");
       ck(cudaMemcpyAsync(Sdst, cs.p + mat, mat * sizeof(double2), cudaMemcpyDeviceToHost, stream), "S download");
     }
-    ck(cudaStreamSynchronize(stream), "green finish");
+    sync("green finish");
   }
 
   void greenDims(unsigned nThreads, const uint8_t* useIn, size_t nUseIn, const uint8_t* useOut, size_t nUseOut,
@@ -3021,7 +3061,7 @@ struct Medium {
     propagate(a, (long long)rows, true);
     if (!device)
       ck(cudaMemcpyAsync(out, dout, rows * nOut * N * sizeof(double2), cudaMemcpyDeviceToHost, stream), "batch download");
-    ck(cudaStreamSynchronize(stream), "batch");
+    sync("batch");
   }
 
   // ---- getters ------------------------------------------------------------------------------
@@ -3053,7 +3093,7 @@ struct Medium {
         ck(cudaMemcpyAsync(h.data(), dev->p + (size_t)idx * nrows * N, len * sizeof(double), cudaMemcpyDeviceToHost,
                            stream),
            "grid download");
-        ck(cudaStreamSynchronize(stream), "grid download");
+        sync("grid download");
       }
       (*vers)[idx] = ver;
     }

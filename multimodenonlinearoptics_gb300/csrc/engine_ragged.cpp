@@ -551,6 +551,7 @@ nlm_status nlm_ragged_batch(nlm_medium* const* media, size_t n_media, const doub
     ck(cudaEventRecord(g_ragged.t1, origin), "ragged timing");
     g_ragged.lastKey = key.bytes;
     ck(cudaStreamSynchronize(origin), "ragged batch");
+    g_exchange.check();
     float gpuMs = 0;
     ck(cudaEventElapsedTime(&gpuMs, g_ragged.t0, g_ragged.t1), "ragged timing");
     // host-side state of what ran: the matrices built; one launch per propagation, build and ragged

@@ -35,6 +35,7 @@ struct FxArgs {
   int etRaman, etSteep;
   int A0;            // log2 bound of the field's 2-norm on entry
   int sh;            // places a transform shifts right in all
+  int* err;          // host memory: raised when an exchange between the CTAs of a cluster does not arrive
   int ls;            // places the table product after a forward transform is shifted left
 };
 
@@ -188,7 +189,7 @@ constexpr int kSpreadW16Key = 900;
 // two from 32 to 1024.
 cudaError_t launch_pump_chi3_spread(double2* pumpFreq, double2* pumpTime, const double2* env, const double2* halfP,
                                     const double2* dstepP, const double2* backP, const double2* rel, int nRows, int N,
-                                    const int4* tw, cudaStream_t s);
+                                    const int4* tw, int* err, cudaStream_t s);
 
 // The Chi3 pump march's grids and per-point tables (k_pump_chi3_spread's arguments).
 struct PumpMarchArgs {

@@ -12,8 +12,7 @@
 //           then a G-point DFT across the warps through shared memory (one barrier: each thread reads its
 //           lane's G values and forms its own output); then the twiddle exp(-2 pi i c j / N) and the C-point
 //           DFT over the CTAs: every thread pushes its value to all C CTAs through distributed shared
-//           memory, one cluster barrier, and each thread combines the C values of its own column for
-//           its CTA's output row;
+//           memory, and each thread combines the C values of its own column for its CTA's output row;
 // inverse:  the C-point inverse DFT over the CTAs first, the conjugate twiddle, then the local inverse
 //           (the G-point DFT across warps, the conjugate W_M^(g l), the 32-point DFT in the warps;
 //           unscaled, 1/N is in the tables).  It runs the forward transform's parts on values with real and
@@ -26,10 +25,15 @@
 // that code along with its values through each exchange; the receivers shift the values to the exponent of
 // the total.  Starting below 2^59, the norm grows by sqrt(32) in the warps, sqrt(G) across them and sqrt(C)
 // across the CTAs, and is shifted back where it would pass 2^61.5 (spread_shift).
+// Exchanges over the cluster: each value travels by st.async, which counts its bytes on the receiving warp's
+// mbarrier, and a warp waits for the C x 32 values of its own columns.  No barrier of the cluster and no fence
+// of earlier global stores: with cluster barriers those were a third of a step.  Two mbarriers per warp and two
+// halves of the receive buffer serve the exchanges in turn: a thread writes half n again only after it has
+// received exchange n + 1 from the thread that reads that column, which pushed it after reading half n.
+// Waits give up after kSpreadWait polls and raise *err; every CTA then still runs to the closing cluster barrier.
 // Shared memory: M twiddles, two M-point exchange buffers (alternating: a thread writes a buffer only after
-// the barrier that every reader of that buffer's previous contents has passed), and two halves of C x M
-// cluster receive buffers (alternating per transform: a CTA writes a half only after the cluster barrier that
-// its readers passed after their last read of it); the exponent codes lie beside each.
+// the barrier that every reader of that buffer's previous contents has passed), the two halves of C x M values;
+// the exponent codes lie beside each.
 // M is a power of two of at least 32, N = C M at most 4096.
 #pragma once
 #include <cooperative_groups.h>
@@ -47,6 +51,7 @@ constexpr int kSpreadA0 = 59;      // log2 bound of a warp's 2-norm on entry
 constexpr int kSpreadPeak = 5;     // half bits the norm may stand above it
 constexpr int kSpreadZero = -(1 << 20), kSpreadBad = 1 << 20;   // codes of a zero warp, of one with Inf or NaN
 constexpr int kSpreadMaxCodes = 4096 / 32 * 4;                  // warps of a cluster times fields
+constexpr int kSpreadWait = 1 << 16;                            // polls of an exchange before it gives up
 
 struct SpreadFFT {
   const int4* twM;      // [M] exp(-2 pi i m / M) in Q62, shared memory
@@ -57,18 +62,27 @@ struct SpreadFFT {
   int4* recv;           // [2][C][K][M] cluster receive buffers
   int* code;            // [2][K][G] exponent codes of the exchange buffers
   int* rcode;           // [2][C][K][G] and of the receive buffers
+  unsigned bar;         // shared address of this warp's two mbarriers
+  unsigned parity;      // bit p: the phase that mbarrier p completes next
+  int* err;             // raised (host memory) when an exchange does not arrive
+  bool dead;            // an exchange has timed out: no more waiting
   int M, rank, j;
   int l, g, t;          // lane, warp and local time index g + (M / 32) l of this thread
   int sel, phase;       // next exchange buffer / receive half
   int base;             // cluster rank of the group's first CTA (clusters holding two groups of four)
 };
 
+__device__ __forceinline__ unsigned spread_saddr(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
+
 // Sets up the spread transform of this CTA: the M-point twiddles (every C-th entry of the N-point Q62
-// table `tw`) and this thread's factors.  Ends with a CTA barrier.  K: fields transformed
-// together (spread_fwd_k, spread_inv_store_k), which sizes the exchange and receive buffers.
+// table `tw`), this thread's factors and the warps' mbarriers.  The cluster must pass a barrier (cl.sync) after
+// it and before the first exchange, and one after the last.  K: fields transformed
+// together (the _k forms), which sizes the exchange and receive buffers.
 template <int C = kSpreadC, int K = 1>
-__device__ __forceinline__ void spread_init(SpreadFFT& f, double2* smem, const int4* __restrict__ tw, int M, int rank) {
+__device__ __forceinline__ void spread_init(SpreadFFT& f, double2* smem, const int4* __restrict__ tw, int M, int rank,
+                                            int* err) {
   __shared__ int s_code[2 * 4 * 16], s_rcode[2 * kSpreadMaxCodes];
+  __shared__ unsigned long long s_bar[2 * 16];
   f.M = M;
   f.rank = rank;
   f.j = threadIdx.x;
@@ -80,12 +94,20 @@ __device__ __forceinline__ void spread_init(SpreadFFT& f, double2* smem, const i
   f.base = 0;
   f.code = s_code;
   f.rcode = s_rcode;
+  f.bar = spread_saddr(s_bar + 2 * f.g);
+  f.parity = 0;
+  f.err = err;
+  f.dead = false;
   int4* twM = reinterpret_cast<int4*>(smem);
   f.buf = twM + M;
   f.recv = twM + (1 + 2 * K) * M;
   for (int k = threadIdx.x; k < M; k += blockDim.x) twM[k] = tw[(long long)k * C];
   f.twM = twM;
   f.twC = tw[(long long)rank * f.j];
+  if (f.l < 2) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(f.bar + 8 * f.l) : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
   __syncthreads();
   // decimation in frequency: the upper lane of a pair takes W_2s^(l mod s), the lower one 1
   auto lane = [&](int s) { return twM[(f.l & s) ? (f.l & (s - 1)) * (M / (2 * s)) : 0]; };
@@ -93,6 +115,24 @@ __device__ __forceinline__ void spread_init(SpreadFFT& f, double2* smem, const i
   f.w8 = lane(8);
   f.w4 = lane(4);
   f.wgl = twM[f.g * f.l];
+}
+
+// Waits for the exchange in flight (half f.phase) of this warp.
+__device__ __forceinline__ void spread_wait(SpreadFFT& f) {
+  const unsigned bar = f.bar + 8 * f.phase, par = (f.parity >> f.phase) & 1;
+  f.parity ^= 1u << f.phase;
+  if (f.dead) return;
+  for (int n = 0; n < kSpreadWait; n++) {
+    unsigned ok;
+    asm volatile(
+        "{\n.reg .pred p;\nmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}"
+        : "=r"(ok)
+        : "r"(bar), "r"(par)
+        : "memory");
+    if (ok) return;
+  }
+  f.dead = true;
+  if (f.err) *(volatile int*)f.err = 1;
 }
 
 // Local time index of thread j of a CTA of M threads (the time ownership above).
@@ -220,74 +260,109 @@ __device__ __forceinline__ void spread_warp_dft(const SpreadFFT& f, fxc (&x)[K])
   for (int m = 0; m < K; m++) x[m] = spread_shfl(x[m], src);
 }
 
-// G-point DFT across the warps of a CTA for every lane; h: the warp's codes in, the CTA's out.
-template <int G, int K>
+// G-point DFT across the warps of a CTA for every lane; CODES: the warps' exponents differ (h: the warp's codes
+// in, the CTA's out), else they are the cluster's.
+template <int G, bool CODES, int K>
 __device__ __forceinline__ void spread_cross_g(SpreadFFT& f, fxc (&x)[K], int (&h)[K]) {
   int4* b = f.buf + f.sel * K * f.M;
   int* cd = f.code + f.sel * K * G;
 #pragma unroll
   for (int m = 0; m < K; m++) {
     b[m * f.M + f.j] = fx_pack(x[m]);
-    if (f.l == 0) cd[m * G + f.g] = h[m];
+    if (CODES && f.l == 0) cd[m * G + f.g] = h[m];
   }
   __syncthreads();
 #pragma unroll
   for (int m = 0; m < K; m++) {
     int hs[G], r[G];
     fxc v[G];
+    if constexpr (CODES) {
 #pragma unroll
-    for (int c = 0; c < G; c++) hs[c] = cd[m * G + c];
-    h[m] = spread_total<G>(hs, r);
+      for (int c = 0; c < G; c++) hs[c] = cd[m * G + c];
+      h[m] = spread_total<G>(hs, r);
+    }
 #pragma unroll
-    for (int c = 0; c < G; c++) v[c] = spread_align(fx_unpack(b[m * f.M + c * 32 + f.l]), r[c]);
+    for (int c = 0; c < G; c++) {
+      v[c] = fx_unpack(b[m * f.M + c * 32 + f.l]);
+      if constexpr (CODES) v[c] = spread_align(v[c], r[c]);
+    }
     x[m] = spread_combine<G>(v, f.g, f.twM, f.M);
   }
   f.sel ^= 1;
 }
 
-template <int K>
+template <bool CODES, int K>
 __device__ __forceinline__ void spread_cross(SpreadFFT& f, fxc (&x)[K], int (&h)[K]) {
   switch (f.M >> 5) {
-    case 2: spread_cross_g<2>(f, x, h); break;
-    case 4: spread_cross_g<4>(f, x, h); break;
-    case 8: spread_cross_g<8>(f, x, h); break;
-    case 16: spread_cross_g<16>(f, x, h); break;
+    case 2: spread_cross_g<2, CODES>(f, x, h); break;
+    case 4: spread_cross_g<4, CODES>(f, x, h); break;
+    case 8: spread_cross_g<8, CODES>(f, x, h); break;
+    case 16: spread_cross_g<16, CODES>(f, x, h); break;
     default: break;   // one warp
   }
 }
 
-// C-point DFT over the cluster's CTAs: thread j of every CTA pushes its value to column j of row `rank` in all
-// C CTAs (and lane v of each warp its code to CTA v); after the barrier thread j of CTA r forms output r.
-template <int C, int K>
-__device__ __forceinline__ void spread_exchange(SpreadFFT& f, fxc (&y)[K], int (&h)[K], cg::cluster_group& cl) {
+// The push of an exchange: thread j of every CTA sends its value to column j of row `rank` in all C CTAs (and,
+// with CODES, lane v of each warp its code to CTA v).
+template <int C, bool CODES, int K>
+__device__ __forceinline__ void spread_push(SpreadFFT& f, const fxc (&y)[K], const int (&h)[K]) {
   static_assert(C == 4 || C == 8 || C == 16, "four, eight or sixteen CTAs");
   const int M = f.M, G = M >> 5;
-  int4* half = f.recv + (long long)f.phase * C * K * M;
-  int* cd = f.rcode + f.phase * C * K * G;
+  const unsigned bar = f.bar + 8 * f.phase;
+  const unsigned dst = spread_saddr(f.recv + ((long long)f.phase * C + f.rank) * K * M + f.j);
+  if (f.l == 0)
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar),
+                 "r"(C * K * (32 * 16 + (CODES ? 4 : 0)))
+                 : "memory");
   int4 out[K];
 #pragma unroll
   for (int m = 0; m < K; m++) out[m] = fx_pack(y[m]);
 #pragma unroll
   for (int v = 0; v < C; v++) {
-    int4* dst = cl.map_shared_rank(half + (long long)f.rank * K * M + f.j, f.base + v);
+    unsigned rd, rb;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(rd) : "r"(dst), "r"(f.base + v));
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(rb) : "r"(bar), "r"(f.base + v));
 #pragma unroll
-    for (int m = 0; m < K; m++) dst[m * M] = out[m];
+    for (int m = 0; m < K; m++)
+      asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(
+                       rd + 16 * m * M),
+                   "r"(out[m].x), "r"(out[m].y), "r"(out[m].z), "r"(out[m].w), "r"(rb)
+                   : "memory");
   }
-  if (f.l < C) {
-    int* dst = cl.map_shared_rank(cd + f.rank * K * G + f.g, f.base + f.l);
+  if (CODES && f.l < C) {
+    const unsigned cd = spread_saddr(f.rcode + (f.phase * C + f.rank) * K * G + f.g);
+    unsigned rd, rb;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(rd) : "r"(cd), "r"(f.base + f.l));
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(rb) : "r"(bar), "r"(f.base + f.l));
 #pragma unroll
-    for (int m = 0; m < K; m++) dst[m * G] = h[m];
+    for (int m = 0; m < K; m++)
+      asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(rd + 4 * m * G),
+                   "r"(h[m]), "r"(rb)
+                   : "memory");
   }
-  cl.sync();
+}
+
+// The other half: the C values of this thread's column, combined into output `rank` of their C-point DFT.
+template <int C, bool CODES, int K>
+__device__ __forceinline__ void spread_pull(SpreadFFT& f, fxc (&y)[K], int (&h)[K]) {
+  const int M = f.M, G = M >> 5;
+  const int4* half = f.recv + (long long)f.phase * C * K * M;
+  const int* cd = f.rcode + f.phase * C * K * G;
+  spread_wait(f);
 #pragma unroll
   for (int m = 0; m < K; m++) {
     int hs[C], r[C];
     fxc v[C];
+    if constexpr (CODES) {
 #pragma unroll
-    for (int c = 0; c < C; c++) hs[c] = cd[(c * K + m) * G + f.g];
-    h[m] = spread_total<C>(hs, r);
+      for (int c = 0; c < C; c++) hs[c] = cd[(c * K + m) * G + f.g];
+      h[m] = spread_total<C>(hs, r);
+    }
 #pragma unroll
-    for (int c = 0; c < C; c++) v[c] = spread_align(fx_unpack(half[((long long)c * K + m) * M + f.j]), r[c]);
+    for (int c = 0; c < C; c++) {
+      v[c] = fx_unpack(half[((long long)c * K + m) * M + f.j]);
+      if constexpr (CODES) v[c] = spread_align(v[c], r[c]);
+    }
     y[m] = spread_combine<C>(v, f.rank, f.twM, M);
   }
   f.phase ^= 1;
@@ -296,80 +371,141 @@ __device__ __forceinline__ void spread_exchange(SpreadFFT& f, fxc (&y)[K], int (
 // a w / 2^s
 __device__ __forceinline__ fxc spread_mul(fxc a, int4 w, int s) { return fx_cmul(a, w, 2 - s); }
 
-// time-domain ownership -> frequency-domain ownership, K fields together: one barrier and one cluster barrier for
-// all of them
+// time-domain ownership -> frequency-domain ownership, K fields together.  Returns in `places` the shifts so far:
+// y = X 2^(A0 - ceil(h / 2) - places), h the cluster's code, the norm at most `level` half bits above 2^A0.
 template <int C, int K>
-__device__ __forceinline__ void spread_fwd_k(SpreadFFT& f, double2 (&x)[K], cg::cluster_group& cl) {
-  const int g = 26 - __clz(f.M);   // log2 G, the half bits a G-point DFT adds (M = 32 G)
-  const int s1 = spread_shift(5, g), s2 = spread_shift(5 + g - 2 * s1, fx_log2(C));
-  fxc y[K];
-  int h[K];
+__device__ __forceinline__ void spread_forward(SpreadFFT& f, const double2 (&x)[K], fxc (&y)[K], int (&h)[K], int& places,
+                                               int& level) {
+  const int g = 26 - __clz(f.M), lc = fx_log2(C);   // log2 G: the half bits a G-point DFT adds (M = 32 G)
+  const int s1 = spread_shift(5, g), s2 = spread_shift(5 + g - 2 * s1, lc);
 #pragma unroll
   for (int m = 0; m < K; m++) h[m] = spread_enter(x[m], y[m]);
   spread_warp_dft<K>(f, y);
 #pragma unroll
   for (int m = 0; m < K; m++) y[m] = f.g > 0 ? spread_mul(y[m], f.wgl, s1) : fx_shift(y[m], s1);
-  spread_cross<K>(f, y, h);
+  spread_cross<true, K>(f, y, h);
 #pragma unroll
   for (int m = 0; m < K; m++) y[m] = spread_mul(y[m], f.twC, s2);
-  spread_exchange<C, K>(f, y, h, cl);
+  spread_push<C, true, K>(f, y, h);
+  spread_pull<C, true, K>(f, y, h);
+  places = s1 + s2;
+  level = 5 + g - 2 * s1 + lc - 2 * s2;
+}
+
+// The inverse transform's part after its push (of swapped values): pull, DFT across the warps, in the warps.
+// CODES: the warps' codes travel with the values; otherwise h is the cluster's.  level: of the pushed values.
+template <int C, bool CODES, int K>
+__device__ __forceinline__ void spread_backward(SpreadFFT& f, fxc (&y)[K], int (&h)[K], int& places, int level) {
+  const int g = 26 - __clz(f.M), lc = fx_log2(C);
+  // the last product shifts two places at most: the one before it takes what that leaves
+  const int s1 = max(0, (level + lc + g - 3) >> 1), s2 = spread_shift(level + lc + g - 2 * s1, 5);
+  spread_pull<C, CODES, K>(f, y, h);
 #pragma unroll
-  for (int m = 0; m < K; m++) x[m] = spread_leave(y[m], h[m], s1 + s2);
+  for (int m = 0; m < K; m++) y[m] = spread_mul(y[m], f.twC, s1);
+  spread_cross<CODES, K>(f, y, h);
+#pragma unroll
+  for (int m = 0; m < K; m++) y[m] = f.g > 0 ? spread_mul(y[m], f.wgl, s2) : fx_shift(y[m], s2);
+  spread_warp_dft<K>(f, y);
+  places += s1 + s2;
+}
+
+template <int C, int K>
+__device__ __forceinline__ void spread_fwd_k(SpreadFFT& f, double2 (&x)[K]) {
+  fxc y[K];
+  int h[K], places, level;
+  spread_forward<C, K>(f, x, y, h, places, level);
+#pragma unroll
+  for (int m = 0; m < K; m++) x[m] = spread_leave(y[m], h[m], places);
 }
 
 // frequency-domain ownership -> time-domain ownership (unscaled), K fields.  store(m, v) receives each field's
-// frequency-domain value right after the exchange's cluster barrier (the barrier's release fence then does not
-// wait for the store, which drains during the local transform).
+// frequency-domain value while the exchange is in flight.
 template <int C, int K, class Store>
-__device__ __forceinline__ void spread_inv_store_k(SpreadFFT& f, double2 (&x)[K], cg::cluster_group& cl, Store store) {
-  const int g = 26 - __clz(f.M), lc = fx_log2(C);
-  // the second product shifts two places at most: the first takes what that leaves
-  const int s1 = max(0, (lc + g - 3) >> 1), s2 = spread_shift(lc + g - 2 * s1, 5);
+__device__ __forceinline__ void spread_inv_store_k(SpreadFFT& f, double2 (&x)[K], Store store) {
   fxc y[K];
-  int h[K];
+  int h[K], places = 0;
 #pragma unroll
   for (int m = 0; m < K; m++) {
     h[m] = spread_enter(x[m], y[m]);
     y[m] = spread_swap(y[m]);
   }
-  spread_exchange<C, K>(f, y, h, cl);
+  spread_push<C, true, K>(f, y, h);
 #pragma unroll
-  for (int m = 0; m < K; m++) {
-    store(m, x[m]);
-    y[m] = spread_mul(y[m], f.twC, s1);
-  }
-  spread_cross<K>(f, y, h);
+  for (int m = 0; m < K; m++) store(m, x[m]);
+  spread_backward<C, true, K>(f, y, h, places, 0);
 #pragma unroll
-  for (int m = 0; m < K; m++) y[m] = f.g > 0 ? spread_mul(y[m], f.wgl, s2) : fx_shift(y[m], s2);
-  spread_warp_dft<K>(f, y);
-#pragma unroll
-  for (int m = 0; m < K; m++) x[m] = spread_leave(spread_swap(y[m]), h[m], s1 + s2);
+  for (int m = 0; m < K; m++) x[m] = spread_leave(spread_swap(y[m]), h[m], places);
 }
 
-// n bare cluster barriers: the transform slots of a group that has no transform to do while the other
-// group of the same cluster does (every exchange ends with a barrier of the whole cluster)
-__device__ __forceinline__ void spread_idle(cg::cluster_group& cl, int n) {
-  for (int q = 0; q < n; q++) cl.sync();
+// Forward transform, factors, inverse transform, with the values in integers throughout: one exponent decision
+// and one conversion each way for both transforms.  fac: this thread's Q62 factors per field (relative to 2^et).
+// want: spec(m, v) receives the spectrum times its factor, while the inverse's exchange is in flight.
+template <int C, int K, class Spec>
+__device__ __forceinline__ void spread_pair_k(SpreadFFT& f, double2 (&x)[K], const int4 (&fac)[K], int et, bool want,
+                                              Spec spec) {
+  fxc y[K];
+  int h[K], places, level;
+  spread_forward<C, K>(f, x, y, h, places, level);
+  const int g = 26 - __clz(f.M), lc = fx_log2(C);
+  // leave the inverse's two products no more than they can shift
+  const int s = max(spread_shift(level, lc), (level + lc + g - 7) >> 1);
+#pragma unroll
+  for (int m = 0; m < K; m++) y[m] = spread_swap(spread_mul(y[m], fac[m], s));
+  places += s;
+  spread_push<C, false, K>(f, y, h);
+  if (want) {
+#pragma unroll
+    for (int m = 0; m < K; m++) spec(m, spread_leave(spread_swap(y[m]), h[m], places + et));
+  }
+  spread_backward<C, false, K>(f, y, h, places, level - 2 * s);
+#pragma unroll
+  for (int m = 0; m < K; m++) x[m] = spread_leave(spread_swap(y[m]), h[m], places + et);
 }
 
 // One field.
 template <int C = kSpreadC>
-__device__ __forceinline__ double2 spread_fwd(SpreadFFT& f, double2 x, cg::cluster_group& cl) {
+__device__ __forceinline__ double2 spread_fwd(SpreadFFT& f, double2 x) {
   double2 v[1] = {x};
-  spread_fwd_k<C, 1>(f, v, cl);
+  spread_fwd_k<C, 1>(f, v);
   return v[0];
 }
 
 template <int C = kSpreadC, class Store>
-__device__ __forceinline__ double2 spread_inv_store(SpreadFFT& f, double2 x, cg::cluster_group& cl, Store store) {
+__device__ __forceinline__ double2 spread_inv_store(SpreadFFT& f, double2 x, Store store) {
   double2 v[1] = {x};
-  spread_inv_store_k<C, 1>(f, v, cl, [&](int, double2 s) { store(s); });
+  spread_inv_store_k<C, 1>(f, v, [&](int, double2 s) { store(s); });
   return v[0];
 }
 
 template <int C = kSpreadC>
-__device__ __forceinline__ double2 spread_inv(SpreadFFT& f, double2 x, cg::cluster_group& cl) {
-  return spread_inv_store<C>(f, x, cl, [](double2) {});
+__device__ __forceinline__ double2 spread_inv(SpreadFFT& f, double2 x) {
+  return spread_inv_store<C>(f, x, [](double2) {});
 }
+
+template <int C = kSpreadC>
+__device__ __forceinline__ double2 spread_pair(SpreadFFT& f, double2 x, int4 fac, int et) {
+  double2 v[1] = {x};
+  const int4 q[1] = {fac};
+  spread_pair_k<C, 1>(f, v, q, et, false, [](int, double2) {});
+  return v[0];
+}
+
+template <int C = kSpreadC, class Spec>
+__device__ __forceinline__ double2 spread_pair_spec(SpreadFFT& f, double2 x, int4 fac, int et, bool want, Spec spec) {
+  double2 v[1] = {x};
+  const int4 q[1] = {fac};
+  spread_pair_k<C, 1>(f, v, q, et, want, [&](int, double2 s) { spec(s); });
+  return v[0];
+}
+
+// A factor of modulus at most 1 as Q62 halves (exact: 53 bits).
+__device__ __forceinline__ int4 fx_factor(double2 v) {
+  const long long x = __double2ll_rn(v.x * 0x1p62), y = __double2ll_rn(v.y * 0x1p62);
+  int4 r;
+  fx_split(x, r.x, r.y);
+  fx_split(y, r.z, r.w);
+  return r;
+}
+__device__ __forceinline__ int4 fx_conj(int4 w) { return make_int4(w.x, w.y, -w.z, -w.w); }
 
 }  // namespace nlm

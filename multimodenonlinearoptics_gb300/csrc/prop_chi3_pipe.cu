@@ -3,24 +3,13 @@
 // Ranks 0..3 march the pump with the arithmetic of k_pump_chi3_spread (solvers/Chi3.cpp:41-70); ranks
 // 4..7 propagate the signal with that of k_propagate_spread<FChi3, 4> (src/_NonlinearMedium.hpp:160-239,
 // the solver's DiffEq at every step), one phase behind the pump.  The signal's step i reads pump rows
-// 2i-2, 2i-1 and 2i of the time-domain grid at its own points; the pump writes row 2p at the end of
-// phase p, and the first cluster barrier of the next phase orders that write before the signal's read
+// 2i-2, 2i-1 and 2i of the time-domain grid at its own points; the pump writes rows 2p-1 and 2p in
+// phase p, and the cluster barrier that ends the phase orders those writes before the signal's reads
 // (barrier.cluster arrive has release and wait acquire semantics at cluster scope).  Each march alone
 // is a chain of latency-bound transforms on four SMs; side by side the signal's march costs about
-// nothing beyond the pump's.
-//
-// Every spread transform ends with one barrier of the whole cluster, so both groups pass the same
-// sequence of barrier slots (4 nZ + 2, after one barrier that all eight CTAs pass first):
-//   start        2 slots   pump: row 0 (forward, inverse)   signal: input (forward or bare), inverse
-//   phase p      4 slots   pump: rows 2p-1 and 2p           signal: 2 bare, step p-1 (2 slots)
-//                (p = 1 .. nZ-1; in phase 1 the signal passes 4 bare barriers)
-// An interval between two barriers lasts as long as the slower group.  The pump's intervals alternate
-// long (a local inverse transform, the store, the phase factor, a local forward transform) and short
-// (the exchange's combination and the dispersion factor); the signal's step has the same shape (its
-// long part: the pump loads, the DiffEq and the local forward transform; then the short part; its
-// local inverse transform falls in the pump's next long interval), placed so that long meets long.
-//   end          4 slots   pump: the last row's half-step   signal: 2 bare, step nZ-1 (forward, then
-//                          undo (inverse), 3 bare                   inverse or bare)
+// nothing beyond the pump's.  The groups' exchanges wait for their own four CTAs only, so the phase
+// barrier is the one place where they meet: nZ of them after the opening one, in both groups
+// (pump: one after each row pair and two at the end; signal: one before each step and one at the end).
 // The pump group runs the operations of k_pump_chi3_spread in the same order; the two kernels' grids
 // agree to rounding (the compiler may pair multiply-adds differently in each).
 #include "nlm_launch.h"
@@ -35,75 +24,66 @@ __global__ void __launch_bounds__(kMaxThreads) k_chi3_pump_signal_spread(const P
   const int role = crank / kSpreadC;   // 0: pump march, 1: signal
   SpreadFFT f;
   const int M = a.plan.N;
-  spread_init(f, smem, a.fx.twN, M, crank - role * kSpreadC);
+  spread_init(f, smem, a.fx.twN, M, crank - role * kSpreadC, a.fx.err);
   f.base = role * kSpreadC;
   const int N = M * kSpreadC;
   const int tn = f.rank + kSpreadC * f.t, fk = f.j + M * f.rank;
   const int nZ = a.nZ;
   cl.sync();   // every CTA of the cluster has started before the first exchange writes to its memory
+  const int et = -(31 - __clz(N));   // the inverse transforms' 1/N
   if (role == 0) {
     const double invN = 1.0 / N;
-    const double2 hp = p.halfP[fk], dp = p.dstepP[fk];
-    double2 x = spread_fwd(f, p.env[tn], cl);
-    x = cmul(x, hp);
-    x = cscale(spread_inv_store(f, x, cl, [&](double2 v) { p.pf[fk] = v; }), invN);
+    const int4 dp = fx_factor(p.dstepP[fk]);
+    double2 x = spread_fwd(f, p.env[tn]);
+    x = cmul(x, p.halfP[fk]);
+    x = cscale(spread_inv_store(f, x, [&](double2 v) { p.pf[fk] = v; }), invN);
     p.pt[tn] = x;
     for (int i = 1; i < p.nRows; i++) {
       const double2 r = p.rel[i - 1];
       const double a2 = cabs2(x);
       x = cmul(x, spm_factor(r.x * a2, r.y * a2));
-      x = cmul(spread_fwd(f, x, cl), dp);
-      x = cscale(spread_inv_store(f, x, cl, [&](double2 v) { p.pf[(long long)i * N + fk] = v; }), invN);
-      p.pt[(long long)i * N + tn] = x;
+      x = spread_pair_spec(f, x, dp, et, true, [&](double2 v) { p.pf[(long long)i * N + fk] = cscale(v, (double)N); });
+      if (i < p.nRows - 1) p.pt[(long long)i * N + tn] = x;
+      if ((i & 1) == 0 && i < p.nRows - 1) cl.sync();   // rows up to i are in place for step i / 2
     }
     // last row: undo half of the last pump dispersion step (each thread rereads its own bin)
     const long long last = (long long)(p.nRows - 1) * N;
     x = cmul(p.pf[last + fk], p.backP[fk]);
-    p.pt[last + tn] = cscale(spread_inv_store(f, x, cl, [&](double2 v) { p.pf[last + fk] = v; }), invN);
-    spread_idle(cl, 3);
+    p.pt[last + tn] = cscale(spread_inv_store(f, x, [&](double2 v) { p.pf[last + fk] = v; }), invN);
+    cl.sync();
+    cl.sync();
     return;
   }
   const long long inst = a.instBase;
   double2 x = a.in[inst * a.inStride + (a.inTime ? tn : fk)];
-  if (a.inTime) x = spread_fwd(f, x, cl);
-  else cl.sync();
+  if (a.inTime) x = spread_fwd(f, x);
   x = cmul(x, __ldg(a.half + fk));
-  x = spread_inv_store(f, x, cl, [&](double2 v) {
+  x = spread_inv_store(f, x, [&](double2 v) {
     if (a.gridF) a.gridF[fk] = cscale(v, (double)N);
   });
   if (a.gridT) a.gridT[tn] = x;
   // step i: the DiffEq with pump rows 2i-2 .. 2i (plain loads: the pump group writes them during this
-  // launch), then the dispersion step; two barrier slots
-  auto step = [&](int i) {
+  // launch), then the dispersion step
+  for (int i = 1; i < nZ; i++) {
+    cl.sync();   // pump rows up to 2i are in place
     const double2* c = a.coef + (long long)(i - 1) * 3 * a.nCoef;
     const double2* pr = a.pump + (long long)(2 * i - 2) * N + tn;
     double2 pp[3][1] = {{pr[0]}, {pr[N]}, {pr[2 * N]}};
     double2 xm[1] = {x};
     rk4_point<FChi3>(xm, pp, c);
     const bool last = i == nZ - 1;
-    const double2* table = last ? a.dlast : a.dstep;
-    const bool wantTime = !last || a.inTime || a.gridT != nullptr;
-    x = cmul(spread_fwd(f, xm[0], cl), __ldg(table + fk));
     auto storeF = [&](double2 v) {
       if (a.gridF) a.gridF[(long long)i * N + fk] = cscale(v, (double)N);
     };
-    if (wantTime) {
-      x = spread_inv_store(f, x, cl, storeF);
+    if (!last || a.inTime || a.gridT != nullptr) {
+      x = spread_pair_spec(f, xm[0], __ldg(a.fx.tab + (last ? N : 0) + fk), a.fx.et, a.gridF != nullptr, storeF);
       if (a.gridT) a.gridT[(long long)i * N + tn] = x;
     } else {
+      x = cmul(spread_fwd(f, xm[0]), __ldg(a.dlast + fk));
       storeF(x);
-      cl.sync();
     }
-  };
-  spread_idle(cl, 4);   // phase 1: the pump computes rows 1 and 2
-  for (int ph = 2; ph < nZ; ph++) {
-    // after the first barrier rows up to 2 ph - 2 are in place; after the second the step's long part
-    // (loads, DiffEq, local forward transform) runs beside the pump's (local transforms, phase factor)
-    spread_idle(cl, 2);
-    step(ph - 1);
   }
-  spread_idle(cl, 2);   // the pump's last row, then the barrier after its store
-  step(nZ - 1);
+  cl.sync();
 }
 
 cudaError_t launch_chi3_pump_signal_spread(const PropArgs& a, const PumpMarchArgs& p, cudaStream_t s, int* regs) {

@@ -6,7 +6,7 @@
 // plus the dispersion pair; with the RK4 sum in the frequency domain, 16 in all.  With four points per thread on four CTAs (prop_cluster_gnlse.cu) a
 // single 4096-point propagation takes about 260 us per step; here it holds N / C points per CTA, one
 // per thread: sixteen CTAs of 256 threads at 4096 points (the full-grid form), eight of 256 at 2048.
-// The per-point tables (Raman response, self-steepening factors, dispersion) stay in registers.
+// The Raman response and self-steepening factors stay in registers.
 #include <vector>
 
 #include "nlm_spread.cuh"
@@ -22,22 +22,22 @@ __global__ void __launch_bounds__(C == 16 ? 256 : kMaxThreads) k_propagate_gnlse
   SpreadFFT f;
   const int rank = (int)cl.block_rank();
   const int M = a.plan.N;
-  spread_init<C>(f, smem, a.fx.twN, M, rank);
+  spread_init<C>(f, smem, a.fx.twN, M, rank, a.fx.err);
+  cl.sync();
   const int N = M * C;
   const int tn = rank + C * f.t;   // time-domain point of this thread
   const int fk = f.j + M * rank;   // frequency bin of this thread
-  const double2 ram = __ldg(a.raman + fk), stp = __ldg(a.steep + fk);
-  const double2 dst = __ldg(a.dstep + fk), dla = __ldg(a.dlast + fk);
+  const int4 ram = __ldg(a.fx.raman + fk), stp = __ldg(a.fx.steep + fk);
   const long long clusterId = blockIdx.x / C, nClusters = gridDim.x / C;
   for (long long local = clusterId; local < a.nInst; local += nClusters) {
     const long long inst = a.instBase + local;
     const double2* row = a.in + inst * a.inStride;
     const bool has = a.inputMode == 0 || (a.inputMode < 1 && a.inChannels > 0);
     double2 x = has ? row[a.inTime ? tn : fk] : czero();
-    if (a.inTime) x = spread_fwd<C>(f, x, cl);
+    if (a.inTime) x = spread_fwd<C>(f, x);
     x = cmul(x, __ldg(a.half + fk));
     double2 xf = x;   // the state's spectrum (whose unscaled inverse transform is x)
-    x = spread_inv_store<C>(f, x, cl, [&](double2 v) {
+    x = spread_inv_store<C>(f, x, [&](double2 v) {
       if (a.gridF) a.gridF[fk] = cscale(v, (double)N);
     });
     if (a.gridT) a.gridT[tn] = x;
@@ -59,22 +59,24 @@ __global__ void __launch_bounds__(C == 16 ? 256 : kMaxThreads) k_propagate_gnlse
         double2 u = make_double2(ri * cabs2(y), 0.0);
         if (stg) stg[(long long)s * N + tn] = y;
         // Raman convolution R~ * (rel |y|^2)
-        u = spread_fwd<C>(f, u, cl);
-        u = spread_inv<C>(f, cmul(u, ram), cl);
+        u = spread_pair<C>(f, u, ram, a.fx.etRaman);
         if (stg) stg[(long long)(4 + s) * N + tn] = u;
         // times the field, then the self-steepening operator (g0 + g1 w)
-        u = cmul(spread_fwd<C>(f, cmul(u, y), cl), stp);
-        acc = s == 0 ? u : caxpy(acc, wgt, u);
-        if (s < 3) k = spread_inv<C>(f, u, cl);
+        u = cmul(u, y);
+        if (s < 3) {
+          k = spread_pair_spec<C>(f, u, stp, a.fx.etSteep, true, [&](double2 v) { acc = s == 0 ? v : caxpy(acc, wgt, v); });
+        } else {
+          acc = cadd(acc, cmul(spread_fwd<C>(f, u), __ldg(a.steep + fk)));
+        }
       }
       const bool last = i == a.nZ - 1;
-      x = cmul(cscale(caxpy(xf, 1.0 / 6.0, acc), (double)N), last ? dla : dst);
+      x = cmul(cscale(caxpy(xf, 1.0 / 6.0, acc), (double)N), __ldg((last ? a.dlast : a.dstep) + fk));
       if (!last) xf = x;
       auto storeF = [&](double2 v) {
         if (a.gridF) a.gridF[(long long)i * N + fk] = cscale(v, (double)N);
       };
       if (!last || a.inTime || a.gridT) {
-        x = spread_inv_store<C>(f, x, cl, storeF);
+        x = spread_inv_store<C>(f, x, storeF);
         if (a.gridT) a.gridT[(long long)i * N + tn] = x;
         if (ckRow && !last && i % a.ckK == 0) ckRow[(long long)(i / a.ckK) * N + tn] = x;
       } else {
@@ -82,10 +84,10 @@ __global__ void __launch_bounds__(C == 16 ? 256 : kMaxThreads) k_propagate_gnlse
       }
     }
     if (a.nZ == 1) {
-      x = cmul(spread_fwd<C>(f, x, cl), __ldg(a.back + fk));
+      x = cmul(spread_fwd<C>(f, x), __ldg(a.back + fk));
       if (a.gridF) a.gridF[fk] = cscale(x, (double)N);
       if (a.inTime || a.gridT) {
-        x = spread_inv<C>(f, x, cl);
+        x = spread_inv<C>(f, x);
         if (a.gridT) a.gridT[tn] = x;
       }
     }
@@ -95,6 +97,7 @@ __global__ void __launch_bounds__(C == 16 ? 256 : kMaxThreads) k_propagate_gnlse
       o[a.inTime ? tn : fk] = cscale(x, a.inTime ? 1.0 : (double)N);
     }
   }
+  cl.sync();
 }
 
 // kind kKindCluster, R = 1 (one point per thread): key Chi3GNLSE (four CTAs), + kSpreadWideKey (eight),

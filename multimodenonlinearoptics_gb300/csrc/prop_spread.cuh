@@ -17,56 +17,74 @@ __global__ void __launch_bounds__(kMaxThreads) k_pump_chi3_spread(double2* __res
                                                                   const double2* __restrict__ dstepP,
                                                                   const double2* __restrict__ backP,
                                                                   const double2* __restrict__ rel, int nRows, int M,
-                                                                  const int4* __restrict__ tw) {
+                                                                  const int4* __restrict__ tw, int* err) {
   extern __shared__ double2 smem[];
   cg::cluster_group cl = cg::this_cluster();
   SpreadFFT f;
   const int rank = (int)cl.block_rank();
-  spread_init<C>(f, smem, tw, M, rank);
+  spread_init<C>(f, smem, tw, M, rank, err);
+  cl.sync();
   const int N = M * C;
   const int tn = rank + C * f.t;          // time-domain point of this thread
   const int fk = f.j + M * rank;          // frequency bin of this thread
   const double invN = 1.0 / N;
-  const double2 hp = halfP[fk], dp = dstepP[fk];
-  double2 x = spread_fwd<C>(f, env[tn], cl);
-  x = cmul(x, hp);
-  x = cscale(spread_inv_store<C>(f, x, cl, [&](double2 v) { pf[fk] = v; }), invN);
+  const int et = -(31 - __clz(N));        // the inverse transform's 1/N
+  const int4 dp = fx_factor(dstepP[fk]);
+  double2 x = spread_fwd<C>(f, env[tn]);
+  x = cmul(x, halfP[fk]);
+  x = cscale(spread_inv_store<C>(f, x, [&](double2 v) { pf[fk] = v; }), invN);
   pt[tn] = x;
   for (int i = 1; i < nRows; i++) {
     const double2 r = rel[i - 1];
     const double a2 = cabs2(x);
     x = cmul(x, spm_factor(r.x * a2, r.y * a2));
-    x = cmul(spread_fwd<C>(f, x, cl), dp);
-    x = cscale(spread_inv_store<C>(f, x, cl, [&](double2 v) { pf[(long long)i * N + fk] = v; }), invN);
+    // the spectrum comes with the 1/N of the field
+    x = spread_pair_spec<C>(f, x, dp, et, true, [&](double2 v) { pf[(long long)i * N + fk] = cscale(v, (double)N); });
     pt[(long long)i * N + tn] = x;
   }
   // last row: undo half of the last pump dispersion step (each thread rereads its own bin)
   const long long last = (long long)(nRows - 1) * N;
   x = cmul(pf[last + fk], backP[fk]);
-  pt[last + tn] = cscale(spread_inv_store<C>(f, x, cl, [&](double2 v) { pf[last + fk] = v; }), invN);
+  pt[last + tn] = cscale(spread_inv_store<C>(f, x, [&](double2 v) { pf[last + fk] = v; }), invN);
+  cl.sync();
 }
 
 // All MD modes: time -> frequency domain; K = MD together, K = 1 one after another.
 template <int C, int K, int MD>
-__device__ __forceinline__ void spread_fwd_all(SpreadFFT& f, double2 (&x)[MD], cg::cluster_group& cl) {
+__device__ __forceinline__ void spread_fwd_all(SpreadFFT& f, double2 (&x)[MD]) {
   if constexpr (K > 1) {
-    spread_fwd_k<C, MD>(f, x, cl);
+    spread_fwd_k<C, MD>(f, x);
   } else {
 #pragma unroll
-    for (int m = 0; m < MD; m++) x[m] = spread_fwd<C>(f, x[m], cl);
+    for (int m = 0; m < MD; m++) x[m] = spread_fwd<C>(f, x[m]);
   }
 }
 
 // All MD modes: frequency -> time domain, store(m, v) given each mode's spectrum after its exchange.
 template <int C, int K, int MD, class Store>
-__device__ __forceinline__ void spread_inv_all(SpreadFFT& f, double2 (&x)[MD], cg::cluster_group& cl, Store store) {
+__device__ __forceinline__ void spread_inv_all(SpreadFFT& f, double2 (&x)[MD], Store store) {
   if constexpr (K > 1) {
-    spread_inv_store_k<C, MD>(f, x, cl, store);
+    spread_inv_store_k<C, MD>(f, x, store);
   } else {
 #pragma unroll
     for (int m = 0; m < MD; m++) {
       const int mm = m;
-      x[m] = spread_inv_store<C>(f, x[m], cl, [&](double2 v) { store(mm, v); });
+      x[m] = spread_inv_store<C>(f, x[m], [&](double2 v) { store(mm, v); });
+    }
+  }
+}
+
+// All MD modes through the dispersion pair.
+template <int C, int K, int MD, class Spec>
+__device__ __forceinline__ void spread_pair_all(SpreadFFT& f, double2 (&x)[MD], const int4 (&fac)[MD], int et, bool want,
+                                                Spec spec) {
+  if constexpr (K > 1) {
+    spread_pair_k<C, MD>(f, x, fac, et, want, spec);
+  } else {
+#pragma unroll
+    for (int m = 0; m < MD; m++) {
+      const int mm = m;
+      x[m] = spread_pair_spec<C>(f, x[m], fac[m], et, want, [&](double2 v) { spec(mm, v); });
     }
   }
 }
@@ -74,8 +92,7 @@ __device__ __forceinline__ void spread_inv_all(SpreadFFT& f, double2 (&x)[MD], c
 // One propagation per cluster (clusters take instances in turn); a.plan.N = M, a.fx.twN the N-point table.
 // Point-wise work: the pump-driven solvers' RK4 matrices (a.prop) or the solver's DiffEq.  K = 1: the
 // modes' transforms one after another; K = the solver's mode count: all modes in each transform
-// together (spread_fwd_k, spread_inv_store_k: one barrier per stage and one cluster barrier per
-// exchange for all of them), with K times the exchange and receive buffers.  Either way every mode
+// together (the _k forms: one barrier and one exchange per transform for all of them), with K times the exchange and receive buffers.  Either way every mode
 // goes through the same operations, so the results are identical.
 template <class S, int C, int K = 1>
 __global__ void __launch_bounds__(kMaxThreads) k_propagate_spread(const PropArgs a) {
@@ -86,7 +103,8 @@ __global__ void __launch_bounds__(kMaxThreads) k_propagate_spread(const PropArgs
   SpreadFFT f;
   const int rank = (int)cl.block_rank();
   const int M = a.plan.N;
-  spread_init<C, K>(f, smem, a.fx.twN, M, rank);
+  spread_init<C, K>(f, smem, a.fx.twN, M, rank, a.fx.err);
+  cl.sync();
   const int N = M * C;
   const int tn = rank + C * f.t;
   const int fk = f.j + M * rank;
@@ -103,10 +121,10 @@ __global__ void __launch_bounds__(kMaxThreads) k_propagate_spread(const PropArgs
       else if (a.inputMode < 1 && m < a.inChannels) seg = m;
       x[m] = seg >= 0 ? row[(long long)seg * N + (a.inTime ? tn : fk)] : czero();
     }
-    if (a.inTime) spread_fwd_all<C, K, MD>(f, x, cl);
+    if (a.inTime) spread_fwd_all<C, K, MD>(f, x);
 #pragma unroll
     for (int m = 0; m < MD; m++) x[m] = cmul(x[m], __ldg(a.half + (long long)m * N + fk));
-    spread_inv_all<C, K, MD>(f, x, cl, [&](int m, double2 v) {
+    spread_inv_all<C, K, MD>(f, x, [&](int m, double2 v) {
       if (a.gridF) a.gridF[m * ms + fk] = cscale(v, (double)N);
     });
     if (a.gridT) {
@@ -161,23 +179,26 @@ __global__ void __launch_bounds__(kMaxThreads) k_propagate_spread(const PropArgs
         rk4_point<S>(x, p, c);
       }
       const bool last = i == a.nZ - 1;
-      const double2* table = last ? a.dlast : a.dstep;
       const bool wantTime = !last || a.inTime || a.gridT != nullptr;
-      spread_fwd_all<C, K, MD>(f, x, cl);
-#pragma unroll
-      for (int m = 0; m < MD; m++) x[m] = cmul(x[m], __ldg(table + (long long)m * N + fk));
       auto storeF = [&](int m, double2 v) {
         if (a.gridF) a.gridF[m * ms + (long long)i * N + fk] = cscale(v, (double)N);
       };
       if (wantTime) {
-        spread_inv_all<C, K, MD>(f, x, cl, storeF);
+        int4 fac[MD];
+#pragma unroll
+        for (int m = 0; m < MD; m++) fac[m] = __ldg(a.fx.tab + (long long)((last ? MD : 0) + m) * N + fk);
+        spread_pair_all<C, K, MD>(f, x, fac, a.fx.et, a.gridF != nullptr, storeF);
         if (a.gridT) {
 #pragma unroll
           for (int m = 0; m < MD; m++) a.gridT[m * ms + (long long)i * N + tn] = x[m];
         }
       } else {
+        spread_fwd_all<C, K, MD>(f, x);
 #pragma unroll
-        for (int m = 0; m < MD; m++) storeF(m, x[m]);
+        for (int m = 0; m < MD; m++) {
+          x[m] = cmul(x[m], __ldg(a.dlast + (long long)m * N + fk));
+          storeF(m, x[m]);
+        }
       }
       if (ckRow && !last && i % a.ckK == 0) {
 #pragma unroll
@@ -185,14 +206,14 @@ __global__ void __launch_bounds__(kMaxThreads) k_propagate_spread(const PropArgs
       }
     }
     if (a.nZ == 1) {
-      spread_fwd_all<C, K, MD>(f, x, cl);
+      spread_fwd_all<C, K, MD>(f, x);
 #pragma unroll
       for (int m = 0; m < MD; m++) {
         x[m] = cmul(x[m], __ldg(a.back + (long long)m * N + fk));
         if (a.gridF) a.gridF[m * ms + fk] = cscale(x[m], (double)N);
       }
       if (a.inTime || a.gridT) {
-        spread_inv_all<C, K, MD>(f, x, cl, [&](int, double2) {});
+        spread_inv_all<C, K, MD>(f, x, [&](int, double2) {});
         if (a.gridT) {
 #pragma unroll
           for (int m = 0; m < MD; m++) a.gridT[m * ms + tn] = x[m];
@@ -210,6 +231,7 @@ __global__ void __launch_bounds__(kMaxThreads) k_propagate_spread(const PropArgs
       }
     }
   }
+  cl.sync();
 }
 
 }  // namespace nlm
