@@ -17,7 +17,7 @@ namespace nlm {
 // gradient starts in the frequency domain.
 __device__ __forceinline__ double2 spread_adjoint_dispersion(const PropArgs& a, SpreadFFT& f, double2 g, int i, int fk) {
   if (i < a.nZ - 1) return spread_pair(f, g, fx_conj(__ldg(a.fx.tab + fk)), a.fx.et);
-  return spread_inv(f, cmulc(g, __ldg(a.dlast + fk)));
+  return spread_inv_end(f, cmulc(g, __ldg(a.dlast + fk)));
 }
 
 // a.plan.N = M (N / 4 threads per CTA); a.fx.twN: the N-point table.  d.seg: [cluster][K][N] when d.K > 1.
@@ -66,7 +66,7 @@ __global__ void __launch_bounds__(kMaxThreads) k_adjoint_pdc_spread(const PropAr
       segEnd = s0;
     }
     // gradient of the input spectrum: s_0 = IFFT(half X_in)
-    g = spread_fwd(f, g);
+    g = spread_fwd_end(f, g);
     d.gin[inst * (long long)N + fk] = cmulc(g, __ldg(a.half + fk));
   }
   cl.sync();
@@ -133,7 +133,7 @@ __global__ void __launch_bounds__(kMaxThreads) k_adjoint_pdc_spread_pipe(const P
       cl.sync();
     }
     if (role == 0) {
-      g = spread_fwd(f, g);
+      g = spread_fwd_end(f, g);
       d.gin[inst * (long long)N + fk] = cmulc(g, __ldg(a.half + fk));
     }
   }
@@ -248,7 +248,7 @@ __global__ void __launch_bounds__(kMaxThreads) k_adjoint_pdc_spread_stage(const 
       cl.sync();
     }
     if (role == 0) {
-      g = spread_fwd(f, g);
+      g = spread_fwd_end(f, g);
       d.gin[inst * (long long)N + fk] = cmulc(g, __ldg(a.half + fk));
     }
     // segment 0 (reversed in the last iteration): its steps shared by all groups

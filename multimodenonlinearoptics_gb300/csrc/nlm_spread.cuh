@@ -21,9 +21,9 @@
 // The values are FP64 on both sides and 64-bit integers inside (nlm_fx.cuh says why and how).  A warp issues one
 // FP64 instruction in 64 cycles on its scheduler, so the ~30 of a transform in FP64 took about 1 us however
 // few points there were; an IMAD.WIDE or a 64-bit addition takes two cycles.  Every warp scales its 32 points
-// by its own exponent (a bound on its 2-norm in half bits, from two warp reductions and no barrier) and sends
-// that code along with its values through each exchange; the receivers shift the values to the exponent of
-// the total.  Starting below 2^59, the norm grows by sqrt(32) in the warps, sqrt(G) across them and sqrt(C)
+// by its own exponent (a bound on its 2-norm in half bits, from two warp reductions and no barrier).  These codes
+// cross the cluster, in a forward transform while the warps' DFTs run, and each warp then shifts its values to the
+// total's exponent.  Starting below 2^59, the norm grows by sqrt(32) in the warps, sqrt(G) across them and sqrt(C)
 // across the CTAs, and is shifted back where it would pass 2^61.5 (spread_shift).
 // Exchanges over the cluster: each value travels by st.async, which counts its bytes on the receiving warp's
 // mbarrier, and a warp waits for the C x 32 values of its own columns.  No barrier of the cluster and no fence
@@ -32,10 +32,11 @@
 // received exchange n + 1 from the thread that reads that column, which pushed it after reading half n.
 // Waits give up after kSpreadWait polls and raise *err; every CTA then still runs to the closing cluster barrier.
 // Shared memory: M twiddles, two M-point exchange buffers (alternating: a thread writes a buffer only after
-// the barrier that every reader of that buffer's previous contents has passed), the two halves of C x M values;
-// the exponent codes lie beside each.
+// the barrier that every reader of that buffer's previous contents has passed), the two halves of C x M values.
 // M is a power of two of at least 32, N = C M at most 4096.
 #pragma once
+#include <climits>
+
 #include <cooperative_groups.h>
 
 #include "nlm_fx.cuh"
@@ -60,10 +61,11 @@ struct SpreadFFT {
   int4 w16, w8, w4;     // the lane's factors of the warp stages of 16, 8 and 4
   int4* buf;            // [2][K][M] exchange buffers of the local transform
   int4* recv;           // [2][C][K][M] cluster receive buffers
-  int* code;            // [2][K][G] exponent codes of the exchange buffers
-  int* rcode;           // [2][C][K][G] and of the receive buffers
+  int* ecode;           // [2][K][C][G] exponent codes of the cluster's warps
+  unsigned ebar;        // shared address of the CTA's two mbarriers for them
+  int ephase;           // the next of the two
   unsigned bar;         // shared address of this warp's two mbarriers
-  unsigned parity;      // bit p: the phase that mbarrier p completes next
+  unsigned parity;      // bits 0, 1: the phases that the warp's mbarriers complete next; 2, 3: the codes'
   int* err;             // raised (host memory) when an exchange does not arrive
   bool dead;            // an exchange has timed out: no more waiting
   int M, rank, j;
@@ -81,8 +83,8 @@ __device__ __forceinline__ unsigned spread_saddr(const void* p) { return (unsign
 template <int C = kSpreadC, int K = 1>
 __device__ __forceinline__ void spread_init(SpreadFFT& f, double2* smem, const int4* __restrict__ tw, int M, int rank,
                                             int* err) {
-  __shared__ int s_code[2 * 4 * 16], s_rcode[2 * kSpreadMaxCodes];
-  __shared__ unsigned long long s_bar[2 * 16];
+  __shared__ int s_ecode[2 * kSpreadMaxCodes];
+  __shared__ unsigned long long s_bar[2 * 16 + 2];
   f.M = M;
   f.rank = rank;
   f.j = threadIdx.x;
@@ -92,9 +94,10 @@ __device__ __forceinline__ void spread_init(SpreadFFT& f, double2* smem, const i
   f.sel = 0;
   f.phase = 0;
   f.base = 0;
-  f.code = s_code;
-  f.rcode = s_rcode;
+  f.ecode = s_ecode;
+  f.ephase = 0;
   f.bar = spread_saddr(s_bar + 2 * f.g);
+  f.ebar = spread_saddr(s_bar + 2 * 16);
   f.parity = 0;
   f.err = err;
   f.dead = false;
@@ -106,6 +109,7 @@ __device__ __forceinline__ void spread_init(SpreadFFT& f, double2* smem, const i
   f.twC = tw[(long long)rank * f.j];
   if (f.l < 2) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(f.bar + 8 * f.l) : "memory");
+    if (f.g == 0) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(f.ebar + 8 * f.l) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   __syncthreads();
@@ -117,10 +121,10 @@ __device__ __forceinline__ void spread_init(SpreadFFT& f, double2* smem, const i
   f.wgl = twM[f.g * f.l];
 }
 
-// Waits for the exchange in flight (half f.phase) of this warp.
-__device__ __forceinline__ void spread_wait(SpreadFFT& f) {
-  const unsigned bar = f.bar + 8 * f.phase, par = (f.parity >> f.phase) & 1;
-  f.parity ^= 1u << f.phase;
+// Waits for the phase of an mbarrier that bit `bit` of f.parity names, and moves on to the next one.
+__device__ __forceinline__ void spread_wait(SpreadFFT& f, unsigned bar, int bit) {
+  const unsigned par = (f.parity >> bit) & 1;
+  f.parity ^= 1u << bit;
   if (f.dead) return;
   for (int n = 0; n < kSpreadWait; n++) {
     unsigned ok;
@@ -146,8 +150,13 @@ __device__ __forceinline__ fxc spread_swap(fxc v) { return fxc{v.y, v.x}; }
 // Places to shift before a stage that adds `grow` half bits to a norm standing `level` half bits above 2^A0.
 __device__ __forceinline__ int spread_shift(int level, int grow) { return max(0, (level + grow - kSpreadPeak + 1) >> 1); }
 
-// The point as integers below the warp's exponent; returns the warp's code h (norm^2 < 2^h).
-__device__ __forceinline__ int spread_enter(double2 x, fxc& y) {
+struct SpreadPoint {
+  fxc y;
+  int h;
+};
+
+// The point as integers below the warp's exponent, and the warp's code h (norm^2 < 2^h).
+__device__ __forceinline__ SpreadPoint spread_enter(double2 x) {
   auto top = [](double2 v) {
     return __reduce_max_sync(0xffffffffu, max((unsigned)__double2hiint(v.x) & 0x7fffffffu, (unsigned)__double2hiint(v.y) & 0x7fffffffu));
   };
@@ -163,8 +172,8 @@ __device__ __forceinline__ int spread_enter(double2 x, fxc& y) {
   const unsigned S = __reduce_add_sync(0xffffffffu, (unsigned)(fmaf(p, p, q * q) * 65536.f) + 2u);
   const int h = 2 * (e - 1023) + 16 - __clz((int)S);   // S < 2^(32 - clz), in units of 2^-16
   const int rel = 62 - kSpreadA0 + 1023 + ((h + 1) >> 1);
-  y = e == 0 ? fxc{0, 0} : fxc{fx_from(x.x, rel), fx_from(x.y, rel)};
-  return e == 0 ? kSpreadZero : e == 0x7ff ? kSpreadBad : h - 2 * lift;
+  const fxc y = e == 0 ? fxc{0, 0} : fxc{fx_from(x.x, rel), fx_from(x.y, rel)};
+  return SpreadPoint{y, e == 0 ? kSpreadZero : e == 0x7ff ? kSpreadBad : h - 2 * lift};
 }
 
 // y 2^(ceil(h / 2) - A0 + places) as FP64
@@ -178,22 +187,6 @@ __device__ __forceinline__ double2 spread_leave(fxc y, int h, int places) {
     else x = make_double2(scalbn(x.x, k), scalbn(x.y, k));
   }
   return x;
-}
-
-// The code of the total of P fields' codes, and each one's shift to it.
-template <int P>
-__device__ __forceinline__ int spread_total(const int (&h)[P], int (&r)[P]) {
-  int top = h[0];
-#pragma unroll
-  for (int c = 1; c < P; c++) top = max(top, h[c]);
-  float s = 0.f;
-#pragma unroll
-  for (int c = 0; c < P; c++) s += __int_as_float(max(127 + h[c] - top, 0) << 23);
-  const int tot = top + ((__float_as_int(s) + 0x7fffff) >> 23) - 127;
-  const int a = (tot + 1) >> 1;
-#pragma unroll
-  for (int c = 0; c < P; c++) r[c] = min(a - ((h[c] + 1) >> 1), 62);
-  return tot;
 }
 
 // v >> r, rounded
@@ -238,138 +231,148 @@ __device__ __forceinline__ fxc spread_combine(const fxc (&v)[P], int r, const in
   }
 }
 
+// Output r of the P-point DFT of the P values at p, p + stride, ... in shared memory.
+template <int P>
+__device__ __forceinline__ fxc spread_gather(const int4* p, int stride, int r, const int4* twM, int M) {
+  fxc v[P];
+#pragma unroll
+  for (int c = 0; c < P; c++) v[c] = fx_unpack(p[c * stride]);
+  return spread_combine<P>(v, r, twM, M);
+}
+// sixteen warps: a call, since its code in every transform of every kernel would be most of the library
+static __device__ __noinline__ fxc spread_gather16(const int4* p, int r, const int4* twM, int M) {
+  return spread_gather<16>(p, 32, r, twM, M);
+}
+__device__ __forceinline__ fxc spread_gather_warps(const int4* p, int r, const int4* twM, int M) {
+  switch (M >> 5) {
+    case 2: return spread_gather<2>(p, 32, r, twM, M);
+    case 4: return spread_gather<4>(p, 32, r, twM, M);
+    case 8: return spread_gather<8>(p, 32, r, twM, M);
+    default: return spread_gather16(p, r, twM, M);
+  }
+}
+
 // 32-point DFT over the lanes: lane l holds element l on entry and bin l on return.  Decimation in
 // frequency: stage s pairs lane l with l ^ s, the lower lane takes a + b, the upper (a - b) W_2s^(l mod s);
 // then every lane takes its bit-reversed lane's value.  The norm grows by sqrt(32).
-template <int K>
-__device__ __forceinline__ void spread_warp_dft(const SpreadFFT& f, fxc (&x)[K]) {
+__device__ __forceinline__ fxc spread_warp_dft(fxc x, int4 w16, int4 w8, int4 w4, int l) {
 #pragma unroll
   for (int s = 16; s >= 1; s >>= 1) {
-    const long long neg = (f.l & s) ? -1 : 0;
-#pragma unroll
-    for (int m = 0; m < K; m++) {
-      const fxc p = fxc{__shfl_xor_sync(0xffffffffu, x[m].x, s), __shfl_xor_sync(0xffffffffu, x[m].y, s)};
-      fxc t = fxc{p.x + ((x[m].x ^ neg) - neg), p.y + ((x[m].y ^ neg) - neg)};
-      if (s >= 4) t = fx_cmul(t, s == 16 ? f.w16 : s == 8 ? f.w8 : f.w4, 2);
-      if (s == 2 && (f.l & 3) == 3) t = fxc{t.y, -t.x};   // W_4 = -i
-      x[m] = t;
-    }
+    const long long neg = (l & s) ? -1 : 0;
+    const fxc p = fxc{__shfl_xor_sync(0xffffffffu, x.x, s), __shfl_xor_sync(0xffffffffu, x.y, s)};
+    fxc t = fxc{p.x + ((x.x ^ neg) - neg), p.y + ((x.y ^ neg) - neg)};
+    if (s >= 4) t = fx_cmul(t, s == 16 ? w16 : s == 8 ? w8 : w4, 2);
+    if (s == 2 && (l & 3) == 3) t = fxc{t.y, -t.x};   // W_4 = -i
+    x = t;
   }
-  const int src = (int)(__brev((unsigned)f.l) >> 27);
-#pragma unroll
-  for (int m = 0; m < K; m++) x[m] = spread_shfl(x[m], src);
+  return spread_shfl(x, (int)(__brev((unsigned)l) >> 27));
 }
 
-// G-point DFT across the warps of a CTA for every lane; CODES: the warps' exponents differ (h: the warp's codes
-// in, the CTA's out), else they are the cluster's.
-template <int G, bool CODES, int K>
-__device__ __forceinline__ void spread_cross_g(SpreadFFT& f, fxc (&x)[K], int (&h)[K]) {
+// G-point DFT across the warps of a CTA for every lane.
+template <int K>
+__device__ __forceinline__ void spread_cross(SpreadFFT& f, fxc (&x)[K]) {
+  if (f.M == 32) return;   // one warp
   int4* b = f.buf + f.sel * K * f.M;
-  int* cd = f.code + f.sel * K * G;
 #pragma unroll
-  for (int m = 0; m < K; m++) {
-    b[m * f.M + f.j] = fx_pack(x[m]);
-    if (CODES && f.l == 0) cd[m * G + f.g] = h[m];
-  }
+  for (int m = 0; m < K; m++) b[m * f.M + f.j] = fx_pack(x[m]);
   __syncthreads();
 #pragma unroll
-  for (int m = 0; m < K; m++) {
-    int hs[G], r[G];
-    fxc v[G];
-    if constexpr (CODES) {
-#pragma unroll
-      for (int c = 0; c < G; c++) hs[c] = cd[m * G + c];
-      h[m] = spread_total<G>(hs, r);
-    }
-#pragma unroll
-    for (int c = 0; c < G; c++) {
-      v[c] = fx_unpack(b[m * f.M + c * 32 + f.l]);
-      if constexpr (CODES) v[c] = spread_align(v[c], r[c]);
-    }
-    x[m] = spread_combine<G>(v, f.g, f.twM, f.M);
-  }
+  for (int m = 0; m < K; m++) x[m] = spread_gather_warps(b + m * f.M + f.l, f.g, f.twM, f.M);
   f.sel ^= 1;
 }
 
-template <bool CODES, int K>
-__device__ __forceinline__ void spread_cross(SpreadFFT& f, fxc (&x)[K], int (&h)[K]) {
-  switch (f.M >> 5) {
-    case 2: spread_cross_g<2, CODES>(f, x, h); break;
-    case 4: spread_cross_g<4, CODES>(f, x, h); break;
-    case 8: spread_cross_g<8, CODES>(f, x, h); break;
-    case 16: spread_cross_g<16, CODES>(f, x, h); break;
-    default: break;   // one warp
-  }
-}
-
-// The push of an exchange: thread j of every CTA sends its value to column j of row `rank` in all C CTAs (and,
-// with CODES, lane v of each warp its code to CTA v).
-template <int C, bool CODES, int K>
-__device__ __forceinline__ void spread_push(SpreadFFT& f, const fxc (&y)[K], const int (&h)[K]) {
+// C-point DFT over the cluster's CTAs, in two halves.  Push: thread j of every CTA sends its value to column j of
+// row `rank` in all C CTAs.
+template <int C, int K>
+__device__ __forceinline__ void spread_push(SpreadFFT& f, const fxc (&y)[K]) {
   static_assert(C == 4 || C == 8 || C == 16, "four, eight or sixteen CTAs");
-  const int M = f.M, G = M >> 5;
+  const int M = f.M;
   const unsigned bar = f.bar + 8 * f.phase;
   const unsigned dst = spread_saddr(f.recv + ((long long)f.phase * C + f.rank) * K * M + f.j);
   if (f.l == 0)
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar),
-                 "r"(C * K * (32 * 16 + (CODES ? 4 : 0)))
-                 : "memory");
-  int4 out[K];
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(C * K * 32 * 16) : "memory");
 #pragma unroll
-  for (int m = 0; m < K; m++) out[m] = fx_pack(y[m]);
+  for (int m = 0; m < K; m++) {
+    const int4 out = fx_pack(y[m]);
 #pragma unroll
-  for (int v = 0; v < C; v++) {
-    unsigned rd, rb;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(rd) : "r"(dst), "r"(f.base + v));
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(rb) : "r"(bar), "r"(f.base + v));
-#pragma unroll
-    for (int m = 0; m < K; m++)
-      asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(
-                       rd + 16 * m * M),
-                   "r"(out[m].x), "r"(out[m].y), "r"(out[m].z), "r"(out[m].w), "r"(rb)
+    for (int v = 0; v < C; v++) {
+      unsigned rd, rb;
+      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(rd) : "r"(dst + 16 * m * M), "r"(f.base + v));
+      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(rb) : "r"(bar), "r"(f.base + v));
+      asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(rd),
+                   "r"(out.x), "r"(out.y), "r"(out.z), "r"(out.w), "r"(rb)
                    : "memory");
-  }
-  if (CODES && f.l < C) {
-    const unsigned cd = spread_saddr(f.rcode + (f.phase * C + f.rank) * K * G + f.g);
-    unsigned rd, rb;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(rd) : "r"(cd), "r"(f.base + f.l));
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(rb) : "r"(bar), "r"(f.base + f.l));
-#pragma unroll
-    for (int m = 0; m < K; m++)
-      asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(rd + 4 * m * G),
-                   "r"(h[m]), "r"(rb)
-                   : "memory");
+    }
   }
 }
 
-// The other half: the C values of this thread's column, combined into output `rank` of their C-point DFT.
-template <int C, bool CODES, int K>
-__device__ __forceinline__ void spread_pull(SpreadFFT& f, fxc (&y)[K], int (&h)[K]) {
-  const int M = f.M, G = M >> 5;
-  const int4* half = f.recv + (long long)f.phase * C * K * M;
-  const int* cd = f.rcode + f.phase * C * K * G;
-  spread_wait(f);
+// Pull: the C values of this thread's column, combined into output `rank` of their C-point DFT.
+template <int C, int K>
+__device__ __forceinline__ void spread_pull(SpreadFFT& f, fxc (&y)[K]) {
+  const int4* half = f.recv + (long long)f.phase * C * K * f.M;
+  spread_wait(f, f.bar + 8 * f.phase, f.phase);
 #pragma unroll
-  for (int m = 0; m < K; m++) {
-    int hs[C], r[C];
-    fxc v[C];
-    if constexpr (CODES) {
-#pragma unroll
-      for (int c = 0; c < C; c++) hs[c] = cd[(c * K + m) * G + f.g];
-      h[m] = spread_total<C>(hs, r);
-    }
-#pragma unroll
-    for (int c = 0; c < C; c++) {
-      v[c] = fx_unpack(half[((long long)c * K + m) * M + f.j]);
-      if constexpr (CODES) v[c] = spread_align(v[c], r[c]);
-    }
-    y[m] = spread_combine<C>(v, f.rank, f.twM, M);
-  }
+  for (int m = 0; m < K; m++) y[m] = spread_gather<C>(half + m * f.M + f.j, K * f.M, f.rank, f.twM, f.M);
   f.phase ^= 1;
 }
 
 // a w / 2^s
 __device__ __forceinline__ fxc spread_mul(fxc a, int4 w, int s) { return fx_cmul(a, w, 2 - s); }
+
+// The warps' codes over the cluster: lane v sends the warp's to CTA v, and every warp then knows all C G of them and
+// shifts its values to the exponent of the total once.  A forward transform sends them before its warp DFTs and
+// needs them after.  The halves of ecode alternate; a warp writes half n again after code exchange n + 1, for which
+// every warp of the cluster has read half n.
+template <int C, int K>
+__device__ __forceinline__ void spread_push_codes(SpreadFFT& f, const int (&h)[K]) {
+  const int G = f.M >> 5;
+  const unsigned bar = f.ebar + 8 * f.ephase;
+  if (f.j == 0)
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(C * K * G * 4) : "memory");
+  if (f.l < C) {
+    const unsigned cd = spread_saddr(f.ecode + ((f.ephase * K) * C + f.rank) * G + f.g);
+    unsigned rd, rb;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(rd) : "r"(cd), "r"(f.base + f.l));
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(rb) : "r"(bar), "r"(f.base + f.l));
+#pragma unroll
+    for (int m = 0; m < K; m++)
+      asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(rd + 4 * m * C * G),
+                   "r"(h[m]), "r"(rb)
+                   : "memory");
+  }
+}
+
+// The code of the total of n <= 32 Q warps' codes (lane l takes l, l + 32, ...).
+template <int Q>
+__device__ __forceinline__ int spread_total(const int* cd, int n, int l) {
+  int v[Q], top = kSpreadZero;
+#pragma unroll
+  for (int q = 0; q < Q; q++) {
+    v[q] = l + 32 * q < n ? cd[l + 32 * q] : kSpreadZero;
+    top = max(top, v[q]);
+  }
+  top = __reduce_max_sync(0xffffffffu, top);
+  unsigned s = 0;
+#pragma unroll
+  for (int q = 0; q < Q; q++)
+    if (l + 32 * q < n) s += 65536u >> min(top - v[q], 31);
+  s = __reduce_add_sync(0xffffffffu, s);
+  return top + 16 - __clz((int)(s - 1));   // top + ceil(log2(s / 65536))
+}
+
+template <int C, int K>
+__device__ __forceinline__ void spread_pull_codes(SpreadFFT& f, fxc (&y)[K], int (&h)[K]) {
+  const int n = C * (f.M >> 5);
+  const int* cd = f.ecode + f.ephase * K * n;
+  spread_wait(f, f.ebar + 8 * f.ephase, 2 + f.ephase);
+  f.ephase ^= 1;
+#pragma unroll
+  for (int m = 0; m < K; m++) {
+    const int tot = spread_total<C == 4 ? 2 : 4>(cd + m * n, n, f.l);   // at most 16 warps per CTA, 128 per cluster
+    y[m] = spread_align(y[m], min(((tot + 1) >> 1) - ((h[m] + 1) >> 1), 62));
+    h[m] = tot;
+  }
+}
 
 // time-domain ownership -> frequency-domain ownership, K fields together.  Returns in `places` the shifts so far:
 // y = X 2^(A0 - ceil(h / 2) - places), h the cluster's code, the norm at most `level` half bits above 2^A0.
@@ -379,33 +382,42 @@ __device__ __forceinline__ void spread_forward(SpreadFFT& f, const double2 (&x)[
   const int g = 26 - __clz(f.M), lc = fx_log2(C);   // log2 G: the half bits a G-point DFT adds (M = 32 G)
   const int s1 = spread_shift(5, g), s2 = spread_shift(5 + g - 2 * s1, lc);
 #pragma unroll
-  for (int m = 0; m < K; m++) h[m] = spread_enter(x[m], y[m]);
-  spread_warp_dft<K>(f, y);
+  for (int m = 0; m < K; m++) {
+    const SpreadPoint p = spread_enter(x[m]);
+    y[m] = p.y;
+    h[m] = p.h;
+  }
+  spread_push_codes<C, K>(f, h);
+#pragma unroll
+  for (int m = 0; m < K; m++) y[m] = spread_warp_dft(y[m], f.w16, f.w8, f.w4, f.l);
+  spread_pull_codes<C, K>(f, y, h);
 #pragma unroll
   for (int m = 0; m < K; m++) y[m] = f.g > 0 ? spread_mul(y[m], f.wgl, s1) : fx_shift(y[m], s1);
-  spread_cross<true, K>(f, y, h);
+  spread_cross<K>(f, y);
 #pragma unroll
   for (int m = 0; m < K; m++) y[m] = spread_mul(y[m], f.twC, s2);
-  spread_push<C, true, K>(f, y, h);
-  spread_pull<C, true, K>(f, y, h);
+  spread_push<C, K>(f, y);
+  spread_pull<C, K>(f, y);
   places = s1 + s2;
   level = 5 + g - 2 * s1 + lc - 2 * s2;
 }
 
 // The inverse transform's part after its push (of swapped values): pull, DFT across the warps, in the warps.
-// CODES: the warps' codes travel with the values; otherwise h is the cluster's.  level: of the pushed values.
-template <int C, bool CODES, int K>
-__device__ __forceinline__ void spread_backward(SpreadFFT& f, fxc (&y)[K], int (&h)[K], int& places, int level) {
+// level: of the pushed values.
+template <int C, int K>
+__device__ __forceinline__ void spread_backward(SpreadFFT& f, fxc (&y)[K], int& places, int level) {
   const int g = 26 - __clz(f.M), lc = fx_log2(C);
   // the last product shifts two places at most: the one before it takes what that leaves
   const int s1 = max(0, (level + lc + g - 3) >> 1), s2 = spread_shift(level + lc + g - 2 * s1, 5);
-  spread_pull<C, CODES, K>(f, y, h);
+  spread_pull<C, K>(f, y);
 #pragma unroll
   for (int m = 0; m < K; m++) y[m] = spread_mul(y[m], f.twC, s1);
-  spread_cross<CODES, K>(f, y, h);
+  spread_cross<K>(f, y);
 #pragma unroll
-  for (int m = 0; m < K; m++) y[m] = f.g > 0 ? spread_mul(y[m], f.wgl, s2) : fx_shift(y[m], s2);
-  spread_warp_dft<K>(f, y);
+  for (int m = 0; m < K; m++) {
+    y[m] = f.g > 0 ? spread_mul(y[m], f.wgl, s2) : fx_shift(y[m], s2);
+    y[m] = spread_warp_dft(y[m], f.w16, f.w8, f.w4, f.l);
+  }
   places += s1 + s2;
 }
 
@@ -426,13 +438,16 @@ __device__ __forceinline__ void spread_inv_store_k(SpreadFFT& f, double2 (&x)[K]
   int h[K], places = 0;
 #pragma unroll
   for (int m = 0; m < K; m++) {
-    h[m] = spread_enter(x[m], y[m]);
-    y[m] = spread_swap(y[m]);
+    const SpreadPoint p = spread_enter(x[m]);
+    y[m] = spread_swap(p.y);
+    h[m] = p.h;
   }
-  spread_push<C, true, K>(f, y, h);
+  spread_push_codes<C, K>(f, h);
+  spread_pull_codes<C, K>(f, y, h);
+  spread_push<C, K>(f, y);
 #pragma unroll
   for (int m = 0; m < K; m++) store(m, x[m]);
-  spread_backward<C, true, K>(f, y, h, places, 0);
+  spread_backward<C, K>(f, y, places, 0);
 #pragma unroll
   for (int m = 0; m < K; m++) x[m] = spread_leave(spread_swap(y[m]), h[m], places);
 }
@@ -452,12 +467,12 @@ __device__ __forceinline__ void spread_pair_k(SpreadFFT& f, double2 (&x)[K], con
 #pragma unroll
   for (int m = 0; m < K; m++) y[m] = spread_swap(spread_mul(y[m], fac[m], s));
   places += s;
-  spread_push<C, false, K>(f, y, h);
+  spread_push<C, K>(f, y);
   if (want) {
 #pragma unroll
     for (int m = 0; m < K; m++) spec(m, spread_leave(spread_swap(y[m]), h[m], places + et));
   }
-  spread_backward<C, false, K>(f, y, h, places, level - 2 * s);
+  spread_backward<C, K>(f, y, places, level - 2 * s);
 #pragma unroll
   for (int m = 0; m < K; m++) x[m] = spread_leave(spread_swap(y[m]), h[m], places + et);
 }
@@ -506,6 +521,35 @@ __device__ __forceinline__ int4 fx_factor(double2 v) {
   fx_split(y, r.z, r.w);
   return r;
 }
+// The same out of line, for the ends of a march: the state travels by value, so that the march's copy stays in
+// registers.
+struct SpreadCall {
+  SpreadFFT f;
+  double2 x;
+};
+template <int C>
+__device__ __noinline__ SpreadCall spread_fwd_call(SpreadFFT f, double2 x) {
+  x = spread_fwd<C>(f, x);
+  return SpreadCall{f, x};
+}
+template <int C>
+__device__ __noinline__ SpreadCall spread_inv_call(SpreadFFT f, double2 x) {
+  x = spread_inv<C>(f, x);
+  return SpreadCall{f, x};
+}
+template <int C = kSpreadC>
+__device__ __forceinline__ double2 spread_fwd_end(SpreadFFT& f, double2 x) {
+  const SpreadCall r = spread_fwd_call<C>(f, x);
+  f.sel = r.f.sel, f.phase = r.f.phase, f.ephase = r.f.ephase, f.parity = r.f.parity, f.dead = r.f.dead;
+  return r.x;
+}
+template <int C = kSpreadC>
+__device__ __forceinline__ double2 spread_inv_end(SpreadFFT& f, double2 x) {
+  const SpreadCall r = spread_inv_call<C>(f, x);
+  f.sel = r.f.sel, f.phase = r.f.phase, f.ephase = r.f.ephase, f.parity = r.f.parity, f.dead = r.f.dead;
+  return r.x;
+}
+
 __device__ __forceinline__ int4 fx_conj(int4 w) { return make_int4(w.x, w.y, -w.z, -w.w); }
 
 }  // namespace nlm

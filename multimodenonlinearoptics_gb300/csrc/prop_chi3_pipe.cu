@@ -34,9 +34,10 @@ __global__ void __launch_bounds__(kMaxThreads) k_chi3_pump_signal_spread(const P
   if (role == 0) {
     const double invN = 1.0 / N;
     const int4 dp = fx_factor(p.dstepP[fk]);
-    double2 x = spread_fwd(f, p.env[tn]);
+    double2 x = spread_fwd_end(f, p.env[tn]);
     x = cmul(x, p.halfP[fk]);
-    x = cscale(spread_inv_store(f, x, [&](double2 v) { p.pf[fk] = v; }), invN);
+    p.pf[fk] = x;
+    x = cscale(spread_inv_end(f, x), invN);
     p.pt[tn] = x;
     for (int i = 1; i < p.nRows; i++) {
       const double2 r = p.rel[i - 1];
@@ -49,18 +50,18 @@ __global__ void __launch_bounds__(kMaxThreads) k_chi3_pump_signal_spread(const P
     // last row: undo half of the last pump dispersion step (each thread rereads its own bin)
     const long long last = (long long)(p.nRows - 1) * N;
     x = cmul(p.pf[last + fk], p.backP[fk]);
-    p.pt[last + tn] = cscale(spread_inv_store(f, x, [&](double2 v) { p.pf[last + fk] = v; }), invN);
+    p.pf[last + fk] = x;
+    p.pt[last + tn] = cscale(spread_inv_end(f, x), invN);
     cl.sync();
     cl.sync();
     return;
   }
   const long long inst = a.instBase;
   double2 x = a.in[inst * a.inStride + (a.inTime ? tn : fk)];
-  if (a.inTime) x = spread_fwd(f, x);
+  if (a.inTime) x = spread_fwd_end(f, x);
   x = cmul(x, __ldg(a.half + fk));
-  x = spread_inv_store(f, x, [&](double2 v) {
-    if (a.gridF) a.gridF[fk] = cscale(v, (double)N);
-  });
+  if (a.gridF) a.gridF[fk] = cscale(x, (double)N);
+  x = spread_inv_end(f, x);
   if (a.gridT) a.gridT[tn] = x;
   // step i: the DiffEq with pump rows 2i-2 .. 2i (plain loads: the pump group writes them during this
   // launch), then the dispersion step
@@ -79,7 +80,7 @@ __global__ void __launch_bounds__(kMaxThreads) k_chi3_pump_signal_spread(const P
       x = spread_pair_spec(f, xm[0], __ldg(a.fx.tab + (last ? N : 0) + fk), a.fx.et, a.gridF != nullptr, storeF);
       if (a.gridT) a.gridT[(long long)i * N + tn] = x;
     } else {
-      x = cmul(spread_fwd(f, xm[0]), __ldg(a.dlast + fk));
+      x = cmul(spread_fwd_end(f, xm[0]), __ldg(a.dlast + fk));
       storeF(x);
     }
   }

@@ -34,12 +34,11 @@ __global__ void __launch_bounds__(C == 16 ? 256 : kMaxThreads) k_propagate_gnlse
     const double2* row = a.in + inst * a.inStride;
     const bool has = a.inputMode == 0 || (a.inputMode < 1 && a.inChannels > 0);
     double2 x = has ? row[a.inTime ? tn : fk] : czero();
-    if (a.inTime) x = spread_fwd<C>(f, x);
+    if (a.inTime) x = spread_fwd_end<C>(f, x);
     x = cmul(x, __ldg(a.half + fk));
     double2 xf = x;   // the state's spectrum (whose unscaled inverse transform is x)
-    x = spread_inv_store<C>(f, x, [&](double2 v) {
-      if (a.gridF) a.gridF[fk] = cscale(v, (double)N);
-    });
+    if (a.gridF) a.gridF[fk] = cscale(x, (double)N);
+    x = spread_inv_end<C>(f, x);
     if (a.gridT) a.gridT[tn] = x;
     // checkpoints for the reverse sweep: the time-domain state before steps 1, K + 1, 2 K + 1, ...
     double2* ckRow = a.ckpt ? a.ckpt + inst * a.ckN * (long long)N : nullptr;
@@ -84,10 +83,10 @@ __global__ void __launch_bounds__(C == 16 ? 256 : kMaxThreads) k_propagate_gnlse
       }
     }
     if (a.nZ == 1) {
-      x = cmul(spread_fwd<C>(f, x), __ldg(a.back + fk));
+      x = cmul(spread_fwd_end<C>(f, x), __ldg(a.back + fk));
       if (a.gridF) a.gridF[fk] = cscale(x, (double)N);
       if (a.inTime || a.gridT) {
-        x = spread_inv<C>(f, x);
+        x = spread_inv_end<C>(f, x);
         if (a.gridT) a.gridT[tn] = x;
       }
     }

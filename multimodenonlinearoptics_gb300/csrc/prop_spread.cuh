@@ -30,9 +30,10 @@ __global__ void __launch_bounds__(kMaxThreads) k_pump_chi3_spread(double2* __res
   const double invN = 1.0 / N;
   const int et = -(31 - __clz(N));        // the inverse transform's 1/N
   const int4 dp = fx_factor(dstepP[fk]);
-  double2 x = spread_fwd<C>(f, env[tn]);
+  double2 x = spread_fwd_end<C>(f, env[tn]);
   x = cmul(x, halfP[fk]);
-  x = cscale(spread_inv_store<C>(f, x, [&](double2 v) { pf[fk] = v; }), invN);
+  pf[fk] = x;
+  x = cscale(spread_inv_end<C>(f, x), invN);
   pt[tn] = x;
   for (int i = 1; i < nRows; i++) {
     const double2 r = rel[i - 1];
@@ -45,46 +46,51 @@ __global__ void __launch_bounds__(kMaxThreads) k_pump_chi3_spread(double2* __res
   // last row: undo half of the last pump dispersion step (each thread rereads its own bin)
   const long long last = (long long)(nRows - 1) * N;
   x = cmul(pf[last + fk], backP[fk]);
-  pt[last + tn] = cscale(spread_inv_store<C>(f, x, [&](double2 v) { pf[last + fk] = v; }), invN);
+  pf[last + fk] = x;
+  pt[last + tn] = cscale(spread_inv_end<C>(f, x), invN);
   cl.sync();
 }
 
-// All MD modes: time -> frequency domain; K = MD together, K = 1 one after another.
-template <int C, int K, int MD>
-__device__ __forceinline__ void spread_fwd_all(SpreadFFT& f, double2 (&x)[MD]) {
-  if constexpr (K > 1) {
-    spread_fwd_k<C, MD>(f, x);
-  } else {
+// The modes one place on, the first one last.
+template <class T, int MD>
+__device__ __forceinline__ void spread_turn(T (&x)[MD]) {
+  const T t = x[0];
 #pragma unroll
-    for (int m = 0; m < MD; m++) x[m] = spread_fwd<C>(f, x[m]);
+  for (int q = 0; q < MD - 1; q++) x[q] = x[q + 1];
+  x[MD - 1] = t;
+}
+
+// All MD modes, one after another: time -> frequency domain and back (the ends of a march).
+template <int C, int MD>
+__device__ __forceinline__ void spread_fwd_all(SpreadFFT& f, double2 (&x)[MD]) {
+#pragma unroll 1
+  for (int m = 0; m < MD; m++) {   // mode m sits in x[0] during its turn
+    x[0] = spread_fwd_end<C>(f, x[0]);
+    spread_turn(x);
   }
 }
 
-// All MD modes: frequency -> time domain, store(m, v) given each mode's spectrum after its exchange.
-template <int C, int K, int MD, class Store>
-__device__ __forceinline__ void spread_inv_all(SpreadFFT& f, double2 (&x)[MD], Store store) {
-  if constexpr (K > 1) {
-    spread_inv_store_k<C, MD>(f, x, store);
-  } else {
-#pragma unroll
-    for (int m = 0; m < MD; m++) {
-      const int mm = m;
-      x[m] = spread_inv_store<C>(f, x[m], [&](double2 v) { store(mm, v); });
-    }
+template <int C, int MD>
+__device__ __forceinline__ void spread_inv_all(SpreadFFT& f, double2 (&x)[MD]) {
+#pragma unroll 1
+  for (int m = 0; m < MD; m++) {
+    x[0] = spread_inv_end<C>(f, x[0]);
+    spread_turn(x);
   }
 }
 
 // All MD modes through the dispersion pair.
 template <int C, int K, int MD, class Spec>
-__device__ __forceinline__ void spread_pair_all(SpreadFFT& f, double2 (&x)[MD], const int4 (&fac)[MD], int et, bool want,
+__device__ __forceinline__ void spread_pair_all(SpreadFFT& f, double2 (&x)[MD], int4 (&fac)[MD], int et, bool want,
                                                 Spec spec) {
   if constexpr (K > 1) {
     spread_pair_k<C, MD>(f, x, fac, et, want, spec);
   } else {
-#pragma unroll
+#pragma unroll 1
     for (int m = 0; m < MD; m++) {
-      const int mm = m;
-      x[m] = spread_pair_spec<C>(f, x[m], fac[m], et, want, [&](double2 v) { spec(mm, v); });
+      x[0] = spread_pair_spec<C>(f, x[0], fac[0], et, want, [&](double2 v) { spec(m, v); });
+      spread_turn(x);
+      spread_turn(fac);
     }
   }
 }
@@ -121,12 +127,14 @@ __global__ void __launch_bounds__(kMaxThreads) k_propagate_spread(const PropArgs
       else if (a.inputMode < 1 && m < a.inChannels) seg = m;
       x[m] = seg >= 0 ? row[(long long)seg * N + (a.inTime ? tn : fk)] : czero();
     }
-    if (a.inTime) spread_fwd_all<C, K, MD>(f, x);
+    if (a.inTime) spread_fwd_all<C, MD>(f, x);
 #pragma unroll
     for (int m = 0; m < MD; m++) x[m] = cmul(x[m], __ldg(a.half + (long long)m * N + fk));
-    spread_inv_all<C, K, MD>(f, x, [&](int m, double2 v) {
-      if (a.gridF) a.gridF[m * ms + fk] = cscale(v, (double)N);
-    });
+    if (a.gridF) {
+#pragma unroll
+      for (int m = 0; m < MD; m++) a.gridF[m * ms + fk] = cscale(x[m], (double)N);
+    }
+    spread_inv_all<C, MD>(f, x);
     if (a.gridT) {
 #pragma unroll
       for (int m = 0; m < MD; m++) a.gridT[m * ms + tn] = x[m];
@@ -137,8 +145,41 @@ __global__ void __launch_bounds__(kMaxThreads) k_propagate_spread(const PropArgs
 #pragma unroll
       for (int m = 0; m < MD; m++) ckRow[(long long)m * N + tn] = x[m];
     }
-    for (int i = 1; i < a.nZ; i++) {
+    // What a step reads is loaded during the step before (a load from L2 takes a fifth of a step): the dispersion
+    // factors once, the RK4 matrix of a single mode, or the pump rows.
+    constexpr bool kAhead = MD == 1;
+    constexpr int kWords = kAhead ? 2 : 1;
+    int4 fac[MD];
+    if (a.nZ > 1) {
+#pragma unroll
+      for (int m = 0; m < MD; m++) fac[m] = __ldg(a.fx.tab + (long long)m * N + fk);
+    }
+    double2 ahead[kWords], rows[3][P];
+    auto loadMatrix = [&](int i) {
+      const double2* mat = reinterpret_cast<const double2*>(a.prop) + (long long)(i - 1) * 2 * N + tn;
+#pragma unroll
+      for (int w = 0; w < kWords; w++) ahead[w] = __ldg(mat + (long long)w * N);
+    };
+    auto loadRow = [&](int row, int at) {
+#pragma unroll
+      for (int q = 0; q < P; q++)
+        rows[at][q] = S::kP > 0 ? __ldg(a.pump + q * a.pumpStride + (long long)row * N + tn) : czero();
+    };
+    if (a.nZ > 1) {
       if (a.prop) {
+        if (kAhead) loadMatrix(1);
+      } else {
+        loadRow(0, 0);
+        loadRow(1, 1);
+        loadRow(2, 2);
+      }
+    }
+    for (int i = 1; i < a.nZ; i++) {
+      if (kAhead && a.prop) {
+        const double2 e0 = ahead[0], e1 = ahead[kWords - 1], v = x[0];
+        x[0] = make_double2(fma(e0.y, v.y, e0.x * v.x), fma(e1.y, v.y, e1.x * v.x));
+        if (i < a.nZ - 1) loadMatrix(i + 1);
+      } else if (a.prop) {
         // the RK4 step as its per-point real (2M)x(2M) matrix, stored as pairs (row r, columns 2c and
         // 2c+1) at [step][r * M + c][N]
         constexpr int D = 2 * MD;
@@ -164,19 +205,13 @@ __global__ void __launch_bounds__(kMaxThreads) k_propagate_spread(const PropArgs
         for (int m = 0; m < MD; m++) x[m] = make_double2(outv[2 * m], outv[2 * m + 1]);
       } else {
         const double2* c = a.coef + (long long)(i - 1) * 3 * a.nCoef;
-        double2 p[3][P];
+        rk4_point<S>(x, rows, c);
+        if (i < a.nZ - 1) {   // row 2i is the next step's first
 #pragma unroll
-        for (int q = 0; q < P; q++) {
-          if (S::kP > 0) {
-            const double2* pr = a.pump + q * a.pumpStride + (long long)(2 * i - 2) * N + tn;
-            p[0][q] = __ldg(pr);
-            p[1][q] = __ldg(pr + N);
-            p[2][q] = __ldg(pr + 2 * N);
-          } else {
-            p[0][q] = p[1][q] = p[2][q] = czero();
-          }
+          for (int q = 0; q < P; q++) rows[0][q] = rows[2][q];
+          loadRow(2 * i + 1, 1);
+          loadRow(2 * i + 2, 2);
         }
-        rk4_point<S>(x, p, c);
       }
       const bool last = i == a.nZ - 1;
       const bool wantTime = !last || a.inTime || a.gridT != nullptr;
@@ -184,16 +219,17 @@ __global__ void __launch_bounds__(kMaxThreads) k_propagate_spread(const PropArgs
         if (a.gridF) a.gridF[m * ms + (long long)i * N + fk] = cscale(v, (double)N);
       };
       if (wantTime) {
-        int4 fac[MD];
+        if (last) {
 #pragma unroll
-        for (int m = 0; m < MD; m++) fac[m] = __ldg(a.fx.tab + (long long)((last ? MD : 0) + m) * N + fk);
+          for (int m = 0; m < MD; m++) fac[m] = __ldg(a.fx.tab + (long long)(MD + m) * N + fk);
+        }
         spread_pair_all<C, K, MD>(f, x, fac, a.fx.et, a.gridF != nullptr, storeF);
         if (a.gridT) {
 #pragma unroll
           for (int m = 0; m < MD; m++) a.gridT[m * ms + (long long)i * N + tn] = x[m];
         }
       } else {
-        spread_fwd_all<C, K, MD>(f, x);
+        spread_fwd_all<C, MD>(f, x);
 #pragma unroll
         for (int m = 0; m < MD; m++) {
           x[m] = cmul(x[m], __ldg(a.dlast + (long long)m * N + fk));
@@ -206,14 +242,14 @@ __global__ void __launch_bounds__(kMaxThreads) k_propagate_spread(const PropArgs
       }
     }
     if (a.nZ == 1) {
-      spread_fwd_all<C, K, MD>(f, x);
+      spread_fwd_all<C, MD>(f, x);
 #pragma unroll
       for (int m = 0; m < MD; m++) {
         x[m] = cmul(x[m], __ldg(a.back + (long long)m * N + fk));
         if (a.gridF) a.gridF[m * ms + fk] = cscale(x[m], (double)N);
       }
       if (a.inTime || a.gridT) {
-        spread_inv_all<C, K, MD>(f, x, [&](int, double2) {});
+        spread_inv_all<C, MD>(f, x);
         if (a.gridT) {
 #pragma unroll
           for (int m = 0; m < MD; m++) a.gridT[m * ms + tn] = x[m];
