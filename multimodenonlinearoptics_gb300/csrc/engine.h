@@ -198,7 +198,7 @@ inline void add_prop_key(GraphKey& k, const PropArgs& a) {
   k.add(a.out).add(a.outStride).add(a.tw).add(a.dstep).add(a.dlast).add(a.half).add(a.back).add(a.prop);
   k.add(a.pump).add(a.pumpStride).add(a.nPumps).add(a.coef).add(a.nCoef).add(a.gridF).add(a.gridT);
   k.add(a.ckpt).add(a.ckK).add(a.ckN).add(a.stages).add(a.raman).add(a.steep).add(a.relInt);
-  k.add(a.fx.tw).add(a.fx.twN).add(a.fx.tab).add(a.fx.et).add(a.fx.raman).add(a.fx.steep).add(a.fx.etRaman).add(a.fx.etSteep).add(a.fx.A0).add(a.fx.sh).add(a.fx.ls);
+  k.add(a.fx.tw).add(a.fx.root).add(a.fx.twN).add(a.fx.tab).add(a.fx.et).add(a.fx.raman).add(a.fx.steep).add(a.fx.etRaman).add(a.fx.etSteep).add(a.fx.A0).add(a.fx.sh).add(a.fx.ls);
 }
 
 struct GraphCache {
@@ -340,6 +340,13 @@ struct FxTwiddleCache {
         L *= r;
       }
       h.resize(p.N);   // the kernels stage N entries
+    });
+  }
+  // exp(-2 pi i q / r), q < r, for r = 3, 5, 7 (fx_root_at)
+  const int4* roots(cudaStream_t s) {
+    return find({0}, s, [](std::vector<int4>& h) {
+      for (int r : {3, 5, 7})
+        for (int q = 0; q < r; q++) h.push_back(root(q, r));
     });
   }
   // exp(-2 pi i m / N) for m < N
@@ -720,6 +727,7 @@ struct Medium {
   // block fixed-point tables (dispStep, last, half) and their exponent; empty on grids without them
   DevBuf<int4> fxTab, fxRaman, fxSteep;
   const int4* spreadTwD = nullptr;
+  const int4* fxRoots = nullptr;
   int fxEtRaman = 0, fxEtSteep = 0;
   bool fxBad = false;   // a table has values that are not finite: only the FP64 kernels take this medium
   int fxEt = 0;
@@ -920,8 +928,9 @@ struct Medium {
     upload(half, hh);
     upload(back, hb);
     if (fxSize()) spreadTwD = g_fxTwiddles.natural((int)N, stream);
+    else if (fxGenSize()) fxRoots = g_fxTwiddles.roots(stream);
     // a single z step has an infinite step length, and tables that are not finite: FP64 kernels
-    if (fxSize() && nZ > 1 && std::isfinite(dz)) {
+    if ((fxSize() || fxGenSize()) && nZ > 1 && std::isfinite(dz)) {
       std::vector<double2> all(hd);
       all.insert(all.end(), hl.begin(), hl.end());
       all.insert(all.end(), hh.begin(), hh.end());
@@ -1501,8 +1510,9 @@ struct Medium {
   // default enough for 128 threads, times ipcMul), `cta` resident CTAs per SM (0: the member
   // override or the occupancy maximum), grid = SMs x CTAs per SM, capped by the number of groups.
   Schedule schedule(const KernelEntry* k, long long nInst, int R, int cta = 0, int ipcMul = 1) {
-    const int T = ((int)N + R - 1) / R;   // N / R on the register plan, ceil(N / R) on the general one
+    int T = ((int)N + R - 1) / R;   // N / R on the register plan, ceil(N / R) on the general one
     const bool fx = k->kind == kKindFxLinear || k->kind == kKindFxDirect || k->kind == kKindFxGnlse;
+    if (fx && !is_pow2((int)N)) T = fxGenPlan(R).T;
     int ipc = fx ? 1 : (T >= 128 ? 1 : 128 / T) * ipcMul;
     if (ipc > nInst) ipc = (int)std::max<long long>(1, nInst);
     const int block = T * ipc;
@@ -1696,7 +1706,21 @@ struct Medium {
   // Grids whose one-CTA kernels run them: whole warps of 4 or 8 points per thread, at most 512 threads.
   static constexpr uint kFxMinN = 128, kFxMaxN = 4096;
   bool fxSize() const { return is_pow2((int)N) && N >= kFxMinN && N <= kFxMaxN; }
-  bool fxGrid() const { return fxSize() && fxTab.p && (solver != kChi3GNLSE || (fxRaman.p && fxSteep.p)); }
+  // other grids whose prime factors the kernels have passes for
+  bool fxGenSize() const {
+    if (is_pow2((int)N) || N % 2 != 0 || N < 64 || N > kFxMaxN) return false;
+    uint n = N;
+    for (uint q : {2u, 3u, 5u, 7u})
+      while (n % q == 0) n /= q;
+    return n == 1;
+  }
+  // the general plan with whole warps (padding a grid's last warps)
+  FFTPlanH fxGenPlan(int R) const {
+    FFTPlanH p = make_plan_gen((int)N, R);
+    p.T = 32 * (((int)N + 32 * R - 1) / (32 * R));
+    return p;
+  }
+  bool fxGrid() const { return fxTab.p && (solver != kChi3GNLSE || (fxRaman.p && fxSteep.p)); }
   // the N-point twiddles of the one-point-per-thread cluster kernels (null on grids without them)
   const int4* spreadTw() const { return spreadTwD; }
   int log2N() const { return (int)std::lround(std::log2((double)N)); }
@@ -1714,14 +1738,22 @@ struct Medium {
     f.etRaman = fxEtRaman;
     f.etSteep = fxEtSteep;
     f.err = g_exchange.flag();
+    f.root = fxRoots;
     int level = 0;   // half bits
     for (int i = 0; i < p.nPass; i++) {
-      const int s = i == 0 ? 0 : fx_pass_shift(level, p.radix[i]);
-      f.sh += s;
-      level += fx_log2(p.radix[i]) - 2 * s;
+      const int r = p.radix[i];
+      if (r & 1) {
+        const int s = fx_odd_shift(level);
+        f.sh += s + 2;
+        level += fx_half_bits(r) - 4 - 2 * s;
+      } else {
+        const int s = i == 0 ? 0 : fx_pass_shift(level, r);
+        f.sh += s;
+        level += fx_log2(r) - 2 * s;
+      }
     }
     f.A0 = 60;
-    f.ls = 2 - (level + 1) / 2;
+    f.ls = 2 - (level >= 0 ? (level + 1) / 2 : -((-level) / 2));   // 2 - ceil(level / 2)
     return f;
   }
 
@@ -1730,7 +1762,8 @@ struct Medium {
     // in registers, four where 512 threads hold the grid
     for (int q : {0, 1}) {
       const int r = (nSignal == 1) == (q == 0) ? 8 : 4;
-      if (N / r < 32 || N / r > 512) continue;
+      const int T = is_pow2((int)N) ? (int)N / r : fxGenPlan(r).T;
+      if (T < 32 || T > 512) continue;
       if (const KernelEntry* k = findKernel(kind, key, r)) {
         *R = r;
         return k;
@@ -2057,7 +2090,15 @@ struct Medium {
     if (gen) {
       if (a.ckpt) throw Unsupported("the adjoint's forward takes power-of-two grids (register plan) only");
       int Rg = R;
-      if (!gnlse && allowPropagator && wantPropagator(nInst)) {
+      const bool fx = fxGenSize() && fxGrid() && !plainOne;
+      if (fx && !gnlse && allowPropagator && wantPropagator(nInst) &&
+          (k = fxKernel(kKindFxLinear, (int)nSignal + kGenKey, &Rg))) {
+        buildPropagator(R);
+        a.prop = prop.p;
+      }
+      if (!k && fx && (gnlse || !(allowPropagator && wantPropagator(nInst))))
+        k = fxKernel(gnlse ? kKindFxGnlse : kKindFxDirect, solver + kGenKey, &Rg);
+      if (!k && !gnlse && allowPropagator && wantPropagator(nInst)) {
         k = genKernel(kKindLinear, (int)nSignal, R, &Rg);
         if (k) {
           buildPropagator(R);
@@ -2068,7 +2109,12 @@ struct Medium {
       if (!k)
         throw Unsupported("no fused kernel for a grid of " + std::to_string(N) + " points for this solver (" +
                           std::to_string(nSignal) + " modes)");
-      a.plan = make_plan_gen((int)N, Rg);
+      if (k->kind == kKindFxLinear || k->kind == kKindFxDirect || k->kind == kKindFxGnlse) {
+        a.plan = fxGenPlan(Rg);
+        a.fx = fxArgs(a.plan);
+      } else {
+        a.plan = make_plan_gen((int)N, Rg);
+      }
       a.R = Rg;
     } else if (gnlse) {
       checkGridStrict(R);

@@ -120,23 +120,30 @@ __device__ __forceinline__ void fxdft_r(fxc (&x)[R], int u, int B) {
 // a + a / 8, so that the stride-8 writes of the first pass fall on different banks.
 __device__ __forceinline__ int fx_at(int a) { return a + (a >> 3); }
 
+// where exp(-2 pi i q / r), q < r, starts in the table of roots of the odd radices 3, 5 and 7
+__host__ __device__ constexpr int fx_root_at(int r) { return r == 3 ? 0 : r == 5 ? 3 : 8; }
+
 // NT: the grid's size where the kernel is instantiated for it (every offset is then a constant), 0 where it
 // comes with the launch.
 template <int NT>
-struct FxField {
+struct FxField {   // NT = kFxGen: a grid that is not a power of two
   int4* buf;         // two exchange buffers
   const int4* tw;    // the passes' twiddles, Q62
   uint2* red;        // one (exponent, sum) pair per warp of the group
   int n, t, j, sel, mid;
-  __device__ __forceinline__ int N() const { return NT ? NT : n; }
+  const FFTPlanH* plan;   // the general plan's radices, and its roots of unity (fx_root_at)
+  const int4* root;
+  __device__ __forceinline__ int N() const { return NT > 0 ? NT : n; }
   template <int R>
   __device__ __forceinline__ int T() const {
-    return NT ? NT / R : t;
+    return NT > 0 ? NT / R : t;
   }
+  // thread j's points that the grid has
+  __device__ __forceinline__ bool has(int at) const { return NT >= 0 || at < n; }
   // radix of the second pass where it is not the plan's main one, else 1
   template <int r>
   __device__ __forceinline__ int small() const {
-    if (!NT) return mid;
+    if (NT <= 0) return mid;
     int n2 = NT;
     while (n2 >= r && n2 % r == 0) n2 /= r;
     return n2;
@@ -250,7 +257,7 @@ __device__ __forceinline__ int fx_norm(FxField<NT>& f, const double2 (&x)[R]) {
   int E = 0;
   unsigned S = 0;
   if constexpr (NT > 0) {
-    uint2 p[NT ? NT / R / 32 : 1];
+    uint2 p[NT > 0 ? NT / R / 32 : 1];
 #pragma unroll
     for (int q = 0; q < NT / R / 32; q++) {
       p[q] = f.red[q];
@@ -295,6 +302,124 @@ __device__ __forceinline__ double fx_to(long long v, int k) {
   const unsigned long long n = ((m << (62 - p)) + 0x200u) >> 10;   // 53 bits, bit 52 set
   const int h = (int)(n >> 32) + ((1022 + p + k) << 20);
   return w ? __hiloint2double(h | (sgn & (int)0x80000000), (int)(unsigned)n) : 0.0;
+}
+
+// ---- grids that are not powers of two (NT = kFxGen) ---------------------------------------------
+// T threads (whole warps) of R points, j + v T for those below N.  The points go to an exchange buffer, every pass
+// reads one buffer and writes the other (butterfly b < N / r: inputs b + q N / r, k = b mod L, twiddle q k, outputs
+// (b - k) r + k + s L), and the result comes back to the owners.  A thread takes the butterflies b = j + u T.
+constexpr int kFxGen = -1;
+
+// sum of c[q] a[q] (Q62 constants, q < n) / 4 + acc, rounded; the cross products are folded in pairs, whose sums
+// stay below 2^63
+template <int n>
+__device__ __forceinline__ long long fx_dot(const int (&ah)[n], const int (&al)[n], const int2 (&c)[n], long long acc) {
+#pragma unroll
+  for (int q = 0; q < n; q += 2) {
+    long long m = fx_mad(al[q], c[q].x, fx_mad(ah[q], c[q].y, 1LL << 31));
+    if (q + 1 < n) m = fx_mad(al[q + 1], c[q + 1].x, fx_mad(ah[q + 1], c[q + 1].y, m));
+    acc += m >> 32;
+    acc = fx_mad(ah[q], c[q].x, acc);
+    if (q + 1 < n) acc = fx_mad(ah[q + 1], c[q + 1].x, acc);
+  }
+  return acc;
+}
+
+// r-point DFT / 4, r an odd prime.  With a_q = x_q + x_(r-q), b_q = x_q - x_(r-q), y_s and y_(r-s) are
+// x_0 + sum cos(2 pi q s / r) a_q -+ i sum sin(2 pi q s / r) b_q.  root: cos and -sin of 2 pi q / r in Q62 halves.
+template <int r>
+__device__ __forceinline__ void fx_odd_dft(fxc (&x)[r], const int4* root) {
+  constexpr int h = (r - 1) / 2;
+  int axh[h], axl[h], ayh[h], ayl[h], bxh[h], bxl[h], byh[h], byl[h];
+  fxc s0 = fx_shift(x[0], 2), sum = x[0];
+#pragma unroll
+  for (int q = 1; q <= h; q++) {
+    const fxc a = fxadd(x[q], x[r - q]), b = fxsub(x[q], x[r - q]);
+    sum = fxadd(sum, a);
+    fx_split(a.x, axh[q - 1], axl[q - 1]);
+    fx_split(a.y, ayh[q - 1], ayl[q - 1]);
+    fx_split(b.x, bxh[q - 1], bxl[q - 1]);
+    fx_split(b.y, byh[q - 1], byl[q - 1]);
+  }
+  x[0] = fx_shift(sum, 2);
+#pragma unroll
+  for (int s = 1; s <= h; s++) {
+    int2 cs[h], sn[h];
+#pragma unroll
+    for (int q = 1; q <= h; q++) {
+      const int4 w = root[(q * s) % r];
+      cs[q - 1] = make_int2(w.x, w.y);
+      sn[q - 1] = make_int2(w.z, w.w);   // -sin
+    }
+    const long long cx = fx_dot<h>(axh, axl, cs, s0.x), cy = fx_dot<h>(ayh, ayl, cs, s0.y);
+    const long long dx = fx_dot<h>(bxh, bxl, sn, 0), dy = fx_dot<h>(byh, byl, sn, 0);   // -sum sin b
+    x[s] = fxc{cx - dy, cy + dx};        // C + i D, D = -sum sin b
+    x[r - s] = fxc{cx + dy, cy - dx};
+  }
+}
+
+template <int R, int r>
+__device__ __forceinline__ void fx_gen_pass(const FxField<kFxGen>& f, const int4* __restrict__ src, int4* __restrict__ dst,
+                                            const int4* __restrict__ tw, int L, int S) {
+  constexpr int U = (R + r - 1) / r;
+  const int nb = f.n / r;
+#pragma unroll 1
+  for (int u = 0; u < U; u++) {
+    const int b = f.j + u * f.t;
+    if (b < nb) {
+      const int k = b % L;
+      fxc x[r];
+#pragma unroll
+      for (int q = 0; q < r; q++) {
+        x[q] = fx_unpack(src[fx_at(b + q * nb)]);
+        if (q > 0 && L > 1) x[q] = fx_cmul(x[q], tw[(q - 1) * L + k], 2 - S);
+      }
+      if (L > 1) x[0] = S < 0 ? fxc{x[0].x << 1, x[0].y << 1} : fx_shift(x[0], S);
+      if constexpr (r == 2 || r == 4 || r == 8) {
+        fxdft_r<r>(x, 0, 1);
+      } else {
+        fx_odd_dft<r>(x, f.root + fx_root_at(r));
+      }
+      const int base = (b - k) * r + k;
+#pragma unroll
+      for (int s = 0; s < r; s++) dst[fx_at(base + s * L)] = fx_pack(x[s]);
+    }
+  }
+}
+
+template <int R>
+__device__ __forceinline__ void fx_fft(FxField<kFxGen>& f, fxc (&x)[R]) {
+  f.sel ^= 1;
+  int4* b = f.buf + f.sel * fx_buffer(f.n);
+#pragma unroll
+  for (int v = 0; v < R; v++)
+    if (f.j + v * f.t < f.n) b[fx_at(f.j + v * f.t)] = fx_pack(x[v]);
+  int L = 1, level = 0;
+  const int4* tw = f.tw;
+#pragma unroll 1
+  for (int p = 0; p < f.plan->nPass; p++) {
+    const int r = f.plan->radix[p];
+    const bool odd = (r & 1) != 0;
+    const int S = L == 1 ? 0 : odd ? fx_odd_shift(level) : fx_pass_shift(level, r);
+    __syncthreads();
+    int4* d = f.buf + (f.sel ^ 1) * fx_buffer(f.n);
+    switch (r) {
+      case 2: fx_gen_pass<R, 2>(f, b, d, tw, L, S); break;
+      case 3: fx_gen_pass<R, 3>(f, b, d, tw, L, S); break;
+      case 4: fx_gen_pass<R, 4>(f, b, d, tw, L, S); break;
+      case 5: fx_gen_pass<R, 5>(f, b, d, tw, L, S); break;
+      case 7: fx_gen_pass<R, 7>(f, b, d, tw, L, S); break;
+      default: fx_gen_pass<R, 8>(f, b, d, tw, L, S); break;
+    }
+    level += odd ? fx_half_bits(r) - 4 - 2 * S : fx_log2(r) - 2 * S;
+    if (L > 1) tw += (r - 1) * L;
+    L *= r;
+    f.sel ^= 1;
+    b = d;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int v = 0; v < R; v++) x[v] = f.j + v * f.t < f.n ? fx_unpack(b[fx_at(f.j + v * f.t)]) : fxc{0, 0};
 }
 
 constexpr double kFxLift = 0x1p900;   // applied to fields of tiny or zero norm

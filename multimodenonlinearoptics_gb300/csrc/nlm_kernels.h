@@ -27,6 +27,7 @@ struct FFTPlanH {
 // value as balanced 32-bit halves {re high, re low, im high, im low} with value (h 2^32 + l) 2^(et - 62).
 struct FxArgs {
   const int4* tw;    // the plan's twiddles, pass by pass (one-CTA kernels)
+  const int4* root;  // exp(-2 pi i q / r) of the odd radices (fx_root_at)
   const int4* twN;   // exp(-2 pi i m / N), m < N (cluster kernels with one point per thread)
   const int4* tab;   // [dispStep, last, half][mode][N], each with its 1/N
   int et;            // exponent of the tables: 2^et is at least their largest modulus
@@ -47,6 +48,11 @@ __host__ __device__ constexpr int fx_log2(int r) { return r >= 16 ? 4 : r >= 8 ?
 __host__ __device__ constexpr int fx_pass_shift(int level, int r) {
   return level + fx_log2(r) <= kFxPeak ? 0 : (level + fx_log2(r) - kFxPeak + 1) / 2;
 }
+// Odd radices (grids that are not powers of two) shift two places in their butterfly, which works on products of
+// real constants, and the twiddles one place back (-1) where the norm leaves room.  fx_half_bits: the half bits a
+// pass adds at most, log2 r rounded up.
+__host__ __device__ constexpr int fx_half_bits(int r) { return r <= 4 ? 2 : 3; }
+__host__ __device__ constexpr int fx_odd_shift(int level) { return level + 2 <= kFxPeak ? -1 : 0; }
 
 // Shared memory of a CTA of the block fixed-point kernels: the twiddles, two exchange buffers of
 // fx_buffer(N) values and one pair of words per warp (at most 16).

@@ -21,6 +21,10 @@ void add_kernels_fx(std::vector<KernelEntry>& t) {
   NLM_FX(2, 4, 11)
   NLM_FX(2, 8, 12)
 #undef NLM_FX
+  // key + kGenKey: grids that are not powers of two
+  t.push_back({kKindFxLinear, 1 + kGenKey, 8, (const void*)k_fx_linear<1, 8, kFxGen>});
+  t.push_back({kKindFxLinear, 2 + kGenKey, 4, (const void*)k_fx_linear<2, 4, kFxGen>});
+  t.push_back({kKindFxLinear, 2 + kGenKey, 8, (const void*)k_fx_linear<2, 8, kFxGen>});
   // four modes: one kernel for every size (its fields fill the registers whatever the offsets are)
   for (int log = 7; log <= 11; log++) t.push_back({kKindFxLinear, 4 + 1000 * log, 4, (const void*)k_fx_linear<4, 4>});
 }

@@ -12,7 +12,7 @@
 namespace nlm {
 
 // Launch bounds: the grid's threads (at least 128, at most 512 resident per SM: 128 registers each).
-__host__ __device__ constexpr int fx_threads(int NT, int R) { return NT == 0 ? 512 : NT / R < 128 ? 128 : NT / R; }
+__host__ __device__ constexpr int fx_threads(int NT, int R) { return NT <= 0 ? 512 : NT / R < 128 ? 128 : NT / R; }
 
 template <int NT>
 __device__ __forceinline__ void fx_begin(FxField<NT>& f, const FxArgs& fx, const FFTPlanH& plan, int4* smem) {
@@ -23,9 +23,16 @@ __device__ __forceinline__ void fx_begin(FxField<NT>& f, const FxArgs& fx, const
   f.mid = plan.nPass > 1 && plan.radix[1] != plan.radix[0] ? plan.radix[1] : 1;
   for (int k = threadIdx.x; k < f.n; k += blockDim.x) smem[k] = fx.tw[k];
   f.tw = smem;
+  f.plan = &plan;
+  f.root = fx.root;
   f.buf = smem + f.N();
   f.red = reinterpret_cast<uint2*>(smem + f.N() + 2 * fx_buffer(f.N()));
   __syncthreads();
+}
+
+template <int NT>
+__device__ __forceinline__ int4 fx_load(const FxField<NT>& f, const int4* __restrict__ table, int t) {
+  return __ldg(table + (NT == kFxGen ? min(t, f.n - 1) : t));
 }
 
 // One mode through [forward] x table [inverse].  spec(v, value) receives the spectrum (1/N folded in, as the tables
@@ -48,7 +55,7 @@ __device__ __forceinline__ void fx_pair(FxField<NT>& f, const FxArgs& fx, double
     if (dir == 0) {
       k += 2 - ls;
 #pragma unroll
-      for (int v = 0; v < R; v++) y[v] = fx_cmul(y[v], __ldg(table + f.j + v * f.template T<R>()), ls);
+      for (int v = 0; v < R; v++) y[v] = fx_cmul(y[v], fx_load(f, table, f.j + v * f.template T<R>()), ls);
       if (wantF) {
         fx_leave<R>(y, x, k, bad);
 #pragma unroll
@@ -91,7 +98,7 @@ __device__ __forceinline__ void fx_march(const PropArgs& a, Point point) {
         if (m == a.inputMode) seg = 0;
         else if (a.inputMode < 1 && m < a.inChannels) seg = m;
 #pragma unroll
-        for (int v = 0; v < R; v++) x[m][v] = seg >= 0 ? row[(long long)seg * N + j + v * T] : czero();
+        for (int v = 0; v < R; v++) x[m][v] = seg >= 0 && f.has(j + v * T) ? row[(long long)seg * N + j + v * T] : czero();
       }
     }
     for (int i = 0; i <= last; i++) {
@@ -104,16 +111,17 @@ __device__ __forceinline__ void fx_march(const PropArgs& a, Point point) {
       for (int m = 0; m < M; m++) {
         const int4* table = fx.tab + ((long long)which * M + m) * N;
         fx_pair(f, fx, x[0], table, fx.et, fwd, inv, a.gridF != nullptr || !inv, [&](int v, double2 s) {
-          if (a.gridF) a.gridF[m * ms + (long long)i * N + j + v * T] = cscale(s, (double)N);
+          if (a.gridF && f.has(j + v * T)) a.gridF[m * ms + (long long)i * N + j + v * T] = cscale(s, (double)N);
         });
         if (a.gridT) {
 #pragma unroll
-          for (int v = 0; v < R; v++) a.gridT[m * ms + (long long)i * N + j + v * T] = x[0][v];
+          for (int v = 0; v < R; v++)
+            if (f.has(j + v * T)) a.gridT[m * ms + (long long)i * N + j + v * T] = x[0][v];
         }
         if (a.ckpt && !end && i % a.ckK == 0) {
 #pragma unroll
           for (int v = 0; v < R; v++)
-            a.ckpt[((inst * a.ckN + i / a.ckK) * M + m) * (long long)N + j + v * T] = x[0][v];
+            if (f.has(j + v * T)) a.ckpt[((inst * a.ckN + i / a.ckK) * M + m) * (long long)N + j + v * T] = x[0][v];
         }
         if constexpr (M > 1) {
 #pragma unroll
@@ -126,7 +134,7 @@ __device__ __forceinline__ void fx_march(const PropArgs& a, Point point) {
         }
       }
     }
-    store_output<M, R>(a, inst, true, j, x, a.inTime ? 1.0 : (double)N);
+    store_output<M, R, NT == kFxGen>(a, inst, true, j, x, a.inTime ? 1.0 : (double)N);
     __syncthreads();
   }
 }
@@ -135,12 +143,12 @@ __device__ __forceinline__ void fx_march(const PropArgs& a, Point point) {
 template <int M, int R, int NT = 0>
 __global__ void __launch_bounds__(fx_threads(NT, R), 512 / fx_threads(NT, R)) k_fx_linear(const PropArgs a) {
   constexpr int D = 2 * M;
-  const int N = NT ? NT : a.plan.N, T = NT ? NT / R : a.plan.T, j = threadIdx.x;
+  const int N = NT > 0 ? NT : a.plan.N, T = NT > 0 ? NT / R : a.plan.T, j = threadIdx.x;
   fx_march<M, R, NT>(a, [&](int i, double2 (&x)[M][R]) {
     const double2* mat = reinterpret_cast<const double2*>(a.prop) + (long long)(i - 1) * (D * M) * N;
 #pragma unroll
     for (int v = 0; v < R; v++) {
-      const int t = j + v * T;
+      const int t = NT == kFxGen ? min(j + v * T, N - 1) : j + v * T;   // past the grid: zeros stay zero
       double in[D], out[D];
 #pragma unroll
       for (int m = 0; m < M; m++) {
@@ -165,15 +173,15 @@ __global__ void __launch_bounds__(fx_threads(NT, R), 512 / fx_threads(NT, R)) k_
 }
 
 // Every solver with a point-wise DiffEq.
-template <class S, int R>
+template <class S, int R, int NT = 0>
 __global__ void __launch_bounds__(512) k_fx_direct(const PropArgs a) {
   constexpr int M = S::kM, P = S::kP > 0 ? S::kP : 1;
   const int N = a.plan.N, T = a.plan.T, j = threadIdx.x;
-  fx_march<M, R, 0>(a, [&](int i, double2 (&x)[M][R]) {
+  fx_march<M, R, NT>(a, [&](int i, double2 (&x)[M][R]) {
     const double2* c = a.coef + (long long)(i - 1) * 3 * a.nCoef;
 #pragma unroll
     for (int v = 0; v < R; v++) {
-      const int t = j + v * T;
+      const int t = NT == kFxGen ? min(j + v * T, N - 1) : j + v * T;
       double2 p[3][P], xm[M];
 #pragma unroll
       for (int q = 0; q < P; q++) {

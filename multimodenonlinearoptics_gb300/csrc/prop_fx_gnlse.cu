@@ -18,14 +18,15 @@ __device__ __forceinline__ void fx_gnlse_load(const PropArgs& a, FxField<NT>& f,
   const int N = f.N(), T = f.template T<R>(), j = f.j;
   double2 x[R];
 #pragma unroll
-  for (int v = 0; v < R; v++) x[v] = active && a.inChannels > 0 ? a.in[inst * a.inStride + j + v * T] : czero();
+  for (int v = 0; v < R; v++) x[v] = active && a.inChannels > 0 && f.has(j + v * T) ? a.in[inst * a.inStride + j + v * T] : czero();
   fx_pair(f, a.fx, x, a.fx.tab + 2LL * N, a.fx.et, a.inTime != 0, true, true, [&](int v, double2 s) {
     XF[j + v * T] = s;
-    if (a.gridF && active) a.gridF[j + v * T] = cscale(s, (double)N);
+    if (a.gridF && active && f.has(j + v * T)) a.gridF[j + v * T] = cscale(s, (double)N);
   });
 #pragma unroll
   for (int v = 0; v < R; v++) {
     X[j + v * T] = x[v];
+    if (!f.has(j + v * T)) continue;
     if (a.gridT && active) a.gridT[j + v * T] = x[v];
     if (a.ckpt && active) a.ckpt[inst * a.ckN * (long long)N + j + v * T] = x[v];
   }
@@ -43,13 +44,14 @@ __device__ __forceinline__ void fx_gnlse_end(const PropArgs& a, FxField<NT>& f, 
   const bool inv = !last || a.inTime || a.gridT != nullptr;
   fx_pair(f, a.fx, x, a.fx.tab + (last ? N : 0), a.fx.et, false, inv, true, [&](int v, double2 s) {
     XF[j + v * T] = s;
-    if (a.gridF && active) a.gridF[(long long)i * N + j + v * T] = cscale(s, (double)N);
+    if (a.gridF && active && f.has(j + v * T)) a.gridF[(long long)i * N + j + v * T] = cscale(s, (double)N);
   });
 #pragma unroll
   for (int v = 0; v < R; v++) {
     const int t = j + v * T;
+    if (!last) X[t] = x[v];
+    if (!f.has(t)) continue;
     if (!last) {
-      X[t] = x[v];
       if (a.ckpt && active && i % a.ckK == 0) a.ckpt[(inst * a.ckN + i / a.ckK) * (long long)N + t] = x[v];
     }
     if (a.gridT && active) a.gridT[(long long)i * N + t] = x[v];
@@ -67,9 +69,9 @@ __global__ void __launch_bounds__(fx_threads(NT, R), 512 / fx_threads(NT, R))
   __shared__ long long s_group;
   FxField<NT> f;
   fx_begin(f, a.fx, a.plan, fxsm);
-  const int T = NT / R, j = f.j;
-  double2* X = scratch + (long long)blockIdx.x * 3 * NT;
-  double2 *A = X + NT, *XF = X + 2 * NT;
+  const int T = f.template T<R>(), j = f.j, slot = T * R;
+  double2* X = scratch + (long long)blockIdx.x * 3 * slot;
+  double2 *A = X + slot, *XF = X + 2 * slot;
   for (long long local = blockIdx.x; local < a.nInst; local = next_group(a, local, &s_group)) {
     const long long inst = a.instBase + local;
     fx_gnlse_load<R>(a, f, inst, true, XF, X);
@@ -193,6 +195,8 @@ void add_kernels_fx_gnlse(std::vector<KernelEntry>& t) {
   NLM_FX(8, 11)
   NLM_FX(8, 12)
 #undef NLM_FX
+  // key + kGenKey: grids that are not powers of two
+  t.push_back({kKindFxGnlse, kChi3GNLSE + kGenKey, 8, (const void*)k_fx_gnlse<8, kFxGen>});
 }
 
 }  // namespace nlm

@@ -65,6 +65,39 @@ def test_every_solver_matches_oracle(nlm, oracle, name, n):
             assert np.array_equal(out[k], out[ROWS - 2 + k])
 
 
+# every odd radix, alone and repeated, with each power-of-two part; 66 has a factor without a pass (FP64)
+GENERAL = [66, 70, 96, 100, 250, 294, 600, 1000, 1536, 2058, 4050]
+
+
+@pytest.mark.parametrize("n", GENERAL)
+@pytest.mark.parametrize("name", ["Chi2PDC", "Chi2SFGPDC", "Chi2SHG", "Chi2SFGII", "Chi3GNLSE"])
+def test_general_grids_match_oracle(nlm, oracle, name, n):
+    """Grids that are not powers of two: batches (DiffEq and propagator) and full grids, in both domains."""
+    kw = dict(cases.CASES[name], tPrecision=n)
+    if name == "Chi3GNLSE":
+        kw.update(zPrecision=2000, relativeLength=0.02, tMax=20)
+    med, ref = getattr(nlm, name)(**kw), getattr(oracle, name)(**kw)
+    fnl = name in cases.FULLY_NONLINEAR
+    if not fnl:
+        med.runPumpSimulation()
+        ref.run_pump_simulation()
+    modes = med._dims["nSignalModes"]
+    t = np.fft.fftshift(np.linspace(-8, 8, n, endpoint=False))
+    spec = cases.noise(np.random.default_rng(n), 2 * n * modes, 0.1).reshape(2, modes, n) * np.exp(-t ** 2)
+    for in_time in (False, True):
+        x = (np.fft.ifft(spec, axis=2) if in_time else spec).reshape(2, -1)
+        want = ref.batch_signal_simulation(x, in_time) if fnl else ref.batch_signal_simulation(x, in_time, False)
+        for use in ((-1,) if fnl else (0, 1)):
+            med._set_schedule(use_propagator=use)
+            out = med.batchSignalSimulation(x, in_time) if fnl else med.batchSignalSimulation(x, in_time, False)
+            assert cases.rel_l2(out, want) < TOL
+        med.runSignalSimulation(x[0], in_time)
+        ref.run_signal_simulation(x[0], in_time)
+        for m in range(modes):
+            assert cases.rel_l2(med.signalTimes(m), ref.signal_time[m]) < TOL
+            assert cases.rel_l2(med.signalFreqs(m), ref.signal_freq[m]) < TOL
+
+
 @pytest.mark.parametrize("in_time", [False, True])
 @pytest.mark.parametrize("n", [128, 256, 512, 1024, 2048, 4096])
 def test_gnlse_matches_oracle(nlm, oracle, n, in_time):
