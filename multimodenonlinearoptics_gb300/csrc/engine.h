@@ -198,7 +198,7 @@ inline void add_prop_key(GraphKey& k, const PropArgs& a) {
   k.add(a.out).add(a.outStride).add(a.tw).add(a.dstep).add(a.dlast).add(a.half).add(a.back).add(a.prop);
   k.add(a.pump).add(a.pumpStride).add(a.nPumps).add(a.coef).add(a.nCoef).add(a.gridF).add(a.gridT);
   k.add(a.ckpt).add(a.ckK).add(a.ckN).add(a.stages).add(a.raman).add(a.steep).add(a.relInt);
-  k.add(a.fx.tw).add(a.fx.root).add(a.fx.twN).add(a.fx.tab).add(a.fx.et).add(a.fx.raman).add(a.fx.steep).add(a.fx.etRaman).add(a.fx.etSteep).add(a.fx.A0).add(a.fx.sh).add(a.fx.ls);
+  k.add(a.fx.tw).add(a.fx.L).add(a.fx.chirp).add(a.fx.conv).add(a.fx.lsL).add(a.fx.root).add(a.fx.twN).add(a.fx.tab).add(a.fx.et).add(a.fx.raman).add(a.fx.steep).add(a.fx.etRaman).add(a.fx.etSteep).add(a.fx.A0).add(a.fx.sh).add(a.fx.ls);
 }
 
 struct GraphCache {
@@ -339,7 +339,7 @@ struct FxTwiddleCache {
           for (int k = 0; k < L; k++) h.push_back(root(q * k, L * r));
         L *= r;
       }
-      h.resize(p.N);   // the kernels stage N entries
+      h.resize(L);   // the kernels stage as many entries as the transform has points
     });
   }
   // exp(-2 pi i q / r), q < r, for r = 3, 5, 7 (fx_root_at)
@@ -436,7 +436,7 @@ inline FFTPlanH make_plan(int N, int R) {
   p.T = N / R;
   int n = 0;
   while ((1 << n) < N) n++;
-  const int rl = R >= 8 ? 3 : 2;
+  const int rl = R >= 8 ? 3 : R == 2 ? 1 : 2;
   int a = n / rl, rem = n % rl;
   std::vector<int> rad(a, 1 << rl);
   if (rem) rad.insert(rad.begin() + (a >= 1 ? 1 : 0), 1 << rem);
@@ -728,6 +728,8 @@ struct Medium {
   DevBuf<int4> fxTab, fxRaman, fxSteep;
   const int4* spreadTwD = nullptr;
   const int4* fxRoots = nullptr;
+  DevBuf<int4> fxChirp, fxConv;
+  int fxConvEt = 0;
   int fxEtRaman = 0, fxEtSteep = 0;
   bool fxBad = false;   // a table has values that are not finite: only the FP64 kernels take this medium
   int fxEt = 0;
@@ -928,7 +930,8 @@ struct Medium {
     upload(half, hh);
     upload(back, hb);
     if (fxSize()) spreadTwD = g_fxTwiddles.natural((int)N, stream);
-    else if (fxGenSize()) fxRoots = g_fxTwiddles.roots(stream);
+    else if (fxSmooth()) fxRoots = g_fxTwiddles.roots(stream);
+    else if (fxConvSize()) buildConvolution();
     // a single z step has an infinite step length, and tables that are not finite: FP64 kernels
     if ((fxSize() || fxGenSize()) && nZ > 1 && std::isfinite(dz)) {
       std::vector<double2> all(hd);
@@ -979,6 +982,49 @@ struct Medium {
     d.alloc(q.size());
     ck(cudaMemcpyAsync(d.p, q.data(), q.size() * sizeof(int4), cudaMemcpyHostToDevice, stream), "upload");
     sync("upload");   // q goes out of scope
+  }
+  // The chirp exp(-pi i t^2 / N), t < N, and the transform over L points of its conjugate (t^2 mod 2N taken exactly),
+  // divided by L.
+  void buildConvolution() {
+    const long long L = fxConvL(), n = N;
+    std::vector<std::complex<long double>> b(L);
+    std::vector<double2> c(n), h(L);
+    std::vector<int4> q;
+    for (long long t = 0; t < n; t++) {
+      const long double ang = 3.141592653589793238462643383279502884L * (long double)(t * t % (2 * n)) / (long double)n;
+      const std::complex<long double> w(std::cos(ang), std::sin(ang));
+      q.push_back(fx_quantise(w.real(), -w.imag(), 0));
+      b[t] = w;
+      if (t > 0) b[L - t] = w;
+    }
+    q.resize(n + kTablePad);
+    fxChirp.alloc(q.size());
+    ck(cudaMemcpyAsync(fxChirp.p, q.data(), q.size() * sizeof(int4), cudaMemcpyHostToDevice, stream), "upload");
+    sync("convolution tables");
+    // radix-2 transform of b in extended precision
+    for (long long i = 1, r = 0; i < L; i++) {
+      long long bit = L >> 1;
+      for (; r & bit; bit >>= 1) r ^= bit;
+      r ^= bit;
+      if (i < r) std::swap(b[i], b[r]);
+    }
+    for (long long len = 2; len <= L; len *= 2) {
+      std::vector<std::complex<long double>> w(len / 2);
+      for (long long k = 0; k < len / 2; k++) {
+        const long double ang = -2.0L * 3.141592653589793238462643383279502884L * (long double)k / (long double)len;
+        w[k] = {std::cos(ang), std::sin(ang)};
+      }
+      for (long long i = 0; i < L; i += len)
+        for (long long k = 0; k < len / 2; k++) {
+          const auto u = b[i + k], v = b[i + k + len / 2];
+          const std::complex<long double> p(v.real() * w[k].real() - v.imag() * w[k].imag(),
+                                            v.real() * w[k].imag() + v.imag() * w[k].real());
+          b[i + k] = u + p;
+          b[i + k + len / 2] = u - p;
+        }
+    }
+    for (long long k = 0; k < L; k++) h[k] = make_double2((double)(b[k].real() / L), (double)(b[k].imag() / L));
+    uploadFx(fxConv, &fxConvEt, h);
   }
   void uploadD(DevBuf<double>& d, const std::vector<double>& h) {
     if (h.empty()) {
@@ -1517,7 +1563,7 @@ struct Medium {
     if (ipc > nInst) ipc = (int)std::max<long long>(1, nInst);
     const int block = T * ipc;
     // exchange buffers of the ipc propagations, plus the staged twiddle table when R != 16
-    const size_t smem = fx ? fx_smem((int)N) : (size_t)(ipc + (k->R != 16 ? 1 : 0)) * N * sizeof(double2);
+    const size_t smem = fx ? fx_smem(fxConvSize() ? (int)fxConvL() : (int)N) : (size_t)(ipc + (k->R != 16 ? 1 : 0)) * N * sizeof(double2);
     int dev = 0, sms = 1, optin = 0;
     ck(cudaGetDevice(&dev), "device");
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -1708,17 +1754,28 @@ struct Medium {
   bool fxSize() const { return is_pow2((int)N) && N >= kFxMinN && N <= kFxMaxN; }
   // other grids whose prime factors the kernels have passes for
   bool fxGenSize() const {
-    if (is_pow2((int)N) || N % 2 != 0 || N < 64 || N > kFxMaxN) return false;
+    return !is_pow2((int)N) && N % 2 == 0 && N >= 64 && N <= kFxMaxN && (fxSmooth() || fxConvSize());
+  }
+  // the general plan with whole warps (padding a grid's last warps)
+  FFTPlanH fxGenPlan(int R) const {
+    FFTPlanH p = fxConvSize() ? make_plan((int)fxConvL(), R) : make_plan_gen((int)N, R);
+    p.T = fxConvSize() ? (int)fxConvL() / R : 32 * (((int)N + 32 * R - 1) / (32 * R));
+    p.N = (int)N;
+    return p;
+  }
+  // Grids with a larger prime factor: the convolution form on the next power of two L >= 2 N - 1, which must fit one
+  // CTA (4096 points).  Its two transforms over L replace passes that cost a product per point and unit of the factor.
+  bool fxConvSize() const { return !is_pow2((int)N) && N % 2 == 0 && N >= 64 && 2 * N - 1 <= kFxMaxN && !fxSmooth(); }
+  uint fxConvL() const {
+    uint l = 128;
+    while (l < 2 * N - 1) l *= 2;
+    return l;
+  }
+  bool fxSmooth() const {
     uint n = N;
     for (uint q : {2u, 3u, 5u, 7u})
       while (n % q == 0) n /= q;
     return n == 1;
-  }
-  // the general plan with whole warps (padding a grid's last warps)
-  FFTPlanH fxGenPlan(int R) const {
-    FFTPlanH p = make_plan_gen((int)N, R);
-    p.T = 32 * (((int)N + 32 * R - 1) / (32 * R));
-    return p;
   }
   bool fxGrid() const { return fxTab.p && (solver != kChi3GNLSE || (fxRaman.p && fxSteep.p)); }
   // the N-point twiddles of the one-point-per-thread cluster kernels (null on grids without them)
@@ -1754,6 +1811,15 @@ struct Medium {
     }
     f.A0 = 60;
     f.ls = 2 - (level >= 0 ? (level + 1) / 2 : -((-level) / 2));   // 2 - ceil(level / 2)
+    if (!is_pow2(p.N) && fxConvSize()) {
+      // a transform: two of L points, the product with conv and the closing chirp, both shifted back to 2^A0
+      f.L = (int)fxConvL();
+      f.chirp = fxChirp.p;
+      f.conv = fxConv.p;
+      f.lsL = f.ls;
+      f.sh = 2 * f.sh + 2 * (2 - f.lsL) + fxConvEt;
+      f.ls = 2;
+    }
     return f;
   }
 
@@ -2091,13 +2157,15 @@ struct Medium {
       if (a.ckpt) throw Unsupported("the adjoint's forward takes power-of-two grids (register plan) only");
       int Rg = R;
       const bool fx = fxGenSize() && fxGrid() && !plainOne;
+      const int fxKey = fxConvSize() ? kConvKey : kGenKey;
       if (fx && !gnlse && allowPropagator && wantPropagator(nInst) &&
-          (k = fxKernel(kKindFxLinear, (int)nSignal + kGenKey, &Rg))) {
+          (k = fxKernel(kKindFxLinear, (int)nSignal + fxKey, &Rg))) {
         buildPropagator(R);
         a.prop = prop.p;
       }
       if (!k && fx && (gnlse || !(allowPropagator && wantPropagator(nInst))))
-        k = fxKernel(gnlse ? kKindFxGnlse : kKindFxDirect, solver + kGenKey, &Rg);
+        k = gnlse ? fxKernel(kKindFxGnlse, solver + fxKey, &Rg)
+                  : fxKernel(kKindFxDirect, solver + (fxConvSize() ? 0 : kGenKey), &Rg);
       if (!k && !gnlse && allowPropagator && wantPropagator(nInst)) {
         k = genKernel(kKindLinear, (int)nSignal, R, &Rg);
         if (k) {

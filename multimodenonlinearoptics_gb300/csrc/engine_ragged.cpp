@@ -38,11 +38,17 @@ constexpr double kStepUs[2][kForms][5] = {
     {{26.4, 27.9, 34.8, 67.9, 137.8}, {9.8, 10.5, 12.0, 21.0, 41.8}, {0, 0, 0, 14.3, 25.5}, {0, 0, 0, 0, 20.6}},
     {{18.4, 19.9, 27.8, 51.8, 99.5}, {7.7, 8.5, 10.0, 16.9, 33.7}, {0, 0, 0, 12.5, 21.5}, {0, 0, 0, 0, 19.3}}};
 
-double step_us(int form, uint N, uint modes, bool prop) {
+// The same of the kernels with block fixed-point transforms, which the ragged call runs and plans with (the table
+// above stays the cost model of nlm_ragged_plan, a planner for given costs).
+constexpr double kCallStepUs[2][kForms][5] = {
+    {{11.7, 13.2, 20.0, 35.0, 67.8}, {6.9, 7.5, 8.4, 13.8, 41.7}, {0, 0, 0, 10.1, 16.5}, {0, 0, 0, 0, 14.0}},
+    {{7.6, 8.5, 10.6, 16.3, 29.7}, {4.7, 5.4, 6.4, 9.9, 33.6}, {0, 0, 0, 8.2, 12.6}, {0, 0, 0, 0, 12.1}}};
+
+double step_us(int form, uint N, uint modes, bool prop, const double (*table)[kForms][5] = kStepUs) {
   int lg = 0;
   while ((1u << lg) < N) lg++;
   const int i = std::min(std::max(lg - 7, 0), 4);
-  double t = kStepUs[prop ? 1 : 0][form][i];
+  double t = table[prop ? 1 : 0][form][i];
   if (t == 0) return -1;
   if (lg > 11) t *= (double)N * lg / (2048.0 * 11);
   return t * std::max(1u, modes) / 2.0;
@@ -322,13 +328,13 @@ nlm_status nlm_ragged_batch(nlm_medium* const* media, size_t n_media, const doub
       while ((1u << lg) < m->N) lg++;
       Job j{k, m->solver * 64 + lg, {-1, -1, -1, -1}};
       const double steps = (double)(m->nZ > 1 ? m->nZ - 1 : 1);
-      j.t[kOne] = step_us(kOne, m->N, m->nSignal, withProp[k]) * steps;
+      j.t[kOne] = step_us(kOne, m->N, m->nSignal, withProp[k], kCallStepUs) * steps;
       // four CTAs: one point per thread on the spread grids, four points per thread from 1024 points
       const bool c4 = (m->spreadGrid() && m->findKernel(kKindCluster, m->solver, 1)) || m->clusterGrid();
-      if (c4) j.t[kC4] = step_us(kC4, m->N, m->nSignal, withProp[k]) * steps;
+      if (c4) j.t[kC4] = step_us(kC4, m->N, m->nSignal, withProp[k], kCallStepUs) * steps;
       if (m->w8Grid() && m->findKernel(kKindCluster, m->solver + kSpreadWideKey, 1))
-        j.t[kW8] = step_us(kW8, m->N, m->nSignal, withProp[k]) * steps;
-      if (m->w16Kernel()) j.t[kW16] = step_us(kW16, m->N, m->nSignal, withProp[k]) * steps;
+        j.t[kW8] = step_us(kW8, m->N, m->nSignal, withProp[k], kCallStepUs) * steps;
+      if (m->w16Kernel()) j.t[kW16] = step_us(kW16, m->N, m->nSignal, withProp[k], kCallStepUs) * steps;
       jobs.push_back(j);
     }
     int maxW16 = 0;
@@ -433,11 +439,23 @@ nlm_status nlm_ragged_batch(nlm_medium* const* media, size_t n_media, const doub
       // N/4 threads per medium when the largest grid allows it (four warps from N = 512), else N/8
       const KernelEntry* k4 = maxN / 4 <= 512 ? lead->findKernel(kKindRagged, solver, 4) : nullptr;
       const KernelEntry* ke = k4 ? k4 : lead->findKernel(kKindRagged, solver, 8);
+      // block fixed-point transforms where every medium has their tables (a class has one grid)
+      bool fx = lead->fxSize();
+      for (size_t i : js) fx = fx && ms[jobs[i].k]->fxGrid();
+      if (fx) {
+        const int r = maxN <= 256 ? 2 : maxN <= 2048 ? 4 : 8;
+        if (const KernelEntry* kx = lead->findKernel(kKindRagged, solver + kFxRaggedKey, r)) ke = kx;
+        else fx = false;
+      }
       const int Rg = ke->R;
       RaggedLaunch rl{ke, 0, (int)((maxN / Rg + 31) / 32 * 32), (int)items.size(), (int)js.size(), 0};
       for (size_t i : js) {
         Medium* m = ms[jobs[i].k];
         PropArgs a = rowArgs(m, jobs[i].k, Rg);
+        if (fx) {
+          a.plan = make_plan((int)m->N, Rg);
+          a.fx = m->fxArgs(a.plan);
+        }
         a.nInst = 1;
         a.ipc = 1;
         a.prop = withProp[jobs[i].k] ? m->prop.p : nullptr;
@@ -447,7 +465,7 @@ nlm_status nlm_ragged_batch(nlm_medium* const* media, size_t n_media, const doub
       // One CTA per SM: every medium is a sequential march bound by its SM's FP64 units.  Asking for
       // more than half of the SM's shared memory keeps other CTAs off its SM.
       cudaFuncAttributes fa;
-      ck(exclusive_smem(ke->fn, maxN * sizeof(double2), &rl.smem, &fa), "smem attribute");
+      ck(exclusive_smem(ke->fn, fx ? fx_smem((int)maxN) : maxN * sizeof(double2), &rl.smem, &fa), "smem attribute");
       if (rl.smem == 0) throw Unsupported("ragged kernel does not fit on an SM");
       if (rl.block > fa.maxThreadsPerBlock) throw Unsupported("ragged kernel cannot launch that many threads");
       // a share of the SMs the plan leaves free, in proportion to the launch's work

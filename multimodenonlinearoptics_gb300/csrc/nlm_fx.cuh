@@ -131,6 +131,10 @@ struct FxField {   // NT = kFxGen: a grid that is not a power of two
   const int4* tw;    // the passes' twiddles, Q62
   uint2* red;        // one (exponent, sum) pair per warp of the group
   int n, t, j, sel, mid;
+  int grid;               // the grid's points (n where the transform has as many)
+  const int4* chirp;      // convolution form: FxArgs::chirp, conv, lsL
+  const int4* conv;
+  int lsL;
   const FFTPlanH* plan;   // the general plan's radices, and its roots of unity (fx_root_at)
   const int4* root;
   __device__ __forceinline__ int N() const { return NT > 0 ? NT : n; }
@@ -139,7 +143,7 @@ struct FxField {   // NT = kFxGen: a grid that is not a power of two
     return NT > 0 ? NT / R : t;
   }
   // thread j's points that the grid has
-  __device__ __forceinline__ bool has(int at) const { return NT >= 0 || at < n; }
+  __device__ __forceinline__ bool has(int at) const { return NT > 0 || at < grid; }
   // radix of the second pass where it is not the plan's main one, else 1
   template <int r>
   __device__ __forceinline__ int small() const {
@@ -201,7 +205,7 @@ struct FxInt {
 // The forward transform of the plan of make_plan(N, R): passes of radix R (8, 4 or 2) with one of another radix (1:
 // none) in second place; ownership j + v T in and out.  f.tw holds the passes' twiddles one after another.
 template <int R, int NT>
-__device__ __forceinline__ void fx_fft(FxField<NT>& f, fxc (&x)[R]) {
+__device__ __forceinline__ void fx_fft_pow2(FxField<NT>& f, fxc (&x)[R]) {
   constexpr int r = R >= 8 ? 8 : R >= 4 ? 4 : 2;
   const int N = f.N(), mid = f.template small<r>();
   int L = 1, level = 0;
@@ -224,6 +228,39 @@ __device__ __forceinline__ void fx_fft(FxField<NT>& f, fxc (&x)[R]) {
   } else {
 #pragma unroll 1
     while (L < N) pass(FxInt<r>{});
+  }
+}
+
+// Grids of N points with a prime factor that has no pass (NT = 0, f.chirp set): with 2 t k = t^2 + k^2 - (k - t)^2 the
+// transform is a convolution with the conjugate chirp, run cyclically on L >= 2 N - 1 points, L a power of two
+// (Bluestein 1970): x c, forward transform over L, x conv, inverse transform, x c.  Points past the grid are zero.
+// The field comes back below 2^A0.
+template <int R, int NT>
+__device__ __forceinline__ void fx_fft(FxField<NT>& f, fxc (&x)[R]) {
+  if constexpr (NT > 0) {
+    fx_fft_pow2(f, x);
+  } else {
+    const bool conv = f.chirp != nullptr;
+    auto chirp = [&](int ls) {
+#pragma unroll
+      for (int v = 0; v < R; v++) {
+        const int t = f.j + v * f.t;
+        x[v] = t < f.grid ? fx_cmul(x[v], __ldg(f.chirp + t), ls) : fxc{0, 0};
+      }
+    };
+    if (conv) chirp(2);
+#pragma unroll 1
+    for (int d = 0; d < (conv ? 2 : 1); d++) {
+      fx_fft_pow2(f, x);
+      if (conv) {
+#pragma unroll
+        for (int v = 0; v < R; v++) {
+          if (d == 0) x[v] = fx_cmul(x[v], __ldg(f.conv + f.j + v * f.t), f.lsL);
+          x[v] = fxc{x[v].y, x[v].x};
+        }
+      }
+    }
+    if (conv) chirp(f.lsL);
   }
 }
 

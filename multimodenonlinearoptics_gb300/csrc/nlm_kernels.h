@@ -27,6 +27,12 @@ struct FFTPlanH {
 // value as balanced 32-bit halves {re high, re low, im high, im low} with value (h 2^32 + l) 2^(et - 62).
 struct FxArgs {
   const int4* tw;    // the plan's twiddles, pass by pass (one-CTA kernels)
+  // grids with a prime factor above 7: the convolution form on L points (0: none), its chirp exp(-pi i t^2 / N) and the
+  // transform of the conjugate chirp over L, relative to a power of two that sh carries
+  int L;
+  const int4* chirp;
+  const int4* conv;
+  int lsL;           // places the product with conv, and the chirp after it, are shifted left
   const int4* root;  // exp(-2 pi i q / r) of the odd radices (fx_root_at)
   const int4* twN;   // exp(-2 pi i m / N), m < N (cluster kernels with one point per thread)
   const int4* tab;   // [dispStep, last, half][mode][N], each with its 1/N
@@ -187,6 +193,10 @@ constexpr long long kSpreadSmemPerPoint = spread_smem_per_point(4);
 // Registry key offset of the instantiations for the general plan (FFTPlanH::gen == 1): grids that are
 // not powers of two (kKindDirect, kKindLinear, kKindGnlse).
 constexpr int kGenKey = 2000;
+// and (kKindRagged) of the block fixed-point kernels
+constexpr int kFxRaggedKey = 1000;
+// and of their convolution form, where it needs a kernel of its own (kKindFxDirect's runtime-size kernels serve it too)
+constexpr int kConvKey = 3000;
 // Registry key offset (kKindCluster) of the one-point-per-thread kernels on eight CTAs, and on sixteen.
 constexpr int kSpreadWideKey = 800;
 constexpr int kSpreadW16Key = 900;

@@ -27,6 +27,12 @@ void add_kernels_fx(std::vector<KernelEntry>& t) {
   t.push_back({kKindFxLinear, 2 + kGenKey, 8, (const void*)k_fx_linear<2, 8, kFxGen>});
   // four modes: one kernel for every size (its fields fill the registers whatever the offsets are)
   for (int log = 7; log <= 11; log++) t.push_back({kKindFxLinear, 4 + 1000 * log, 4, (const void*)k_fx_linear<4, 4>});
+  // key + kConvKey: the convolution form
+  t.push_back({kKindFxLinear, 1 + kConvKey, 8, (const void*)k_fx_linear<1, 8>});
+  t.push_back({kKindFxLinear, 1 + kConvKey, 4, (const void*)k_fx_linear<1, 4>});
+  t.push_back({kKindFxLinear, 2 + kConvKey, 8, (const void*)k_fx_linear<2, 8>});
+  t.push_back({kKindFxLinear, 2 + kConvKey, 4, (const void*)k_fx_linear<2, 4>});
+  t.push_back({kKindFxLinear, 4 + kConvKey, 4, (const void*)k_fx_linear<4, 4>});
 }
 
 }  // namespace nlm

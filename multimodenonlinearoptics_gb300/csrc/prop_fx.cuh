@@ -16,7 +16,11 @@ __host__ __device__ constexpr int fx_threads(int NT, int R) { return NT <= 0 ? 5
 
 template <int NT>
 __device__ __forceinline__ void fx_begin(FxField<NT>& f, const FxArgs& fx, const FFTPlanH& plan, int4* smem) {
-  f.n = plan.N;
+  f.n = fx.L ? fx.L : plan.N;
+  f.grid = plan.N;
+  f.chirp = fx.chirp;
+  f.conv = fx.conv;
+  f.lsL = fx.lsL;
   f.t = plan.T;
   f.j = threadIdx.x;
   f.sel = 0;
@@ -32,7 +36,7 @@ __device__ __forceinline__ void fx_begin(FxField<NT>& f, const FxArgs& fx, const
 
 template <int NT>
 __device__ __forceinline__ int4 fx_load(const FxField<NT>& f, const int4* __restrict__ table, int t) {
-  return __ldg(table + (NT == kFxGen ? min(t, f.n - 1) : t));
+  return __ldg(table + (NT <= 0 ? min(t, f.grid - 1) : t));
 }
 
 // One mode through [forward] x table [inverse].  spec(v, value) receives the spectrum (1/N folded in, as the tables
@@ -68,139 +72,152 @@ __device__ __forceinline__ void fx_pair(FxField<NT>& f, const FxArgs& fx, double
   if (inv) fx_leave<R>(y, x, k, bad);
 }
 
+// One propagation.
+template <int M, int R, int NT, class Point>
+__device__ __forceinline__ void fx_propagate(const PropArgs& a, FxField<NT>& f, long long inst, Point point) {
+  const FxArgs& fx = a.fx;
+  const int N = NT > 0 ? NT : f.grid, T = f.template T<R>(), j = f.j;
+  const long long ms = (long long)a.nZ * N;
+  const int last = a.nZ - 1;
+  double2 x[M][R];
+  if (a.inKind == 0) {
+    const long long pair = inst >> 1;
+    const int bin = (int)(pair % N), im = (int)(pair / N);
+    const int mode = a.impModes[im < kMaxModes ? im : 0];
+    const double2 val = (inst & 1) ? make_double2(0.0, 1.0) : make_double2(1.0, 0.0);
+#pragma unroll
+    for (int m = 0; m < M; m++)
+#pragma unroll
+      for (int v = 0; v < R; v++) x[m][v] = (m == mode && j + v * T == bin) ? val : czero();
+  } else {
+    const double2* row = a.in + inst * a.inStride;
+#pragma unroll
+    for (int m = 0; m < M; m++) {
+      int seg = -1;
+      if (m == a.inputMode) seg = 0;
+      else if (a.inputMode < 1 && m < a.inChannels) seg = m;
+#pragma unroll
+      for (int v = 0; v < R; v++) x[m][v] = seg >= 0 && f.has(j + v * T) ? row[(long long)seg * N + j + v * T] : czero();
+    }
+  }
+  for (int i = 0; i <= last; i++) {
+    if (i > 0) point(i, x);
+    const bool end = i == last;
+    const bool fwd = i > 0 || a.inTime, inv = !end || a.inTime || a.gridT != nullptr;
+    const int which = i == 0 ? 2 : !end ? 0 : 1;
+    // the modes in turn through one copy of the pair: mode m sits in x[0] during its turn
+#pragma unroll 1
+    for (int m = 0; m < M; m++) {
+      const int4* table = fx.tab + ((long long)which * M + m) * N;
+      fx_pair(f, fx, x[0], table, fx.et, fwd, inv, a.gridF != nullptr || !inv, [&](int v, double2 s) {
+        if (a.gridF && f.has(j + v * T)) a.gridF[m * ms + (long long)i * N + j + v * T] = cscale(s, (double)N);
+      });
+      if (a.gridT) {
+#pragma unroll
+        for (int v = 0; v < R; v++)
+          if (f.has(j + v * T)) a.gridT[m * ms + (long long)i * N + j + v * T] = x[0][v];
+      }
+      if (a.ckpt && !end && i % a.ckK == 0) {
+#pragma unroll
+        for (int v = 0; v < R; v++)
+          if (f.has(j + v * T)) a.ckpt[((inst * a.ckN + i / a.ckK) * M + m) * (long long)N + j + v * T] = x[0][v];
+      }
+      if constexpr (M > 1) {
+#pragma unroll
+        for (int v = 0; v < R; v++) {
+          const double2 t = x[0][v];
+#pragma unroll
+          for (int q = 0; q < M - 1; q++) x[q][v] = x[q + 1][v];
+          x[M - 1][v] = t;
+        }
+      }
+    }
+  }
+  store_output<M, R, NT <= 0>(a, inst, true, j, x, a.inTime ? 1.0 : (double)N);
+  __syncthreads();
+}
+
 template <int M, int R, int NT, class Point>
 __device__ __forceinline__ void fx_march(const PropArgs& a, Point point) {
   extern __shared__ int4 fxsm[];
   __shared__ long long s_group;
   FxField<NT> f;
-  const FxArgs& fx = a.fx;
-  fx_begin(f, fx, a.plan, fxsm);
-  const int N = f.N(), T = f.template T<R>(), j = f.j;
-  const long long ms = (long long)a.nZ * N;
-  const int last = a.nZ - 1;
-  for (long long inst0 = blockIdx.x; inst0 < a.nInst; inst0 = next_group(a, inst0, &s_group)) {
-    const long long inst = a.instBase + inst0;
-    double2 x[M][R];
-    if (a.inKind == 0) {
-      const long long pair = inst >> 1;
-      const int bin = (int)(pair % N), im = (int)(pair / N);
-      const int mode = a.impModes[im < kMaxModes ? im : 0];
-      const double2 val = (inst & 1) ? make_double2(0.0, 1.0) : make_double2(1.0, 0.0);
+  fx_begin(f, a.fx, a.plan, fxsm);
+  for (long long local = blockIdx.x; local < a.nInst; local = next_group(a, local, &s_group))
+    fx_propagate<M, R, NT>(a, f, a.instBase + local, point);
+}
+
+// Step i of a pump-driven solver as its per-point real (2M) x (2M) matrix (layout as k_propagate_linear).
+template <int M, int R, int NT>
+__device__ __forceinline__ void fx_matrix_step(const PropArgs& a, int i, int N, int T, int j, double2 (&x)[M][R]) {
+  constexpr int D = 2 * M;
+  const double2* mat = reinterpret_cast<const double2*>(a.prop) + (long long)(i - 1) * (D * M) * N;
 #pragma unroll
-      for (int m = 0; m < M; m++)
+  for (int v = 0; v < R; v++) {
+    const int t = j + v * T;
+    if (NT <= 0 && t >= N) continue;   // past the grid: zeros stay zero
+    double in[D], out[D];
 #pragma unroll
-        for (int v = 0; v < R; v++) x[m][v] = (m == mode && j + v * T == bin) ? val : czero();
-    } else {
-      const double2* row = a.in + inst * a.inStride;
-#pragma unroll
-      for (int m = 0; m < M; m++) {
-        int seg = -1;
-        if (m == a.inputMode) seg = 0;
-        else if (a.inputMode < 1 && m < a.inChannels) seg = m;
-#pragma unroll
-        for (int v = 0; v < R; v++) x[m][v] = seg >= 0 && f.has(j + v * T) ? row[(long long)seg * N + j + v * T] : czero();
-      }
+    for (int m = 0; m < M; m++) {
+      in[2 * m] = x[m][v].x;
+      in[2 * m + 1] = x[m][v].y;
     }
-    for (int i = 0; i <= last; i++) {
-      if (i > 0) point(i, x);
-      const bool end = i == last;
-      const bool fwd = i > 0 || a.inTime, inv = !end || a.inTime || a.gridT != nullptr;
-      const int which = i == 0 ? 2 : !end ? 0 : 1;
-      // the modes in turn through one copy of the pair: mode m sits in x[0] during its turn
-#pragma unroll 1
-      for (int m = 0; m < M; m++) {
-        const int4* table = fx.tab + ((long long)which * M + m) * N;
-        fx_pair(f, fx, x[0], table, fx.et, fwd, inv, a.gridF != nullptr || !inv, [&](int v, double2 s) {
-          if (a.gridF && f.has(j + v * T)) a.gridF[m * ms + (long long)i * N + j + v * T] = cscale(s, (double)N);
-        });
-        if (a.gridT) {
 #pragma unroll
-          for (int v = 0; v < R; v++)
-            if (f.has(j + v * T)) a.gridT[m * ms + (long long)i * N + j + v * T] = x[0][v];
-        }
-        if (a.ckpt && !end && i % a.ckK == 0) {
+    for (int r = 0; r < D; r++) {
+      const double2 e0 = __ldg(mat + (long long)(r * M) * N + t);
+      double s = fma(e0.y, in[1], e0.x * in[0]);
 #pragma unroll
-          for (int v = 0; v < R; v++)
-            if (f.has(j + v * T)) a.ckpt[((inst * a.ckN + i / a.ckK) * M + m) * (long long)N + j + v * T] = x[0][v];
-        }
-        if constexpr (M > 1) {
-#pragma unroll
-          for (int v = 0; v < R; v++) {
-            const double2 t = x[0][v];
-#pragma unroll
-            for (int q = 0; q < M - 1; q++) x[q][v] = x[q + 1][v];
-            x[M - 1][v] = t;
-          }
-        }
+      for (int c = 1; c < M; c++) {
+        const double2 e = __ldg(mat + (long long)(r * M + c) * N + t);
+        s = fma(e.y, in[2 * c + 1], fma(e.x, in[2 * c], s));
       }
+      out[r] = s;
     }
-    store_output<M, R, NT == kFxGen>(a, inst, true, j, x, a.inTime ? 1.0 : (double)N);
-    __syncthreads();
+#pragma unroll
+    for (int m = 0; m < M; m++) x[m][v] = make_double2(out[2 * m], out[2 * m + 1]);
   }
 }
 
-// Pump-driven solvers: the RK4 step as its per-point real (2M) x (2M) matrix (layout as k_propagate_linear).
-template <int M, int R, int NT = 0>
-__global__ void __launch_bounds__(fx_threads(NT, R), 512 / fx_threads(NT, R)) k_fx_linear(const PropArgs a) {
-  constexpr int D = 2 * M;
-  const int N = NT > 0 ? NT : a.plan.N, T = NT > 0 ? NT / R : a.plan.T, j = threadIdx.x;
-  fx_march<M, R, NT>(a, [&](int i, double2 (&x)[M][R]) {
-    const double2* mat = reinterpret_cast<const double2*>(a.prop) + (long long)(i - 1) * (D * M) * N;
+// Step i with the solver's DiffEq.
+template <class S, int R, int NT>
+__device__ __forceinline__ void fx_diffeq_step(const PropArgs& a, int i, int N, int T, int j, double2 (&x)[S::kM][R]) {
+  constexpr int M = S::kM, P = S::kP > 0 ? S::kP : 1;
+  const double2* c = a.coef + (long long)(i - 1) * 3 * a.nCoef;
 #pragma unroll
-    for (int v = 0; v < R; v++) {
-      const int t = NT == kFxGen ? min(j + v * T, N - 1) : j + v * T;   // past the grid: zeros stay zero
-      double in[D], out[D];
+  for (int v = 0; v < R; v++) {
+    const int t = j + v * T;
+    if (NT <= 0 && t >= N) continue;
+    double2 p[3][P], xm[M];
 #pragma unroll
-      for (int m = 0; m < M; m++) {
-        in[2 * m] = x[m][v].x;
-        in[2 * m + 1] = x[m][v].y;
+    for (int q = 0; q < P; q++) {
+      if (S::kP > 0) {
+        const double2* pr = a.pump + q * a.pumpStride + (long long)(2 * i - 2) * N + t;
+        p[0][q] = __ldg(pr);
+        p[1][q] = __ldg(pr + N);
+        p[2][q] = __ldg(pr + 2 * N);
+      } else {
+        p[0][q] = p[1][q] = p[2][q] = czero();
       }
-#pragma unroll
-      for (int r = 0; r < D; r++) {
-        const double2 e0 = __ldg(mat + (long long)(r * M) * N + t);
-        double s = fma(e0.y, in[1], e0.x * in[0]);
-#pragma unroll
-        for (int c = 1; c < M; c++) {
-          const double2 e = __ldg(mat + (long long)(r * M + c) * N + t);
-          s = fma(e.y, in[2 * c + 1], fma(e.x, in[2 * c], s));
-        }
-        out[r] = s;
-      }
-#pragma unroll
-      for (int m = 0; m < M; m++) x[m][v] = make_double2(out[2 * m], out[2 * m + 1]);
     }
-  });
+#pragma unroll
+    for (int m = 0; m < M; m++) xm[m] = x[m][v];
+    rk4_point<S>(xm, p, c);
+#pragma unroll
+    for (int m = 0; m < M; m++) x[m][v] = xm[m];
+  }
 }
 
-// Every solver with a point-wise DiffEq.
+template <int M, int R, int NT = 0>
+__global__ void __launch_bounds__(fx_threads(NT, R), 512 / fx_threads(NT, R)) k_fx_linear(const PropArgs a) {
+  const int N = NT > 0 ? NT : a.plan.N, T = NT > 0 ? NT / R : a.plan.T, j = threadIdx.x;
+  fx_march<M, R, NT>(a, [&](int i, double2 (&x)[M][R]) { fx_matrix_step<M, R, NT>(a, i, N, T, j, x); });
+}
+
 template <class S, int R, int NT = 0>
 __global__ void __launch_bounds__(512) k_fx_direct(const PropArgs a) {
-  constexpr int M = S::kM, P = S::kP > 0 ? S::kP : 1;
-  const int N = a.plan.N, T = a.plan.T, j = threadIdx.x;
-  fx_march<M, R, NT>(a, [&](int i, double2 (&x)[M][R]) {
-    const double2* c = a.coef + (long long)(i - 1) * 3 * a.nCoef;
-#pragma unroll
-    for (int v = 0; v < R; v++) {
-      const int t = NT == kFxGen ? min(j + v * T, N - 1) : j + v * T;
-      double2 p[3][P], xm[M];
-#pragma unroll
-      for (int q = 0; q < P; q++) {
-        if (S::kP > 0) {
-          const double2* pr = a.pump + q * a.pumpStride + (long long)(2 * i - 2) * N + t;
-          p[0][q] = __ldg(pr);
-          p[1][q] = __ldg(pr + N);
-          p[2][q] = __ldg(pr + 2 * N);
-        } else {
-          p[0][q] = p[1][q] = p[2][q] = czero();
-        }
-      }
-#pragma unroll
-      for (int m = 0; m < M; m++) xm[m] = x[m][v];
-      rk4_point<S>(xm, p, c);
-#pragma unroll
-      for (int m = 0; m < M; m++) x[m][v] = xm[m];
-    }
-  });
+  constexpr int M = S::kM;
+  const int N = NT > 0 ? NT : a.plan.N, T = NT > 0 ? NT / R : a.plan.T, j = threadIdx.x;
+  fx_march<M, R, NT>(a, [&](int i, double2 (&x)[M][R]) { fx_diffeq_step<S, R, NT>(a, i, N, T, j, x); });
 }
 
 }  // namespace nlm

@@ -15,7 +15,7 @@ namespace nlm {
 template <int R, int NT>
 __device__ __forceinline__ void fx_gnlse_load(const PropArgs& a, FxField<NT>& f, long long inst, bool active, double2* XF,
                                               double2* X) {
-  const int N = f.N(), T = f.template T<R>(), j = f.j;
+  const int N = NT > 0 ? NT : f.grid, T = f.template T<R>(), j = f.j;
   double2 x[R];
 #pragma unroll
   for (int v = 0; v < R; v++) x[v] = active && a.inChannels > 0 && f.has(j + v * T) ? a.in[inst * a.inStride + j + v * T] : czero();
@@ -36,7 +36,7 @@ __device__ __forceinline__ void fx_gnlse_load(const PropArgs& a, FxField<NT>& f,
 template <int R, int NT>
 __device__ __forceinline__ void fx_gnlse_end(const PropArgs& a, FxField<NT>& f, int i, long long inst, bool active,
                                              double2* XF, const double2* A, double2* X) {
-  const int N = f.N(), T = f.template T<R>(), j = f.j;
+  const int N = NT > 0 ? NT : f.grid, T = f.template T<R>(), j = f.j;
   const bool last = i == a.nZ - 1;
   double2 x[R];
 #pragma unroll
@@ -138,6 +138,7 @@ __global__ void __launch_bounds__(fx_threads(NT, R), 512 / fx_threads(NT, R))
         const double fac = s == 0 ? 0.0 : (s == 3 ? 1.0 : 0.5);
         const double wgt = (s == 1 || s == 2) ? 2.0 : 1.0;
         const double ri = __ldg(rel + (s == 0 ? 0 : (s == 3 ? 2 : 1)));
+        const bool scaled = __double_as_longlong(ri) != 0x3ff0000000000000LL;   // 1 without an intensity profile
         // c = 0: both rows' Raman convolutions; c = 1, 2: row c - 1's product and self-steepening
 #pragma unroll 1
         for (int c = 0; c < 3; c++) {
@@ -146,18 +147,23 @@ __global__ void __launch_bounds__(fx_threads(NT, R), 512 / fx_threads(NT, R))
 #pragma unroll
             for (int v = 0; v < R; v++) {
               const int t = j + v * T;
-              const double2 yA = s == 0 ? X(0)[t] : caxpy(X(0)[t], fac, K(0)[t]);
-              const double2 yB = s == 0 ? X(1)[t] : caxpy(X(1)[t], fac, K(1)[t]);
-              u[v] = make_double2(ri * cabs2(yA), ri * cabs2(yB));
+              double2 yA = X(0)[t], yB = X(1)[t];
+              if (s > 0) {   // the stage's input, kept in K's place for the product with the convolution
+                yA = caxpy(yA, fac, K(0)[t]);
+                yB = caxpy(yB, fac, K(1)[t]);
+                K(0)[t] = yA;
+                K(1)[t] = yB;
+              }
+              u[v] = make_double2(cabs2(yA), cabs2(yB));
+              if (scaled) u[v] = cscale(u[v], ri);
             }
           } else {
-            const double2 *x = X(c - 1), *k = K(c - 1);
+            const double2* y = s == 0 ? X(c - 1) : K(c - 1);
             const double* cv = U + (c - 1) * NT;
 #pragma unroll
             for (int v = 0; v < R; v++) {
               const int t = j + v * T;
-              const double2 y = s == 0 ? x[t] : caxpy(x[t], fac, k[t]);
-              u[v] = cscale(y, cv[t]);
+              u[v] = cscale(y[t], cv[t]);
             }
           }
           double2* acc = A(c == 2);
@@ -197,6 +203,7 @@ void add_kernels_fx_gnlse(std::vector<KernelEntry>& t) {
 #undef NLM_FX
   // key + kGenKey: grids that are not powers of two
   t.push_back({kKindFxGnlse, kChi3GNLSE + kGenKey, 8, (const void*)k_fx_gnlse<8, kFxGen>});
+  t.push_back({kKindFxGnlse, kChi3GNLSE + kConvKey, 8, (const void*)k_fx_gnlse<8, 0>});
 }
 
 }  // namespace nlm

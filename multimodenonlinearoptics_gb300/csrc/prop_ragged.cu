@@ -12,7 +12,7 @@
 // instead of the four stage evaluations.
 #include <vector>
 
-#include "nlm_propagate.cuh"
+#include "prop_fx.cuh"
 
 namespace nlm {
 
@@ -154,7 +154,50 @@ __global__ void __launch_bounds__(kMaxThreads) k_propagate_ragged(const PropArgs
   }
 }
 
+// The same with block fixed-point transforms (nlm_fx.cuh), for launches whose media share a grid of N = T R points.
+// A medium's march is bound by its SM's FP64 units (the RK4 step), so it wants four warps: R = 2 up to 256
+// points, 4 up to 2048, 8 at 4096.
+template <class S, int R>
+__global__ void __launch_bounds__(kMaxThreads) k_fx_ragged(const PropArgs* __restrict__ items, int nItems,
+                                                           unsigned long long* __restrict__ work) {
+  constexpr int M = S::kM;
+  extern __shared__ int4 fxsm[];
+  __shared__ PropArgs sa;
+  __shared__ int s_item;
+  const int j = threadIdx.x;
+  int item = blockIdx.x;
+  while (item < nItems) {
+    __syncthreads();  // the previous item's readers of sa are done
+    {
+      const unsigned* src = reinterpret_cast<const unsigned*>(items + item);
+      unsigned* dst = reinterpret_cast<unsigned*>(&sa);
+      for (int w = threadIdx.x; w < (int)(sizeof(PropArgs) / sizeof(unsigned)); w += blockDim.x) dst[w] = src[w];
+    }
+    __syncthreads();
+    const PropArgs& a = sa;
+    const int N = a.plan.N, T = a.plan.T;
+    FxField<0> f;
+    fx_begin(f, a.fx, a.plan, fxsm);
+    fx_propagate<M, R, 0>(a, f, 0, [&](int i, double2 (&x)[M][R]) {
+      if (a.prop) fx_matrix_step<M, R, 0>(a, i, N, T, j, x);
+      else fx_diffeq_step<S, R, 0>(a, i, N, T, j, x);
+    });
+    if (threadIdx.x == 0) s_item = (int)atomicAdd(work, 1ULL) + (int)gridDim.x;
+    __syncthreads();
+    item = s_item;
+  }
+}
+
 void add_kernels_ragged(std::vector<KernelEntry>& t) {
+  // key + kFxRaggedKey: block fixed-point transforms
+#define NLM_FX(S, id)                                                                        \
+  t.push_back({kKindRagged, id + kFxRaggedKey, 2, (const void*)k_fx_ragged<S, 2>});        \
+  t.push_back({kKindRagged, id + kFxRaggedKey, 4, (const void*)k_fx_ragged<S, 4>});        \
+  t.push_back({kKindRagged, id + kFxRaggedKey, 8, (const void*)k_fx_ragged<S, 8>});
+  NLM_FX(FChi3, kChi3)
+  NLM_FX(FChi2PDC, kChi2PDC)
+  NLM_FX(FChi2SFG, kChi2SFG)
+#undef NLM_FX
   t.push_back({kKindRagged, kChi3, 8, (const void*)k_propagate_ragged<FChi3, 8>});
   t.push_back({kKindRagged, kChi2PDC, 8, (const void*)k_propagate_ragged<FChi2PDC, 8>});
   t.push_back({kKindRagged, kChi2SFG, 8, (const void*)k_propagate_ragged<FChi2SFG, 8>});

@@ -65,8 +65,9 @@ def test_every_solver_matches_oracle(nlm, oracle, name, n):
             assert np.array_equal(out[k], out[ROWS - 2 + k])
 
 
-# every odd radix, alone and repeated, with each power-of-two part; 66 has a factor without a pass (FP64)
-GENERAL = [66, 70, 96, 100, 250, 294, 600, 1000, 1536, 2058, 4050]
+# every odd radix, alone and repeated, with each power-of-two part; then grids with a larger prime factor, in the
+# convolution form (its smallest and largest L)
+GENERAL = [70, 96, 100, 250, 294, 600, 1000, 1536, 2058, 4050, 66, 74, 502, 1022, 2042]
 
 
 @pytest.mark.parametrize("n", GENERAL)
