@@ -1409,12 +1409,38 @@ struct Medium {
       const FFTPlanH local = make_plan((int)N / kClusterSize, kClusterSize);
       ck(launch_pump_chi3_cluster(pumpFreq.p, pumpTime.p, de.p, dh.p, dd.p, db.p, dr.p, (int)nZP, local, tw, stream),
          "chi3 pump (cluster)");
+    } else if (const KernelEntry* k = fxPumpKernel()) {
+      // grids that are not powers of two, with block fixed-point transforms (prop_fx_pump.cu)
+      PropArgs a{};
+      a.plan = fxGenPlan(k->R);
+      a.fx = fxArgs(a.plan);
+      DevBuf<int4> tab;
+      std::vector<double2> all(hP);
+      all.insert(all.end(), dP.begin(), dP.end());
+      all.insert(all.end(), bP.begin(), bP.end());
+      int et = 0;
+      uploadFx(tab, &et, all);
+      if (!tab.p || et != 0) throw std::runtime_error("pump dispersion factors are not finite");
+      a.fx.tab = tab.p;
+      PumpMarchArgs p{pumpFreq.p, pumpTime.p, de.p, dh.p, dd.p, db.p, dr.p, (int)nZP};
+      size_t smem = 0;
+      ck(exclusive_smem(k->fn, fx_smem(fxConvSize() ? (int)fxConvL() : (int)N), &smem), "smem attribute");
+      if (smem == 0) throw Unsupported("grid too large for shared memory");
+      void* args[] = {(void*)&a, (void*)&p};
+      ck(cudaLaunchKernel(k->fn, dim3(1), dim3(a.plan.T), args, smem, stream), "chi3 pump");
+      sync("chi3 pump");   // tab goes out of scope
     } else {
       ck(launch_pump_chi3(pumpFreq.p, pumpTime.p, de.p, dh.p, dd.p, db.p, dr.p, (int)nZP, plan, tw, stream),
          "chi3 pump");
     }
     launches++;
     sync("chi3 pump");
+  }
+
+  const KernelEntry* fxPumpKernel() const {
+    if (!fxGenSize() || !fxGrid()) return nullptr;
+    int R = 0;
+    return fxKernel(kKindFxPump, fxConvSize() ? kConvKey : kGenKey, &R);
   }
 
   // The Chi3 pump march runs beside the next signal propagation: cluster mode 1, 128..1024 points (the

@@ -22,6 +22,7 @@ void add_kernels_fx_direct_a(std::vector<KernelEntry>& t);
 void add_kernels_fx_direct_b(std::vector<KernelEntry>& t);
 void add_kernels_fx_direct_c(std::vector<KernelEntry>& t);
 void add_kernels_fx_gnlse(std::vector<KernelEntry>& t);
+void add_kernels_fx_pump(std::vector<KernelEntry>& t);
 void add_kernels_direct_c(std::vector<KernelEntry>& t);
 void add_kernels_cluster(std::vector<KernelEntry>& t);
 void add_kernels_cluster_b(std::vector<KernelEntry>& t);
@@ -58,6 +59,7 @@ const KernelEntry* kernel_table(int* count) {
     add_kernels_fx_direct_b(table);
     add_kernels_fx_direct_c(table);
     add_kernels_fx_gnlse(table);
+    add_kernels_fx_pump(table);
     add_kernels_direct_c(table);
     add_kernels_cluster(table);
     add_kernels_cluster_b(table);

@@ -145,7 +145,8 @@ enum KernelKind : int {
   kKindSpreadFused = 8, // k_propagate_spread<Solver, C, M>  key as kKindCluster (R = 1): modes transformed together
   kKindFxLinear = 9,   // k_fx_linear<M, R, N>               key = modes + 1000 log2 N; args (PropArgs)
   kKindFxDirect = 10,  // k_fx_direct<Solver, R>             key = solver id; args (PropArgs)
-  kKindFxGnlse = 11    // k_fx_gnlse<R, N>                   key = solver id (+ 400: pairs) + 1000 log2 N; extra arg: scratch
+  kKindFxGnlse = 11,   // k_fx_gnlse<R, N>                   key = solver id (+ 400: pairs) + 1000 log2 N; extra arg: scratch
+  kKindFxPump = 12     // k_fx_pump_chi3<R, N>               key = kConvKey, kGenKey; args (PropArgs, PumpMarchArgs)
 };
 
 // Float-float copies (float4 {re.hi, re.lo, im.hi, im.lo} per complex value) of the tables of a

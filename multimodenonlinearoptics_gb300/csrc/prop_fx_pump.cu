@@ -1,0 +1,59 @@
+// prop_fx_pump.cu -- the Chi3 pump march (solvers/Chi3.cpp:41-70) on one CTA with block fixed-point transforms, for the
+// grids that the cluster kernels do not take: those that are not powers of two (general plan or convolution form).
+// The self-phase factor is FP64; 502 points x 199 rows: 90 ms with the FP64 general plan (a product per point and unit
+// of the factor 251).
+#include <vector>
+
+#include "prop_fx.cuh"
+
+namespace nlm {
+
+// a.plan, a.fx: the transform, with a.fx.tab the three tables [half, dstep, back][N] of modulus 1.
+template <int R, int NT>
+__global__ void __launch_bounds__(512) k_fx_pump_chi3(const PropArgs a, const PumpMarchArgs p) {
+  extern __shared__ int4 fxsm[];
+  FxField<NT> f;
+  fx_begin(f, a.fx, a.plan, fxsm);
+  const int N = f.grid, T = f.template T<R>(), j = f.j;
+  const double invN = 1.0 / N;
+  double2 x[R];
+  // row 0: half a dispersion step; rows 1 ..: self-phase, a step; then half of the last step back
+  for (int i = 0; i <= p.nRows; i++) {
+    const int row = min(i, p.nRows - 1);
+    const long long at = (long long)row * N;
+    const bool back = i == p.nRows;
+#pragma unroll
+    for (int v = 0; v < R; v++) {
+      const int t = j + v * T;
+      if (!f.has(t)) {
+        x[v] = czero();
+      } else if (i == 0) {
+        x[v] = p.env[t];
+      } else if (back) {
+        x[v] = p.pf[at + t];   // this thread's own points
+      } else {
+        const double2 r = p.rel[i - 1];
+        const double a2 = cabs2(x[v]);
+        x[v] = cmul(x[v], spm_factor(r.x * a2, r.y * a2));
+      }
+    }
+    fx_pair(f, a.fx, x, a.fx.tab + (long long)(back ? 2 : i == 0 ? 0 : 1) * N, 0, !back, true, true, [&](int v, double2 s) {
+      if (f.has(j + v * T)) p.pf[at + j + v * T] = s;
+    });
+#pragma unroll
+    for (int v = 0; v < R; v++) {
+      x[v] = cscale(x[v], invN);
+      if (f.has(j + v * T)) p.pt[at + j + v * T] = x[v];
+    }
+  }
+}
+
+void add_kernels_fx_pump(std::vector<KernelEntry>& t) {
+  // key: kConvKey the convolution form, kGenKey the general plan
+  t.push_back({kKindFxPump, kConvKey, 8, (const void*)k_fx_pump_chi3<8, 0>});
+  t.push_back({kKindFxPump, kConvKey, 4, (const void*)k_fx_pump_chi3<4, 0>});
+  t.push_back({kKindFxPump, kGenKey, 8, (const void*)k_fx_pump_chi3<8, kFxGen>});
+  t.push_back({kKindFxPump, kGenKey, 4, (const void*)k_fx_pump_chi3<4, kFxGen>});
+}
+
+}  // namespace nlm

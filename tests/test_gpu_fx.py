@@ -99,6 +99,17 @@ def test_general_grids_match_oracle(nlm, oracle, name, n):
             assert cases.rel_l2(med.signalFreqs(m), ref.signal_freq[m]) < TOL
 
 
+@pytest.mark.parametrize("n", [66, 70, 250, 600, 1022, 1536, 2042, 4050])
+def test_chi3_pump_march_on_general_grids(nlm, oracle, n):
+    """The pump march (self-phase factor, dispersion pair per row) in the general and the convolution form."""
+    kw = dict(relativeLength=1, nlLength=1, beta2=-1, beta3=0.1, pulseType=1, tMax=10, tPrecision=n, zPrecision=15)
+    med, ref = nlm.Chi3(**kw), oracle.Chi3(**kw)
+    med.runPumpSimulation()
+    ref.run_pump_simulation()
+    assert cases.rel_l2(med.pumpTime, ref.pump_time[0]) < TOL
+    assert cases.rel_l2(med.pumpFreq, ref.pump_freq[0]) < TOL
+
+
 @pytest.mark.parametrize("in_time", [False, True])
 @pytest.mark.parametrize("n", [128, 256, 512, 1024, 2048, 4096])
 def test_gnlse_matches_oracle(nlm, oracle, n, in_time):
