@@ -304,9 +304,12 @@ inline TwiddleCache g_twiddles;
 
 // A value as a Q62 integer relative to 2^et, in balanced halves (nlm_fx.cuh): exact for a double of
 // at most 2^et that is no smaller than 2^(et - 9), rounded to 2^(et - 62) below.
-inline int4 fx_quantise(long double re, long double im, int et) {
-  auto halves = [et](long double v, int& h, int& l) {
-    const long long q = std::llrint(std::ldexp(v, 62 - et));
+// T: double for tables of doubles; long double (software arithmetic on some hosts) for roots of unity only.
+template <class T>
+inline int4 fx_quantise(T re, T im, int et) {
+  const T scale = std::ldexp((T)1, 62 - et);
+  auto halves = [scale](T v, int& h, int& l) {
+    const long long q = std::llrint(v * scale);
     l = (int)(uint32_t)(unsigned long long)q;
     h = (int)((q - l) >> 32);
   };
@@ -325,7 +328,7 @@ struct FxTwiddleCache {
   static int4 root(int m, int n) {
     if (4LL * m % n == 0) {
       const int c[4] = {1, 0, -1, 0}, sn[4] = {0, -1, 0, 1}, t = (int)(4LL * m / n) % 4;
-      return fx_quantise(c[t], sn[t], 0);
+      return fx_quantise((double)c[t], (double)sn[t], 0);
     }
     const long double ang = -2.0L * 3.141592653589793238462643383279502884L * (long double)m / (long double)n;
     return fx_quantise(std::cos(ang), std::sin(ang), 0);
@@ -372,6 +375,63 @@ struct FxTwiddleCache {
   }
 };
 inline FxTwiddleCache g_fxTwiddles;
+
+// The chirp exp(-pi i t^2 / N), t < N, and the transform over L points of its conjugate divided by L (relative to
+// 2^et), for the convolution form of grids with a large prime factor; t^2 mod 2N is taken exactly.
+struct FxConvolution {
+  DevBuf<int4> chirp, conv;
+  int et = 0;
+};
+struct FxConvolutionCache {
+  std::mutex mu;
+  std::map<int, std::shared_ptr<FxConvolution>> tables;
+  const FxConvolution& get(int N, int L, cudaStream_t s) {
+    std::lock_guard<std::mutex> lock(mu);
+    auto it = tables.find(N);
+    if (it != tables.end()) return *it->second;
+    using C = std::complex<long double>;
+    const long double pi = 3.141592653589793238462643383279502884L;
+    std::vector<C> b(L), root(L / 2);
+    std::vector<int4> c, k;
+    for (long long t = 0; t < N; t++) {
+      const long double ang = pi * (long double)(t * t % (2LL * N)) / (long double)N;
+      b[t] = C(std::cos(ang), std::sin(ang));
+      if (t > 0) b[L - t] = b[t];
+      c.push_back(fx_quantise(b[t].real(), -b[t].imag(), 0));
+    }
+    for (int q = 0; q < L / 2; q++) root[q] = C(std::cos(-2 * pi * q / L), std::sin(-2 * pi * q / L));
+    for (int i = 1, r = 0; i < L; i++) {   // radix-2 transform of b
+      int bit = L >> 1;
+      for (; r & bit; bit >>= 1) r ^= bit;
+      r ^= bit;
+      if (i < r) std::swap(b[i], b[r]);
+    }
+    for (int len = 2; len <= L; len *= 2)
+      for (int i = 0; i < L; i += len)
+        for (int q = 0; q < len / 2; q++) {
+          const C u = b[i + q], v = b[i + q + len / 2], w = root[q * (L / len)];
+          const C p(v.real() * w.real() - v.imag() * w.imag(), v.real() * w.imag() + v.imag() * w.real());
+          b[i + q] = u + p;
+          b[i + q + len / 2] = u - p;
+        }
+    auto tab = std::make_shared<FxConvolution>();
+    double big = 0;
+    for (C& v : b) {
+      v /= (long double)L;
+      big = std::max(big, (double)std::hypot((double)v.real(), (double)v.imag()));
+    }
+    std::frexp(big, &tab->et);
+    for (const C& v : b) k.push_back(fx_quantise(v.real(), v.imag(), tab->et));
+    tab->chirp.alloc(c.size());
+    tab->conv.alloc(k.size());
+    ck(cudaMemcpyAsync(tab->chirp.p, c.data(), c.size() * sizeof(int4), cudaMemcpyHostToDevice, s), "chirp upload");
+    ck(cudaMemcpyAsync(tab->conv.p, k.data(), k.size() * sizeof(int4), cudaMemcpyHostToDevice, s), "chirp upload");
+    ck(cudaStreamSynchronize(s), "chirp upload");
+    tables[N] = tab;
+    return *tab;
+  }
+};
+inline FxConvolutionCache g_fxConvolutions;
 
 // Host memory that a cluster kernel raises when an exchange between its CTAs does not arrive in time (nlm_spread.cuh);
 // read after every wait for a stream.
@@ -723,12 +783,13 @@ struct Medium {
   const double2* tw = nullptr;
   DevBuf<double2> pumpFreq, pumpTime, sigFreq, sigTime;
   DevBuf<double2> dstep, dlast, half, back, coef, ramanD, steepD;
+  DevBuf<double2> pumpEnv;   // the envelope of the last linear pump simulation
   DevBuf<double> relIntD, dispPumpD, dispSignD, omegaD;
   // block fixed-point tables (dispStep, last, half) and their exponent; empty on grids without them
   DevBuf<int4> fxTab, fxRaman, fxSteep;
   const int4* spreadTwD = nullptr;
   const int4* fxRoots = nullptr;
-  DevBuf<int4> fxChirp, fxConv;
+  const int4 *fxChirp = nullptr, *fxConv = nullptr;
   int fxConvEt = 0;
   int fxEtRaman = 0, fxEtSteep = 0;
   bool fxBad = false;   // a table has values that are not finite: only the FP64 kernels take this medium
@@ -971,10 +1032,10 @@ struct Medium {
     double big = 0;
     for (const double2& v : h) {
       if (!std::isfinite(v.x) || !std::isfinite(v.y)) return;
-      big = std::max(big, std::hypot(v.x, v.y));
+      big = std::max(big, v.x * v.x + v.y * v.y);
     }
     if (!(big > 0) || !std::isfinite(big)) return;
-    std::frexp(big * (1 - 1e-15), et);
+    std::frexp(std::sqrt(big) * (1 - 1e-15), et);
     std::vector<int4> q;
     q.reserve(h.size() + kTablePad);
     for (const double2& v : h) q.push_back(fx_quantise(v.x, v.y, *et));
@@ -983,48 +1044,12 @@ struct Medium {
     ck(cudaMemcpyAsync(d.p, q.data(), q.size() * sizeof(int4), cudaMemcpyHostToDevice, stream), "upload");
     sync("upload");   // q goes out of scope
   }
-  // The chirp exp(-pi i t^2 / N), t < N, and the transform over L points of its conjugate (t^2 mod 2N taken exactly),
-  // divided by L.
+  // The tables of the convolution form (one set per grid size, per process).
   void buildConvolution() {
-    const long long L = fxConvL(), n = N;
-    std::vector<std::complex<long double>> b(L);
-    std::vector<double2> c(n), h(L);
-    std::vector<int4> q;
-    for (long long t = 0; t < n; t++) {
-      const long double ang = 3.141592653589793238462643383279502884L * (long double)(t * t % (2 * n)) / (long double)n;
-      const std::complex<long double> w(std::cos(ang), std::sin(ang));
-      q.push_back(fx_quantise(w.real(), -w.imag(), 0));
-      b[t] = w;
-      if (t > 0) b[L - t] = w;
-    }
-    q.resize(n + kTablePad);
-    fxChirp.alloc(q.size());
-    ck(cudaMemcpyAsync(fxChirp.p, q.data(), q.size() * sizeof(int4), cudaMemcpyHostToDevice, stream), "upload");
-    sync("convolution tables");
-    // radix-2 transform of b in extended precision
-    for (long long i = 1, r = 0; i < L; i++) {
-      long long bit = L >> 1;
-      for (; r & bit; bit >>= 1) r ^= bit;
-      r ^= bit;
-      if (i < r) std::swap(b[i], b[r]);
-    }
-    for (long long len = 2; len <= L; len *= 2) {
-      std::vector<std::complex<long double>> w(len / 2);
-      for (long long k = 0; k < len / 2; k++) {
-        const long double ang = -2.0L * 3.141592653589793238462643383279502884L * (long double)k / (long double)len;
-        w[k] = {std::cos(ang), std::sin(ang)};
-      }
-      for (long long i = 0; i < L; i += len)
-        for (long long k = 0; k < len / 2; k++) {
-          const auto u = b[i + k], v = b[i + k + len / 2];
-          const std::complex<long double> p(v.real() * w[k].real() - v.imag() * w[k].imag(),
-                                            v.real() * w[k].imag() + v.imag() * w[k].real());
-          b[i + k] = u + p;
-          b[i + k + len / 2] = u - p;
-        }
-    }
-    for (long long k = 0; k < L; k++) h[k] = make_double2((double)(b[k].real() / L), (double)(b[k].imag() / L));
-    uploadFx(fxConv, &fxConvEt, h);
+    const FxConvolution& c = g_fxConvolutions.get((int)N, (int)fxConvL(), stream);
+    fxChirp = c.chirp.p;
+    fxConv = c.conv.p;
+    fxConvEt = c.et;
   }
   void uploadD(DevBuf<double>& d, const std::vector<double>& h) {
     if (h.empty()) {
@@ -1316,6 +1341,23 @@ struct Medium {
     }
   }
 
+  // Row transforms: block fixed point on the grids that have it, each row with its own exponent.
+  void fftRows(const double2* in, double2* out, long long rows, bool inverse, double scale) {
+    int R = 0;
+    const KernelEntry* k = fxSize() ? findKernel(kKindFxRows, log2N(), 0)
+                           : fxGenSize() ? fxKernel(kKindFxRows, fxConvSize() ? kConvKey : kGenKey, &R) : nullptr;
+    if (!k) {
+      ck(launch_fft_rows(in, out, rows, fftPlanRows(), tw, inverse, scale, nullptr, stream), "row transforms");
+      return;
+    }
+    FFTPlanH plan = fxSize() ? make_plan((int)N, k->R) : fxGenPlan(k->R);
+    FxArgs fx = fxArgs(plan);
+    const Schedule s = schedule(k, rows, k->R);
+    int inv = inverse ? 1 : 0;
+    void* args[] = {(void*)&in, (void*)&out, (void*)&rows, (void*)&plan, (void*)&fx, (void*)&inv, (void*)&scale};
+    ck(cudaLaunchKernel(k->fn, dim3(s.grid), dim3(s.block), args, s.smem, stream), "row transforms");
+  }
+
   void runPump() {
     if (fnl || isCascade) throw std::runtime_error("Object does not have this method.");
     ensureDevice();
@@ -1323,18 +1365,16 @@ struct Medium {
       runPumpChi3();
     } else {
       // src/_NonlinearMedium.cpp:225-250
-      FFTPlanH plan = fftPlanRows();
-      DevBuf<double2> env;
       for (uint m = 0; m < nPump; m++) {
         std::vector<double2> e(N);
         for (uint k = 0; k < N; k++) e[k] = make_double2(envelope[m][k].real(), envelope[m][k].imag());
-        upload(env, e);
+        upload(pumpEnv, e);
         double2* pf = pumpFreq.p + (size_t)m * nZP * N;
         double2* pt = pumpTime.p + (size_t)m * nZP * N;
-        ck(launch_fft_rows(env.p, pf, 1, plan, tw, false, 1.0, nullptr, stream), "pump fft");
+        fftRows(pumpEnv.p, pf, 1, false, 1.0);
         ck(launch_pump_linear(pf, dispPumpD.p + (size_t)m * N, dzp, (int)nZP, (int)N, pf, stream), "pump phase");
-        if (nZP > 1) ck(launch_fft_rows(pf + N, pt + N, nZP - 1, plan, tw, true, 1.0 / N, nullptr, stream), "pump ifft");
-        ck(cudaMemcpyAsync(pt, env.p, N * sizeof(double2), cudaMemcpyDeviceToDevice, stream), "pump row 0");
+        if (nZP > 1) fftRows(pf + N, pt + N, nZP - 1, true, 1.0 / N);
+        ck(cudaMemcpyAsync(pt, pumpEnv.p, N * sizeof(double2), cudaMemcpyDeviceToDevice, stream), "pump row 0");
         launches += 3;
         if (profile != NLM_CONSTANT) {
           std::vector<double> s;
@@ -1490,7 +1530,7 @@ struct Medium {
     FFTPlanH plan = fftPlanRows();
     // rows 0..nZStepsP-2; the reference then re-transforms row nZSteps-1 (unchanged) and leaves the
     // last time-domain row as it was (src/_NonlinearMedium.cpp:533)
-    if (nZP > 1) ck(launch_fft_rows(pf, pt, nZP - 1, plan, tw, true, 1.0 / N, nullptr, stream), "pump from ifft");
+    if (nZP > 1) fftRows(pf, pt, nZP - 1, true, 1.0 / N);
     launches += 2;
     sync("pump from");
     pumpVersion++;
@@ -1583,7 +1623,8 @@ struct Medium {
   // override or the occupancy maximum), grid = SMs x CTAs per SM, capped by the number of groups.
   Schedule schedule(const KernelEntry* k, long long nInst, int R, int cta = 0, int ipcMul = 1) {
     int T = ((int)N + R - 1) / R;   // N / R on the register plan, ceil(N / R) on the general one
-    const bool fx = k->kind == kKindFxLinear || k->kind == kKindFxDirect || k->kind == kKindFxGnlse;
+    const bool fx = k->kind == kKindFxLinear || k->kind == kKindFxDirect || k->kind == kKindFxGnlse ||
+                    k->kind == kKindFxRows;
     if (fx && !is_pow2((int)N)) T = fxGenPlan(R).T;
     int ipc = fx ? 1 : (T >= 128 ? 1 : 128 / T) * ipcMul;
     if (ipc > nInst) ipc = (int)std::max<long long>(1, nInst);
@@ -1840,8 +1881,8 @@ struct Medium {
     if (!is_pow2(p.N) && fxConvSize()) {
       // a transform: two of L points, the product with conv and the closing chirp, both shifted back to 2^A0
       f.L = (int)fxConvL();
-      f.chirp = fxChirp.p;
-      f.conv = fxConv.p;
+      f.chirp = fxChirp;
+      f.conv = fxConv;
       f.lsL = f.ls;
       f.sh = 2 * f.sh + 2 * (2 - f.lsL) + fxConvEt;
       f.ls = 2;
@@ -2882,7 +2923,7 @@ struct Medium {
         prof = profD.p;
       }
       ck(launch_adj_pump_rows(adjGa.p, coef.p, prof, (int)nZ, (int)N, adjGP.p, stream), "pump rows");
-      ck(launch_fft_rows(adjGP.p, adjFGP.p, (long long)rowsP, fftPlanRows(), tw, false, 1.0, nullptr, stream), "fft");
+      fftRows(adjGP.p, adjFGP.p, (long long)rowsP, false, 1.0);
       ck(launch_adj_pump_reduce(adjFGP.p, dispPumpD.p, dzp, (int)rowsP, (int)N, gpump, stream), "pump reduce");
       launches += 3;
     }

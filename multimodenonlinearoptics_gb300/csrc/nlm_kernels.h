@@ -146,6 +146,7 @@ enum KernelKind : int {
   kKindFxLinear = 9,   // k_fx_linear<M, R, N>               key = modes + 1000 log2 N; args (PropArgs)
   kKindFxDirect = 10,  // k_fx_direct<Solver, R>             key = solver id; args (PropArgs)
   kKindFxGnlse = 11,   // k_fx_gnlse<R, N>                   key = solver id (+ 400: pairs) + 1000 log2 N; extra arg: scratch
+  kKindFxRows = 13,    // k_fx_rows<R, N>                    key = log2 N, kConvKey or kGenKey
   kKindFxPump = 12     // k_fx_pump_chi3<R, N>               key = kConvKey, kGenKey; args (PropArgs, PumpMarchArgs)
 };
 
