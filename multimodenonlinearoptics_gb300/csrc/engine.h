@@ -1905,6 +1905,19 @@ struct Medium {
     return nullptr;
   }
 
+  // Launches whose warps would fill less than half of the 16 per SM are bound by a march's latency: half the points
+  // per thread.  Chi2PDC, us per step, half against all: 256 points, 300 and 310 rows 3.1 and 5.7; 1024 points 8.7 and
+  // 11.0; beyond the line, 2048 points and 300 rows, 23.1 and 16.4.
+  bool fxFewWarps(long long nInst) const {
+    const long long threads = nSignal == 1 && N >= 256 ? N / 8 : N / 4;
+    return nInst * threads <= 32LL * 8 * smCount();
+  }
+  const KernelEntry* fxFew(int key, int* R) const {
+    const KernelEntry* k = findKernel(kKindFxLinear, key, 0);
+    if (k) *R = k->R;
+    return k;
+  }
+
   // The propagator's device buffer at its size, allocated ahead of a graph capture (which may not
   // allocate); buildPropagator then finds it in place.
   void reservePropagator() {
@@ -2277,7 +2290,10 @@ struct Medium {
       buildPropagator(R);
       a.prop = prop.p;
       int Rx = R;
-      if (!plainOne && !wantFF(R, a) && fxGrid() && (k = fxKernel(kKindFxLinear, (int)nSignal + 1000 * log2N(), &Rx))) {
+      if (!plainOne && !wantFF(R, a) && fxGrid() && fxFewWarps(nInst))
+        k = fxFew((int)nSignal + 500 + 1000 * log2N(), &Rx);
+      if (k || (!plainOne && !wantFF(R, a) && fxGrid() &&
+                (k = fxKernel(kKindFxLinear, (int)nSignal + 1000 * log2N(), &Rx)))) {
         a.plan = make_plan((int)N, Rx);
         a.R = Rx;
         a.fx = fxArgs(a.plan);

@@ -223,7 +223,7 @@ __device__ __forceinline__ void fx_fft_pow2(FxField<NT>& f, fxc (&x)[R]) {
   else if (r > 2 && mid == 2) pass(FxInt<2>{});
   if constexpr (NT > 0) {
 #pragma unroll
-    for (int p = 0; p < 6; p++)
+    for (int p = 0; p < 12; p++)
       if (L < N) pass(FxInt<r>{});
   } else {
 #pragma unroll 1

@@ -21,6 +21,17 @@ void add_kernels_fx(std::vector<KernelEntry>& t) {
   NLM_FX(2, 4, 11)
   NLM_FX(2, 8, 12)
 #undef NLM_FX
+  // + 500: half the points per thread, for launches that leave schedulers idle (engine.h, fxFew)
+#define NLM_FX(M, R, LOG) t.push_back({kKindFxLinear, M + 500 + 1000 * LOG, R, (const void*)k_fx_linear<M, R, 1 << LOG>});
+  NLM_FX(1, 2, 7)
+  NLM_FX(1, 4, 8)
+  NLM_FX(1, 4, 9)
+  NLM_FX(1, 4, 10)
+  NLM_FX(1, 4, 11)
+  NLM_FX(2, 2, 7)
+  NLM_FX(2, 2, 8)
+  NLM_FX(2, 2, 9)
+#undef NLM_FX
   // key + kGenKey: grids that are not powers of two
   t.push_back({kKindFxLinear, 1 + kGenKey, 8, (const void*)k_fx_linear<1, 8, kFxGen>});
   t.push_back({kKindFxLinear, 2 + kGenKey, 4, (const void*)k_fx_linear<2, 4, kFxGen>});

@@ -32,14 +32,16 @@ def test_propagator_batches_match_oracle(nlm, oracle, name, n, in_time):
     # a smooth field of a few pulse lengths, so that no step amplifies the grid's edge frequencies
     t = np.fft.fftshift(np.linspace(-8, 8, n, endpoint=False))
     x = cases.noise(np.random.default_rng(n), 3 * n * modes, 0.1).reshape(3, modes, n) * np.exp(-t ** 2)
-    x = np.tile(x.reshape(3, -1), (ROWS // 3 + 1, 1))
+    x = x.reshape(3, -1)
     if in_time:
-        x = np.fft.ifft(x.reshape(-1, modes, n), axis=2).reshape(x.shape)
-    out = med.batchSignalSimulation(x, in_time)
-    want = ref.batch_signal_simulation(x[:3], in_time)
-    for k in range(3):
-        assert cases.rel_l2(out[k], want[k]) < TOL
-        assert np.array_equal(out[k], out[k + 3])
+        x = np.fft.ifft(x.reshape(3, modes, n), axis=2).reshape(3, -1)
+    want = ref.batch_signal_simulation(x, in_time)
+    # few warps take half the points per thread up to 2048 points
+    for rows in (ROWS, 1500):
+        out = med.batchSignalSimulation(np.tile(x, (rows // 3, 1)), in_time)
+        for k in range(3):
+            assert cases.rel_l2(out[k], want[k]) < TOL
+            assert np.array_equal(out[k], out[k + 3])
 
 
 @pytest.mark.parametrize("n", [128, 512, 4096])
