@@ -187,7 +187,7 @@ def dist_info():
 
 def read_profile_value(key):
     """A figure of the committed ncu summary of the benchmark kernel (a line `key: value ...`)."""
-    path = os.path.join(ROOT, "profiles", "k_propagate_linear_green_n1024.md")
+    path = os.path.join(ROOT, "profiles", "k_fx_linear_green_n1024.md")
     if not os.path.exists(path):
         return None
     for line in open(path):
@@ -1019,15 +1019,17 @@ def run_ours(args):
             "gpu_launches": int(launches),
             "roofline": {"bound": "fp64", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
                          "frac": achieved / peak if peak else None, "traffic": traffic,
-                         "kernel": "k_propagate_linear<1,8>", "kernel_ms": 1e3 * avg_kernel_s,
+                         "kernel": "k_fx_linear<1,8,1024>", "kernel_ms": 1e3 * avg_kernel_s,
                          "algorithmic_flops_per_launch": flops,
-                         "traffic_source": "profile: dram__bytes_read.sum + write.sum of one ncu --set full capture "
+                         "traffic_source": "profile: dram__bytes_read.sum + write.sum of one ncu capture "
                                            "of this kernel on the same workload at nZSteps=50, scaled by 999/49 "
-                                           "(profiles/k_propagate_linear_green_n1024.md); not measured in this run",
+                                           "(profiles/k_fx_linear_green_n1024.md); not measured in this run",
                          "ncu_fp64_pipe_active_pct": read_profile_value("fp64_pipe_active_pct"),
                          "ncu_fp64_pipe_active_pct_source": "profile: the same nZSteps=50 capture; not measured in "
                                                             "this run",
                          "peak_source": "FP64 FMA chains measured in this run (MEASURED_PEAKS.json has no FP64 entry)",
+                         "note": "the transforms run on 64-bit integers (IMAD pipe), so the algorithmic flops exceed the "
+                                 "FP64 pipe's rate; the FP64 pipe carries the point-wise work only",
                          "secondary": {
                              "l2_gbs": (read_profile_value("l2_bytes_per_launch_full") or 0) / avg_kernel_s / 1e9
                              if avg_kernel_s and read_profile_value("l2_bytes_per_launch_full") else None,
