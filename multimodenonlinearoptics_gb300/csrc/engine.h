@@ -792,7 +792,6 @@ struct Medium {
   const int4 *fxChirp = nullptr, *fxConv = nullptr;
   int fxConvEt = 0;
   int fxEtRaman = 0, fxEtSteep = 0;
-  bool fxBad = false;   // a table has values that are not finite: only the FP64 kernels take this medium
   int fxEt = 0;
   DevBuf<double> prop;
   long long propVersion = -1, propBuilds = 0;
@@ -999,7 +998,6 @@ struct Medium {
       all.insert(all.end(), hl.begin(), hl.end());
       all.insert(all.end(), hh.begin(), hh.end());
       uploadFx(fxTab, &fxEt, all);
-      fxBad = !fxTab.p;
     }
     std::vector<double> hdp, hds;
     for (auto& v : dispPump) hdp.insert(hdp.end(), v.begin(), v.end());
@@ -1249,7 +1247,6 @@ struct Medium {
     if (fxTab.p) {
       uploadFx(fxRaman, &fxEtRaman, rs);
       uploadFx(fxSteep, &fxEtSteep, st);
-      fxBad = !fxRaman.p || !fxSteep.p;
     }
     std::vector<double> rel((size_t)(nZ > 1 ? nZ - 1 : 0) * 3);
     for (uint i = 1; i < nZ; i++) {
@@ -1844,6 +1841,9 @@ struct Medium {
       while (n % q == 0) n /= q;
     return n == 1;
   }
+  // Whether this medium has its integer tables.  Every form that reads a.fx.tab, a.fx.raman or a.fx.steep asks: they
+  // are not built for one z step (an infinite step length) nor from values that are not finite, and such media run the
+  // FP64 kernels.
   bool fxGrid() const { return fxTab.p && (solver != kChi3GNLSE || (fxRaman.p && fxSteep.p)); }
   // the N-point twiddles of the one-point-per-thread cluster kernels (null on grids without them)
   const int4* spreadTw() const { return spreadTwD; }
@@ -1964,13 +1964,13 @@ struct Medium {
   // cluster mode 3 is mode 1 without the widest forms (sixteen CTAs on 2048 and 4096 points, eight on
   // 1024): four CTAs up to 1024 points and eight above, as a reference for them
   bool spreadGrid() const {
-    return (useCluster == 1 || useCluster == 3) && !fxBad && is_pow2((int)N) && N >= kSpreadMinN && N <= kSpreadMaxN;
+    return (useCluster == 1 || useCluster == 3) && fxGrid() && is_pow2((int)N) && N >= kSpreadMinN && N <= kSpreadMaxN;
   }
   // 2048- and 4096-point grids: one point per thread on eight CTAs (prop_spread_b.cu), twice the SMs of
   // the four-points-per-thread cluster, for the launches that no reverse sweep pairs with (full grids,
   // the media of ragged batches marked by raggedWide) and the Chi3 pump march.
   bool wideGrid() const {
-    return (useCluster == 1 || useCluster == 3) && !fxBad && is_pow2((int)N) && N > kSpreadMaxN && N <= kWideMaxN;
+    return (useCluster == 1 || useCluster == 3) && fxGrid() && is_pow2((int)N) && N > kSpreadMaxN && N <= kWideMaxN;
   }
   bool wideLaunch(const PropArgs& a) const {
     return wideGrid() && !a.ckpt && !a.stages && (a.gridF || a.gridT || raggedWide || raggedW16);
@@ -1978,7 +1978,7 @@ struct Medium {
   // Grids that take eight CTAs with one point per thread: 2048 and 4096 points, and in cluster mode 1
   // also 1024 points (128 per CTA) for full grids and the ragged media a plan gives that form
   bool w8Grid() const {
-    return wideGrid() || (useCluster == 1 && N == kSpreadMaxN);
+    return wideGrid() || (useCluster == 1 && N == kSpreadMaxN && fxGrid());
   }
   bool w8Launch(const PropArgs& a) const {
     if (!w8Grid() || a.ckpt || a.stages) return false;
@@ -2031,7 +2031,7 @@ struct Medium {
   // least 128 threads per CTA (at most 256 on sixteen CTAs, 512 otherwise); 0 when none applies (then
   // four points per thread on four CTAs).  The stored-stage reverse sweep takes the same form.
   int gnlseSpreadC(long long rows) const {
-    if (solver != kChi3GNLSE || useCluster != 1 || fxBad || !is_pow2((int)N)) return 0;
+    if (solver != kChi3GNLSE || useCluster != 1 || !fxGrid() || !is_pow2((int)N)) return 0;
     for (int C : {16, 8, 4}) {
       const int M = (int)N / C;
       if (M < 128 || M > (C == 16 ? 256 : 512) || rows * C > smCount()) continue;
@@ -2048,7 +2048,6 @@ struct Medium {
     // checkpointed forwards (the adjoint's, Chi2PDC and Chi3GNLSE) run on clusters too: their reverse
     // sweeps have cluster forms that read the same checkpoints
     if (!useCluster || plainOne || a.inKind != 1) return nullptr;
-    if (fxBad) return nullptr;
     if (!is_pow2((int)N) || N > (uint)kMaxFFT) return nullptr;
     if (const int Cs = gnlseSpreadC(nInst))
       return Cs == 16 ? findKernel(kKindCluster, solver + kSpreadW16Key, 1)
@@ -2540,7 +2539,7 @@ struct Medium {
   // Stage values of every Chi3GNLSE step fit (at most a quarter of the free device memory and 64 GB),
   // and the forward of `rows` propagations runs on 4-CTA clusters (Medium::clusterKernel).
   bool storeStages(size_t rows) const {
-    if (solver != kChi3GNLSE || !useCluster || fxBad || !is_pow2((int)N) || N < 1024 || N > (uint)kMaxFFT) return false;
+    if (solver != kChi3GNLSE || !useCluster || !is_pow2((int)N) || N < 1024 || N > (uint)kMaxFFT) return false;
     if ((long long)rows * kClusterSize > smCount()) return false;
     if (!findKernel(kKindCluster, solver, kClusterSize) || !findKernel(kKindAdjoint, solver + 300, kClusterSize))
       return false;
@@ -2622,7 +2621,7 @@ struct Medium {
   // such clusters fit on the device at once, or a grid outside its range).
   bool adjointCluster(const double2* gout, double2* gin) {
     constexpr int C = kClusterSize;
-    if (solver != kChi3GNLSE || !useCluster || fxBad || !is_pow2((int)N) || N < 1024 || N > (uint)kMaxFFT) return false;
+    if (solver != kChi3GNLSE || !useCluster || !is_pow2((int)N) || N < 1024 || N > (uint)kMaxFFT) return false;
     const KernelEntry* k = findKernel(kKindAdjoint, solver + 200, C);
     if (!k) return false;
     const int M = (int)N / C;
@@ -2717,7 +2716,7 @@ struct Medium {
     bool staged = false;
     const char* ctasEnv = std::getenv("NLM_ADJOINT_CTAS");
     const int ctasWant = ctasEnv ? std::atoi(ctasEnv) : 12;
-    const bool pointGrid = spread || (useCluster == 1 && N == 2 * kSpreadMaxN);
+    const bool pointGrid = spread || (useCluster == 1 && N == 2 * kSpreadMaxN && fxGrid());
     int T1 = T, R1 = Rk;
     for (int G = 1; G <= 2 && adjK > 1 && pointGrid && a.prop && !staged; G++) {
       const int size = (2 + G) * C;

@@ -1,0 +1,86 @@
+"""Media, fields and calls at the edges of the block fixed-point kernels (csrc/nlm_fx.cuh, csrc/nlm_spread.cuh)."""
+import numpy as np
+import pytest
+
+import cases
+
+pytestmark = pytest.mark.gpu
+
+GNLSE = dict(nlLength=1, selfSteepLength=5, fr=0.18, fb=0.21, tau1=0.0155, tau2=0.2165, tau3=0.4, beta2=-1, beta3=0.05)
+PDC = dict(relativeLength=1, nlLength=0.5, beta2=1, beta2s=0.5, beta1s=2, tMax=40, zPrecision=10)
+SFG = dict(relativeLength=1, nlLength=0.8, nlLengthOrig=1.2, beta2=0.5, beta2s=-0.3, beta2o=0.2, beta1s=1, tMax=20,
+           zPrecision=10)
+
+
+# ---- media without integer tables: FP64 kernels in every form -----------------------------------------------------
+
+@pytest.mark.parametrize("n", [128, 512, 1024, 2048, 4096])
+def test_one_step_gnlse(nlm, oracle, n):
+    """One z step has an infinite step length, and no integer tables: full grids and few-row batches run the FP64
+    kernels (never one point per thread), NaN where the oracle is."""
+    kw = dict(GNLSE, relativeLength=1, tMax=10, tPrecision=n, zPrecision=1)
+    med, ref = nlm.Chi3GNLSE(**kw), oracle.Chi3GNLSE(**kw)
+    assert med._dims["nZSteps"] == 1
+    x = cases.noise(np.random.default_rng(n), 3 * n, 1.0).reshape(3, n)
+    for in_time in (False, True):
+        med.runSignalSimulation(x[0], in_time)
+        assert med._last_schedule()["R"] > 1
+        out = med.batchSignalSimulation(x, in_time)
+        assert med._last_schedule()["R"] > 1
+        with np.errstate(all="ignore"):
+            ref.run_signal_simulation(x[0], in_time)
+            want = ref.batch_signal_simulation(x, in_time)
+        assert np.array_equal(np.isnan(out), np.isnan(want))
+        assert np.array_equal(np.isnan(med.signalFreq), np.isnan(ref.signal_freq[0]))
+    import torch
+    from multimodenonlinearoptics_gb300.autograd import propagate_gnlse
+    with pytest.raises(ValueError):
+        propagate_gnlse(med, torch.zeros((1, n), dtype=torch.complex128, device="cuda"))
+
+
+@pytest.mark.parametrize("interval", [0, 4])
+@pytest.mark.parametrize("n", [128, 1024, 2048, 4096])
+@pytest.mark.parametrize("name", ["Chi2PDC", "Chi3GNLSE"])
+def test_dispersion_that_is_not_finite(nlm, name, n, interval):
+    """A NaN dispersion parameter (an optimiser's step) leaves no integer tables: full grids, batches and gradients come
+    back NaN from the FP64 kernels."""
+    import torch
+    from multimodenonlinearoptics_gb300.autograd import propagate_gnlse, propagate_pdc
+    nan = float("nan")
+    if name == "Chi2PDC":
+        med = nlm.Chi2PDC(**dict(PDC, beta2s=nan, tPrecision=n))
+    else:
+        med = nlm.Chi3GNLSE(**dict(GNLSE, relativeLength=1, beta2=nan, tMax=10, tPrecision=n, zPrecision=10))
+    assert med._dims["nZSteps"] > 9
+    x = cases.noise(np.random.default_rng(n), 2 * n, 0.1).reshape(2, n)
+    med.runSignalSimulation(x[0])
+    assert med._last_schedule()["R"] > 1 and np.all(np.isnan(med.signalFreq))
+    out = med.batchSignalSimulation(x, True)
+    assert med._last_schedule()["R"] > 1 and np.all(np.isnan(out))
+    xt = torch.tensor(x, device="cuda").requires_grad_()
+    if name == "Chi2PDC":
+        pump = torch.ones(n, dtype=torch.complex128, device="cuda")
+        y = propagate_pdc(med, xt, pump, torch.ones(med._dims["nZSteps"], dtype=torch.float64, device="cuda"), interval)
+    else:
+        y = propagate_gnlse(med, xt, interval)
+    grad, = torch.autograd.grad(torch.sum(torch.abs(y) ** 2), xt)
+    assert med._last_schedule()["R"] > 1
+    assert torch.isnan(y).all() and torch.isnan(grad).all()
+
+
+def test_ragged_set_with_a_medium_without_tables(nlm, oracle):
+    """The planner gives a medium without integer tables no one-point-per-thread slot; its neighbours are unaffected."""
+    media, refs, xs = [], [], []
+    for k, n in enumerate((1024, 512, 1024, 2048)):
+        kw = dict(SFG, tPrecision=n, beta2s=float("nan") if k in (0, 3) else -0.3)
+        media.append(nlm.Chi2SFG(**kw))
+        refs.append(oracle.Chi2SFG(**kw))
+        xs.append(cases.noise(np.random.default_rng(k), n, 0.1))
+        media[k].runPumpSimulation()
+    out = nlm.ragged_batch(media, xs)
+    for k in (0, 3):
+        assert np.all(np.isnan(out[k]))
+    for k in (1, 2):
+        refs[k].run_pump_simulation()
+        want = refs[k].batch_signal_simulation(xs[k][None], False, False)[0]
+        assert cases.rel_l2(out[k].ravel(), want.ravel()) < 1e-12   # 20 steps, as in test_gpu_fx.py
