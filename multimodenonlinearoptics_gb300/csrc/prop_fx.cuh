@@ -70,6 +70,8 @@ __device__ __forceinline__ void fx_pair(FxField<NT>& f, const FxArgs& fx, double
     for (int v = 0; v < R; v++) y[v] = fxc{y[v].y, y[v].x};
   }
   if (inv) fx_leave<R>(y, x, k, bad);
+  // without a transform no barrier has followed fx_norm's reads of f.red, which the next field's norm writes
+  if (!fwd && !inv) __syncthreads();
 }
 
 // One propagation.

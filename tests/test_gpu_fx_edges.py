@@ -84,3 +84,29 @@ def test_ragged_set_with_a_medium_without_tables(nlm, oracle):
         refs[k].run_pump_simulation()
         want = refs[k].batch_signal_simulation(xs[k][None], False, False)[0]
         assert cases.rel_l2(out[k].ravel(), want.ravel()) < 1e-12   # 20 steps, as in test_gpu_fx.py
+
+
+# ---- rows that share a CTA ----------------------------------------------------------------------------------------
+
+@pytest.mark.parametrize("in_time", [False, True])
+@pytest.mark.parametrize("n", [128, 512, 1024, 4096])
+def test_paired_rows_of_very_different_norm(nlm, oracle, n, in_time):
+    """Two GNLSE rows per CTA, one ten decades below the other: each keeps its own exponent to the last step (a row
+    rounded with its partner's would be off by 1e10 x 2^-60 = 1e-8), and repeated calls agree bit by bit.  40 steps:
+    tolerance as in test_gpu_fx.py."""
+    kw = dict(cases.CASES["Chi3GNLSE"], tPrecision=n, zPrecision=2000, relativeLength=0.02, tMax=20)
+    med, ref = nlm.Chi3GNLSE(**kw), oracle.Chi3GNLSE(**kw)
+    med._set_cluster(0)
+    rows, rng = 331, np.random.default_rng(n)   # 165 pairs and a last row whose partner is idle
+    t = np.fft.fftshift(np.linspace(-20, 20, n, endpoint=False))
+    x = rng.uniform(0.5, 1.5, (rows, 1)) / np.cosh(t)[None, :] + cases.noise(rng, rows * n, 1e-3).reshape(rows, n)
+    x[0:100:2] *= 1e-10   # the pair's first row, then its second
+    x[101:200:2] *= 1e-10
+    x = x if in_time else np.fft.fft(x, axis=1)
+    out = med.batchSignalSimulation(x, in_time)
+    pick = [0, 1, 2, 100, 101, 198, 199, 200, 329, 330]
+    want = ref.batch_signal_simulation(x[pick], in_time)
+    for k, p in enumerate(pick):
+        assert cases.rel_l2(out[p], want[k]) < 1e-12
+    for _ in range(4):
+        assert np.array_equal(med.batchSignalSimulation(x, in_time), out)
