@@ -1454,7 +1454,6 @@ struct Medium {
       DevBuf<int4> tab;
       std::vector<double2> all(hP);
       all.insert(all.end(), dP.begin(), dP.end());
-      all.insert(all.end(), bP.begin(), bP.end());
       int et = 0;
       uploadFx(tab, &et, all);
       if (!tab.p || et != 0) throw std::runtime_error("pump dispersion factors are not finite");

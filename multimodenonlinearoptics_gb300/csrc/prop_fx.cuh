@@ -2,7 +2,7 @@
 //
 // One CTA of T = N / R threads runs one propagation at a time, groups claimed like in nlm_propagate.cuh.  The march
 // is a loop over stages so that the kernel holds one forward and one inverse transform:
-//   stage 0:        [forward if the input is in the time domain]  x exp(+i dz/2 D)
+//   stage 0:        [forward if the input is in the time domain]  x exp(+i dz/2 D) (of a spectrum: in FP64)
 //   stage i:        RK4 step i point-wise in FP64, forward, x dispStep (the last stage's with exp(-i dz/2 D))
 // (nZ > 1), each followed by the inverse transform unless it is the last and only the spectrum is wanted.
 #pragma once
@@ -39,27 +39,29 @@ __device__ __forceinline__ int4 fx_load(const FxField<NT>& f, const int4* __rest
   return __ldg(table + (NT <= 0 ? min(t, f.grid - 1) : t));
 }
 
-// One mode through [forward] x table [inverse].  spec(v, value) receives the spectrum (1/N folded in, as the tables
-// have it) when wantF; x is the field after the inverse, or the spectrum without it.
+// One mode through [forward x table] [inverse].  spec(v, value) receives the spectrum (1/N folded in, as the tables
+// have it) when wantF; x is the field after the inverse, or the spectrum without it.  Without the forward transform x
+// is a spectrum times its factors: their product is FP64's, since a spectrum that no transform has rounded relative to
+// its norm would lose bits of its small values here.
 template <int R, int NT, class Spec>
 __device__ __forceinline__ void fx_pair(FxField<NT>& f, const FxArgs& fx, double2 (&x)[R], const int4* __restrict__ table,
                                         int et, bool fwd, bool inv, bool wantF, Spec spec) {
+  if (!fwd && !inv) return;
   fxc y[R];
   int lift;
   const int a = fx_enter(f, x, y, fx.A0, &lift);
   const bool bad = a > 2200;
-  int k = a - 1023 - fx.A0 + et - lift;
-  const int ls = fwd ? fx.ls : 2;
+  int k = a - 1023 - fx.A0 - lift;
 #pragma unroll 1
   for (int dir = 0; dir < 2; dir++) {
     if (dir == 0 ? fwd : inv) {
       fx_fft(f, y);
       k += fx.sh;
     }
-    if (dir == 0) {
-      k += 2 - ls;
+    if (dir == 0 && fwd) {
+      k += et + 2 - fx.ls;
 #pragma unroll
-      for (int v = 0; v < R; v++) y[v] = fx_cmul(y[v], fx_load(f, table, f.j + v * f.template T<R>()), ls);
+      for (int v = 0; v < R; v++) y[v] = fx_cmul(y[v], fx_load(f, table, f.j + v * f.template T<R>()), fx.ls);
       if (wantF) {
         fx_leave<R>(y, x, k, bad);
 #pragma unroll
@@ -70,8 +72,6 @@ __device__ __forceinline__ void fx_pair(FxField<NT>& f, const FxArgs& fx, double
     for (int v = 0; v < R; v++) y[v] = fxc{y[v].y, y[v].x};
   }
   if (inv) fx_leave<R>(y, x, k, bad);
-  // without a transform no barrier has followed fx_norm's reads of f.red, which the next field's norm writes
-  if (!fwd && !inv) __syncthreads();
 }
 
 // One propagation.
@@ -101,6 +101,17 @@ __device__ __forceinline__ void fx_propagate(const PropArgs& a, FxField<NT>& f, 
 #pragma unroll
       for (int v = 0; v < R; v++) x[m][v] = seg >= 0 && f.has(j + v * T) ? row[(long long)seg * N + j + v * T] : czero();
     }
+  }
+  if (!a.inTime) {
+#pragma unroll
+    for (int m = 0; m < M; m++)
+#pragma unroll
+      for (int v = 0; v < R; v++) {
+        const int t = j + v * T;
+        if (!f.has(t)) continue;
+        x[m][v] = cmul(x[m][v], __ldg(a.half + (long long)m * N + t));
+        if (a.gridF) a.gridF[m * ms + t] = cscale(x[m][v], (double)N);
+      }
   }
   for (int i = 0; i <= last; i++) {
     if (i > 0) point(i, x);

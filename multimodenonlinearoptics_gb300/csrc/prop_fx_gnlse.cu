@@ -19,10 +19,18 @@ __device__ __forceinline__ void fx_gnlse_load(const PropArgs& a, FxField<NT>& f,
   double2 x[R];
 #pragma unroll
   for (int v = 0; v < R; v++) x[v] = active && a.inChannels > 0 && f.has(j + v * T) ? a.in[inst * a.inStride + j + v * T] : czero();
-  fx_pair(f, a.fx, x, a.fx.tab + 2LL * N, a.fx.et, a.inTime != 0, true, true, [&](int v, double2 s) {
+  auto spectrum = [&](int v, double2 s) {
     XF[j + v * T] = s;
     if (a.gridF && active && f.has(j + v * T)) a.gridF[j + v * T] = cscale(s, (double)N);
-  });
+  };
+  if (!a.inTime) {
+#pragma unroll
+    for (int v = 0; v < R; v++) {
+      if (f.has(j + v * T)) x[v] = cmul(x[v], __ldg(a.half + j + v * T));
+      spectrum(v, x[v]);
+    }
+  }
+  fx_pair(f, a.fx, x, a.fx.tab + 2LL * N, a.fx.et, a.inTime != 0, true, true, spectrum);
 #pragma unroll
   for (int v = 0; v < R; v++) {
     X[j + v * T] = x[v];
@@ -32,20 +40,24 @@ __device__ __forceinline__ void fx_gnlse_load(const PropArgs& a, FxField<NT>& f,
   }
 }
 
-// The end of step i: the dispersion factors on the spectrum of x + sum / 6, N (XF + A / 6); then back to time.
+// The end of step i: the dispersion factors on the spectrum of x + sum / 6, N (XF + A / 6), which stays in FP64 from
+// step to step; then back to time.
 template <int R, int NT>
 __device__ __forceinline__ void fx_gnlse_end(const PropArgs& a, FxField<NT>& f, int i, long long inst, bool active,
                                              double2* XF, const double2* A, double2* X) {
   const int N = NT > 0 ? NT : f.grid, T = f.template T<R>(), j = f.j;
   const bool last = i == a.nZ - 1;
+  const double2* table = last ? a.dlast : a.dstep;
   double2 x[R];
 #pragma unroll
-  for (int v = 0; v < R; v++) x[v] = cscale(caxpy(XF[j + v * T], 1.0 / 6.0, A[j + v * T]), (double)N);
+  for (int v = 0; v < R; v++) {
+    const int t = j + v * T;
+    x[v] = f.has(t) ? cmul(cscale(caxpy(XF[t], 1.0 / 6.0, A[t]), (double)N), __ldg(table + t)) : czero();
+    XF[t] = x[v];
+    if (a.gridF && active && f.has(t)) a.gridF[(long long)i * N + t] = cscale(x[v], (double)N);
+  }
   const bool inv = !last || a.inTime || a.gridT != nullptr;
-  fx_pair(f, a.fx, x, a.fx.tab + (last ? N : 0), a.fx.et, false, inv, true, [&](int v, double2 s) {
-    XF[j + v * T] = s;
-    if (a.gridF && active && f.has(j + v * T)) a.gridF[(long long)i * N + j + v * T] = cscale(s, (double)N);
-  });
+  fx_pair(f, a.fx, x, a.fx.tab, a.fx.et, false, inv, false, [](int, double2) {});
 #pragma unroll
   for (int v = 0; v < R; v++) {
     const int t = j + v * T;

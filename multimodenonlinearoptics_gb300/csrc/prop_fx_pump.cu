@@ -13,7 +13,7 @@
 
 namespace nlm {
 
-// a.plan, a.fx: the transform, with a.fx.tab the three tables [half, dstep, back][N] of modulus 1.
+// a.plan, a.fx: the transform, with a.fx.tab the tables [half, dstep][N] of modulus 1.
 template <int R, int NT>
 __global__ void __launch_bounds__(512) k_fx_pump_chi3(const PropArgs a, const PumpMarchArgs p) {
   extern __shared__ int4 fxsm[];
@@ -34,15 +34,16 @@ __global__ void __launch_bounds__(512) k_fx_pump_chi3(const PropArgs a, const Pu
         x[v] = czero();
       } else if (i == 0) {
         x[v] = p.env[t];
-      } else if (back) {
-        x[v] = p.pf[at + t];   // this thread's own points
+      } else if (back) {   // this thread's own points, as they are in FP64
+        x[v] = cmul(p.pf[at + t], p.backP[t]);
+        p.pf[at + t] = x[v];
       } else {
         const double2 r = p.rel[i - 1];
         const double a2 = cabs2(x[v]);
         x[v] = cmul(x[v], spm_factor(r.x * a2, r.y * a2));
       }
     }
-    fx_pair(f, a.fx, x, a.fx.tab + (long long)(back ? 2 : i == 0 ? 0 : 1) * N, 0, !back, true, true, [&](int v, double2 s) {
+    fx_pair(f, a.fx, x, a.fx.tab + (long long)(i == 0 ? 0 : 1) * N, 0, !back, true, true, [&](int v, double2 s) {
       if (f.has(j + v * T)) p.pf[at + j + v * T] = s;
     });
 #pragma unroll

@@ -110,3 +110,42 @@ def test_paired_rows_of_very_different_norm(nlm, oracle, n, in_time):
         assert cases.rel_l2(out[p], want[k]) < 1e-12
     for _ in range(4):
         assert np.array_equal(med.batchSignalSimulation(x, in_time), out)
+
+
+# ---- spectra that no transform has rounded ------------------------------------------------------------------------
+
+def _wide_spectrum(n, rows):
+    """Bins from 1 down to 1e-25, far below the last bit of the row's norm."""
+    rng = np.random.default_rng(n)
+    phase = np.exp(2j * np.pi * rng.uniform(size=(rows, n)))
+    return phase * 10.0 ** (-25 * np.abs(np.fft.fftfreq(n)) * 2)[None, :]
+
+
+@pytest.mark.parametrize("n", [100, 128, 600, 1022, 1024, 4096])
+@pytest.mark.parametrize("name", ["Chi2PDC", "Chi2SFG", "Chi3GNLSE"])
+def test_first_row_of_a_spectrum_keeps_every_bin(nlm, name, n):
+    """Row 0 of the spectrum grid is the input spectrum times a phase, bin by bin.  Modulus to 1.2e-15: the factor's
+    parts (2.2e-16), its 1/N, the product (2.2e-16), the N, and the test's own two moduli (2.2e-16 each) and ratio."""
+    kw = {"Chi2PDC": PDC, "Chi2SFG": SFG,
+          "Chi3GNLSE": dict(GNLSE, relativeLength=1, tMax=10, zPrecision=10)}[name]
+    med = getattr(nlm, name)(**dict(kw, tPrecision=n))
+    x = _wide_spectrum(n, 1)[0]
+    for cluster in (0, 1):
+        med._set_cluster(cluster)
+        med.runSignalSimulation(x, False)
+        got = np.abs(med.signalFreqs(0)[0])
+        assert np.max(np.abs(got / np.abs(x) - 1)) < 1.2e-15
+
+
+@pytest.mark.parametrize("rows", [3, 161])
+@pytest.mark.parametrize("n", [128, 600, 1022, 1024, 4096])
+def test_gnlse_spectrum_keeps_every_bin(nlm, n, rows):
+    """A nearly linear medium: the state's spectrum takes a phase per step and keeps every bin's modulus.  A step rounds
+    its factor (3.3e-16 in all), sum, scaling and product (1.1, 1.1 and 2.2e-16), 41 times at most: 3.2e-14."""
+    med = nlm.Chi3GNLSE(**dict(GNLSE, nlLength=1e30, selfSteepLength=1e30, relativeLength=1, tMax=10, tPrecision=n,
+                               zPrecision=40))
+    assert med._dims["nZSteps"] <= 41
+    med._set_cluster(0)
+    x = _wide_spectrum(n, rows)
+    out = med.batchSignalSimulation(x)
+    assert np.max(np.abs(np.abs(out) / np.abs(x) - 1)) < 3.2e-14
