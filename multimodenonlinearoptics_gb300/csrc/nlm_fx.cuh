@@ -362,23 +362,39 @@ __device__ __forceinline__ long long fx_dot(const int (&ah)[n], const int (&al)[
   return acc;
 }
 
+// The sum of v[0 .. n - 1] / 4, rounded to nearest, ties to even: the quarters and the remainders apart, since the sum
+// itself can pass 2^63 (sqrt(r) times a norm of 2^62, for a field that a butterfly gathers in one point).
+template <int n>
+__device__ __forceinline__ long long fx_quarter_sum(const long long (&v)[n]) {
+  long long q = 0;
+  int rem = 0;
+#pragma unroll
+  for (int k = 0; k < n; k++) {
+    q += v[k] >> 2;
+    rem += (int)v[k] & 3;
+  }
+  return q + ((rem + 1 + (((int)q + (rem >> 2)) & 1)) >> 2);
+}
+
 // r-point DFT / 4, r an odd prime.  With a_q = x_q + x_(r-q), b_q = x_q - x_(r-q), y_s and y_(r-s) are
 // x_0 + sum cos(2 pi q s / r) a_q -+ i sum sin(2 pi q s / r) b_q.  root: cos and -sin of 2 pi q / r in Q62 halves.
 template <int r>
 __device__ __forceinline__ void fx_odd_dft(fxc (&x)[r], const int4* root) {
   constexpr int h = (r - 1) / 2;
   int axh[h], axl[h], ayh[h], ayl[h], bxh[h], bxl[h], byh[h], byl[h];
-  fxc s0 = fx_shift(x[0], 2), sum = x[0];
+  const fxc s0 = fx_shift(x[0], 2);
+  long long sx[h + 1] = {x[0].x}, sy[h + 1] = {x[0].y};
 #pragma unroll
   for (int q = 1; q <= h; q++) {
     const fxc a = fxadd(x[q], x[r - q]), b = fxsub(x[q], x[r - q]);
-    sum = fxadd(sum, a);
+    sx[q] = a.x;
+    sy[q] = a.y;
     fx_split(a.x, axh[q - 1], axl[q - 1]);
     fx_split(a.y, ayh[q - 1], ayl[q - 1]);
     fx_split(b.x, bxh[q - 1], bxl[q - 1]);
     fx_split(b.y, byh[q - 1], byl[q - 1]);
   }
-  x[0] = fx_shift(sum, 2);
+  x[0] = fxc{fx_quarter_sum(sx), fx_quarter_sum(sy)};
 #pragma unroll
   for (int s = 1; s <= h; s++) {
     int2 cs[h], sn[h];

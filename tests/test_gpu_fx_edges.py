@@ -149,3 +149,40 @@ def test_gnlse_spectrum_keeps_every_bin(nlm, n, rows):
     x = _wide_spectrum(n, rows)
     out = med.batchSignalSimulation(x)
     assert np.max(np.abs(np.abs(out) / np.abs(x) - 1)) < 3.2e-14
+
+
+# ---- fields that a butterfly gathers in one point -----------------------------------------------------------------
+
+@pytest.mark.parametrize("in_time", [False, True])
+@pytest.mark.parametrize("n", [70, 80, 84, 98, 112, 140, 280, 294, 320, 336, 392, 448, 1120, 1280, 1344, 2058, 2240, 3920])
+def test_single_bins_on_general_grids(nlm, oracle, n, in_time):
+    """Plane waves (and single bins), whose transform is one point that sums all others, with norms just below powers of
+    two and a mode of the other kind beside them: grids whose last odd pass runs at the highest norm, and others.
+    Tolerance as in test_gpu_fx.py (20 steps)."""
+    kw = dict(SFG, tPrecision=n)
+    med, ref = nlm.Chi2SFG(**kw), oracle.Chi2SFG(**kw)
+    med.runPumpSimulation()
+    ref.run_pump_simulation()
+    bins = sorted({0, 1, 2, 3, 5, 7, n // 7, n // 5, n // 4, n // 2, n - 1})
+    t = np.arange(n)
+    x = np.zeros((3 * len(bins), 2, n), complex)
+    for i, k in enumerate(bins):
+        for q, norm in enumerate((0.999, 0.71, 1.99)):
+            x[3 * i + q, 0] = norm * np.exp(2j * np.pi * k * t / n) / np.sqrt(n)
+            x[3 * i + q, 1, k] = norm
+    x = x.reshape(len(x), -1)
+    want = ref.batch_signal_simulation(x, in_time, False)
+    for use in (0, 1):
+        med._set_schedule(use_propagator=use)
+        out = med.batchSignalSimulation(x, in_time, False)
+        for k in range(len(x)):
+            assert cases.rel_l2(out[k], want[k]) < 1e-12
+
+
+@pytest.mark.parametrize("n", [70, 80, 294, 448])
+def test_greens_functions_of_small_general_grids(nlm, oracle, n):
+    """Impulses in every bin."""
+    kw = dict(PDC, tPrecision=n)
+    c, s = nlm.Chi2PDC(**kw).computeGreensFunction()
+    cr, sr = oracle.Chi2PDC(**kw).compute_greens_function()
+    assert cases.rel_l2_pair(c, s, cr, sr) < 1e-12
