@@ -198,7 +198,7 @@ inline void add_prop_key(GraphKey& k, const PropArgs& a) {
   k.add(a.out).add(a.outStride).add(a.tw).add(a.dstep).add(a.dlast).add(a.half).add(a.back).add(a.prop);
   k.add(a.pump).add(a.pumpStride).add(a.nPumps).add(a.coef).add(a.nCoef).add(a.gridF).add(a.gridT);
   k.add(a.ckpt).add(a.ckK).add(a.ckN).add(a.stages).add(a.raman).add(a.steep).add(a.relInt);
-  k.add(a.fx.tw).add(a.fx.L).add(a.fx.chirp).add(a.fx.conv).add(a.fx.lsL).add(a.fx.root).add(a.fx.twN).add(a.fx.tab).add(a.fx.et).add(a.fx.raman).add(a.fx.steep).add(a.fx.etRaman).add(a.fx.etSteep).add(a.fx.A0).add(a.fx.sh).add(a.fx.ls);
+  k.add(a.fx.tw).add(a.fx.L).add(a.fx.chirp).add(a.fx.conv).add(a.fx.root).add(a.fx.twN).add(a.fx.tab).add(a.fx.et).add(a.fx.raman).add(a.fx.steep).add(a.fx.etRaman).add(a.fx.etSteep).add(a.fx.A0).add(a.fx.sh).add(a.fx.ls);
 }
 
 struct GraphCache {
@@ -1875,15 +1875,15 @@ struct Medium {
         level += fx_log2(r) - 2 * s;
       }
     }
-    f.A0 = 60;
+    f.A0 = kFxA0;
     f.ls = 2 - (level >= 0 ? (level + 1) / 2 : -((-level) / 2));   // 2 - ceil(level / 2)
     if (!is_pow2(p.N) && fxConvSize()) {
-      // a transform: two of L points, the product with conv and the closing chirp, both shifted back to 2^A0
+      // a transform: two of L points and the product with conv; what it is raised by in between it returns itself, and
+      // the table product leaves it where it stands (fx_fft raises it again before the inverse)
       f.L = (int)fxConvL();
       f.chirp = fxChirp;
       f.conv = fxConv;
-      f.lsL = f.ls;
-      f.sh = 2 * f.sh + 2 * (2 - f.lsL) + fxConvEt;
+      f.sh = 2 * f.sh + fxConvEt;
       f.ls = 2;
     }
     return f;

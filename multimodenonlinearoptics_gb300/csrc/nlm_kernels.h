@@ -32,7 +32,6 @@ struct FxArgs {
   int L;
   const int4* chirp;
   const int4* conv;
-  int lsL;           // places the product with conv, and the chirp after it, are shifted left
   const int4* root;  // exp(-2 pi i q / r) of the odd radices (fx_root_at)
   const int4* twN;   // exp(-2 pi i m / N), m < N (cluster kernels with one point per thread)
   const int4* tab;   // [dispStep, last, half][mode][N], each with its 1/N
@@ -50,6 +49,7 @@ struct FxArgs {
 // half bits above its entry: the fewest that keep it within kFxPeak half bits after the pass (each pass grows the
 // norm by sqrt(r)).  The higher the norm stands, the less a rounding weighs.  Updates level.
 constexpr int kFxPeak = 4;
+constexpr int kFxA0 = 60;   // log2 bound of the 2-norm on entry
 __host__ __device__ constexpr int fx_log2(int r) { return r >= 16 ? 4 : r >= 8 ? 3 : r >= 4 ? 2 : r >= 2 ? 1 : 0; }
 __host__ __device__ constexpr int fx_pass_shift(int level, int r) {
   return level + fx_log2(r) <= kFxPeak ? 0 : (level + fx_log2(r) - kFxPeak + 1) / 2;

@@ -20,7 +20,6 @@ __device__ __forceinline__ void fx_begin(FxField<NT>& f, const FxArgs& fx, const
   f.grid = plan.N;
   f.chirp = fx.chirp;
   f.conv = fx.conv;
-  f.lsL = fx.lsL;
   f.t = plan.T;
   f.j = threadIdx.x;
   f.sel = 0;
@@ -55,8 +54,7 @@ __device__ __forceinline__ void fx_pair(FxField<NT>& f, const FxArgs& fx, double
 #pragma unroll 1
   for (int dir = 0; dir < 2; dir++) {
     if (dir == 0 ? fwd : inv) {
-      fx_fft(f, y);
-      k += fx.sh;
+      k += fx.sh - fx_fft(f, y, dir == 0 || !fwd);
     }
     if (dir == 0 && fwd) {
       k += et + 2 - fx.ls;

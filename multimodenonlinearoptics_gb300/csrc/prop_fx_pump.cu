@@ -67,7 +67,7 @@ __global__ void __launch_bounds__(512) k_fx_rows(const double2* __restrict__ in,
     fxc y[R];
 #pragma unroll
     for (int v = 0; v < R; v++) x[v] = f.has(j + v * T) ? in[row * N + j + v * T] : czero();
-    int lift;
+    int lift, up = 0;
     const int a = fx_enter(f, x, y, fx.A0, &lift);
 #pragma unroll 1
     for (int d = 0; d < 2; d++) {   // swapped components around the forward transform: the inverse one
@@ -75,9 +75,9 @@ __global__ void __launch_bounds__(512) k_fx_rows(const double2* __restrict__ in,
 #pragma unroll
         for (int v = 0; v < R; v++) y[v] = fxc{y[v].y, y[v].x};
       }
-      if (d == 0) fx_fft(f, y);
+      if (d == 0) up = fx_fft(f, y, true);
     }
-    fx_leave<R>(y, x, a - 1023 - fx.A0 - lift + fx.sh, a > 2200);
+    fx_leave<R>(y, x, a - 1023 - fx.A0 - lift + fx.sh - up, a > 2200);
 #pragma unroll
     for (int v = 0; v < R; v++)
       if (f.has(j + v * T)) out[row * N + j + v * T] = cscale(x[v], scale);
