@@ -1862,21 +1862,15 @@ struct Medium {
     f.etSteep = fxEtSteep;
     f.err = g_exchange.flag();
     f.root = fxRoots;
-    int level = 0;   // half bits
+    const int bit = p.gen ? 16 : 2;
+    int level = 0;   // 1 / bit of a bit
     for (int i = 0; i < p.nPass; i++) {
-      const int r = p.radix[i];
-      if (r & 1) {
-        const int s = fx_odd_shift(level);
-        f.sh += s + 2;
-        level += fx_half_bits(r) - 4 - 2 * s;
-      } else {
-        const int s = i == 0 ? 0 : fx_pass_shift(level, r);
-        f.sh += s;
-        level += fx_log2(r) - 2 * s;
-      }
+      const int r = p.radix[i], s = p.gen ? fx_gen_shift(level, r) : i == 0 ? 0 : fx_pass_shift(level, r);
+      f.sh += s;
+      level += (p.gen ? fx_gen_growth(r) : fx_log2(r)) - bit * s;
     }
     f.A0 = kFxA0;
-    f.ls = 2 - (level >= 0 ? (level + 1) / 2 : -((-level) / 2));   // 2 - ceil(level / 2)
+    f.ls = 2 - (level + bit - 1) / bit;
     if (!is_pow2(p.N) && fxConvSize()) {
       // a transform: two of L points and the product with conv; what it is raised by in between it returns itself, and
       // the table product leaves it where it stands (fx_fft raises it again before the inverse)

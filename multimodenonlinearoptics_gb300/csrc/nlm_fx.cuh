@@ -21,6 +21,8 @@
 // are static (fx_pass_shift): the norm of a field that enters below 2^60 peaks below 2^62 through the
 // passes.
 #pragma once
+#include <type_traits>
+
 #include "nlm_device.cuh"
 
 namespace nlm {
@@ -386,54 +388,41 @@ __device__ __forceinline__ double fx_to(long long v, int k) {
 // (b - k) r + k + s L), and the result comes back to the owners.  A thread takes the butterflies b = j + u T.
 constexpr int kFxGen = -1;
 
-// sum of c[q] a[q] (Q62 constants, q < n) / 4 + acc, rounded; the cross products are folded in pairs, whose sums
-// stay below 2^63
+// sum of c[q] a[q] (Q62 constants, q < n), rounded; the cross products are folded in pairs, whose sums stay below 2^63
 template <int n>
-__device__ __forceinline__ long long fx_dot(const int (&ah)[n], const int (&al)[n], const int2 (&c)[n], long long acc) {
+__device__ __forceinline__ long long fx_dot(const int (&ah)[n], const int (&al)[n], const int2 (&c)[n]) {
+  long long acc = 0;
+  std::conditional_t<(n > 2), unsigned long long, unsigned> low = 0;   // carries only from the second pair on
 #pragma unroll
   for (int q = 0; q < n; q += 2) {
-    long long m = fx_mad(al[q], c[q].x, fx_mad(ah[q], c[q].y, 1LL << 31));
+    long long m = fx_mad(al[q], c[q].x, fx_mad(ah[q], c[q].y, q == 0 ? 1LL << 29 : 0));
     if (q + 1 < n) m = fx_mad(al[q + 1], c[q + 1].x, fx_mad(ah[q + 1], c[q + 1].y, m));
     acc += m >> 32;
+    low += (unsigned)m;
     acc = fx_mad(ah[q], c[q].x, acc);
     if (q + 1 < n) acc = fx_mad(ah[q + 1], c[q + 1].x, acc);
   }
-  return acc;
+  if constexpr (n > 2) acc += (long long)(low >> 32);
+  return (long long)((unsigned long long)acc << 2) | ((unsigned)low >> 30);
 }
 
-// The sum of v[0 .. n - 1] / 4, rounded to nearest, ties to even: the quarters and the remainders apart, since the sum
-// itself can pass 2^63 (sqrt(r) times a norm of 2^62, for a field that a butterfly gathers in one point).
-template <int n>
-__device__ __forceinline__ long long fx_quarter_sum(const long long (&v)[n]) {
-  long long q = 0;
-  int rem = 0;
-#pragma unroll
-  for (int k = 0; k < n; k++) {
-    q += v[k] >> 2;
-    rem += (int)v[k] & 3;
-  }
-  return q + ((rem + 1 + (((int)q + (rem >> 2)) & 1)) >> 2);
-}
-
-// r-point DFT / 4, r an odd prime.  With a_q = x_q + x_(r-q), b_q = x_q - x_(r-q), y_s and y_(r-s) are
-// x_0 + sum cos(2 pi q s / r) a_q -+ i sum sin(2 pi q s / r) b_q.  root: cos and -sin of 2 pi q / r in Q62 halves.
+// r-point DFT, r an odd prime, of values whose norm is at most 2^62 / sqrt(r).  With a_q = x_q + x_(r-q),
+// b_q = x_q - x_(r-q), y_s and y_(r-s) are x_0 + sum cos(2 pi q s / r) a_q -+ i sum sin(2 pi q s / r) b_q.  root: cos
+// and -sin of 2 pi q / r in Q62 halves.
 template <int r>
 __device__ __forceinline__ void fx_odd_dft(fxc (&x)[r], const int4* root) {
   constexpr int h = (r - 1) / 2;
   int axh[h], axl[h], ayh[h], ayl[h], bxh[h], bxl[h], byh[h], byl[h];
-  const fxc s0 = fx_shift(x[0], 2);
-  long long sx[h + 1] = {x[0].x}, sy[h + 1] = {x[0].y};
+  const fxc x0 = x[0];
 #pragma unroll
   for (int q = 1; q <= h; q++) {
     const fxc a = fxadd(x[q], x[r - q]), b = fxsub(x[q], x[r - q]);
-    sx[q] = a.x;
-    sy[q] = a.y;
+    x[0] = fxadd(x[0], a);
     fx_split(a.x, axh[q - 1], axl[q - 1]);
     fx_split(a.y, ayh[q - 1], ayl[q - 1]);
     fx_split(b.x, bxh[q - 1], bxl[q - 1]);
     fx_split(b.y, byh[q - 1], byl[q - 1]);
   }
-  x[0] = fxc{fx_quarter_sum(sx), fx_quarter_sum(sy)};
 #pragma unroll
   for (int s = 1; s <= h; s++) {
     int2 cs[h], sn[h];
@@ -443,8 +432,8 @@ __device__ __forceinline__ void fx_odd_dft(fxc (&x)[r], const int4* root) {
       cs[q - 1] = make_int2(w.x, w.y);
       sn[q - 1] = make_int2(w.z, w.w);   // -sin
     }
-    const long long cx = fx_dot<h>(axh, axl, cs, s0.x), cy = fx_dot<h>(ayh, ayl, cs, s0.y);
-    const long long dx = fx_dot<h>(bxh, bxl, sn, 0), dy = fx_dot<h>(byh, byl, sn, 0);   // -sum sin b
+    const long long cx = x0.x + fx_dot<h>(axh, axl, cs), cy = x0.y + fx_dot<h>(ayh, ayl, cs);
+    const long long dx = fx_dot<h>(bxh, bxl, sn), dy = fx_dot<h>(byh, byl, sn);   // -sum sin b
     x[s] = fxc{cx - dy, cy + dx};        // C + i D, D = -sum sin b
     x[r - s] = fxc{cx + dy, cy - dx};
   }
@@ -466,7 +455,7 @@ __device__ __forceinline__ void fx_gen_pass(const FxField<kFxGen>& f, const int4
         x[q] = fx_unpack(src[fx_at(b + q * nb)]);
         if (q > 0 && L > 1) x[q] = fx_cmul(x[q], tw[(q - 1) * L + k], 2 - S);
       }
-      if (L > 1) x[0] = S < 0 ? fxc{x[0].x << 1, x[0].y << 1} : fx_shift(x[0], S);
+      if (L > 1) x[0] = fx_shift(x[0], S);
       if constexpr (r == 2 || r == 4 || r == 8) {
         fxdft_r<r>(x, 0, 1);
       } else {
@@ -491,8 +480,7 @@ __device__ __forceinline__ int fx_fft(FxField<kFxGen>& f, fxc (&x)[R], bool) {
 #pragma unroll 1
   for (int p = 0; p < f.plan->nPass; p++) {
     const int r = f.plan->radix[p];
-    const bool odd = (r & 1) != 0;
-    const int S = L == 1 ? 0 : odd ? fx_odd_shift(level) : fx_pass_shift(level, r);
+    const int S = fx_gen_shift(level, r);
     __syncthreads();
     int4* d = f.buf + (f.sel ^ 1) * fx_buffer(f.n);
     switch (r) {
@@ -503,7 +491,7 @@ __device__ __forceinline__ int fx_fft(FxField<kFxGen>& f, fxc (&x)[R], bool) {
       case 7: fx_gen_pass<R, 7>(f, b, d, tw, L, S); break;
       default: fx_gen_pass<R, 8>(f, b, d, tw, L, S); break;
     }
-    level += odd ? fx_half_bits(r) - 4 - 2 * S : fx_log2(r) - 2 * S;
+    level += fx_gen_growth(r) - 16 * S;
     if (L > 1) tw += (r - 1) * L;
     L *= r;
     f.sel ^= 1;

@@ -54,11 +54,14 @@ __host__ __device__ constexpr int fx_log2(int r) { return r >= 16 ? 4 : r >= 8 ?
 __host__ __device__ constexpr int fx_pass_shift(int level, int r) {
   return level + fx_log2(r) <= kFxPeak ? 0 : (level + fx_log2(r) - kFxPeak + 1) / 2;
 }
-// Odd radices (grids that are not powers of two) shift two places in their butterfly, which works on products of
-// real constants, and the twiddles one place back (-1) where the norm leaves room.  fx_half_bits: the half bits a
-// pass adds at most, log2 r rounded up.
-__host__ __device__ constexpr int fx_half_bits(int r) { return r <= 4 ? 2 : 3; }
-__host__ __device__ constexpr int fx_odd_shift(int level) { return level + 2 <= kFxPeak ? -1 : 0; }
+// The same on the general plan, whose radices are not all powers of two, in sixteenths of a bit: a pass of radix r adds
+// log2(r) / 2 bits (rounded up), and the norm stays within 2 bits of its entry.  The first pass never shifts.
+__host__ __device__ constexpr int fx_gen_growth(int r) {
+  return r == 2 ? 8 : r == 3 ? 13 : r == 4 ? 16 : r == 5 ? 19 : r == 7 ? 23 : 24;
+}
+__host__ __device__ constexpr int fx_gen_shift(int level, int r) {
+  return level + fx_gen_growth(r) <= 32 ? 0 : (level + fx_gen_growth(r) - 32 + 15) / 16;
+}
 
 // Shared memory of a CTA of the block fixed-point kernels: the twiddles, two exchange buffers of
 // fx_buffer(N) values and one pair of words per warp (at most 16).

@@ -205,3 +205,16 @@ def test_convolution_form_rounds_like_fp64(nlm, n):
         med.runSignalSimulation(x, True)
         for row in (250, 999):
             assert cases.rel_l2(med.signalTime[row], x) < 2.3e-16 * row
+
+
+@pytest.mark.parametrize("n", [600, 1536, 2646, 3402, 3750, 4050])
+def test_mixed_radices_round_like_fp64(nlm, n):
+    """The same on grids of many odd factors.  A pair of FP64 transforms in up to seven passes rounds by 2.5e-16 of the
+    norm, the factor 1/N by up to 1.1e-16: 3.6e-16 a step."""
+    kw = dict(relativeLength=1, nlLength=1, beta2=0, beta2s=0, tMax=20, tPrecision=n, zPrecision=401)
+    med = nlm.Chi2PDC(customPump=np.zeros(n, complex), **kw)
+    med.runPumpSimulation()
+    x = cases.noise(np.random.default_rng(n), n, 1.0)
+    med.runSignalSimulation(x, True)
+    for row in (100, 399):
+        assert cases.rel_l2(med.signalTime[row], x) < 3.6e-16 * row
