@@ -63,6 +63,15 @@ __host__ __device__ constexpr int fx_gen_shift(int level, int r) {
   return level + fx_gen_growth(r) <= 32 ? 0 : (level + fx_gen_growth(r) - 32 + 15) / 16;
 }
 
+// v / 2^r (0 <= r <= 62) rounded to nearest, ties to even.  r is mostly 1 to 3, where every 2^r-th value is a tie: ties
+// upwards would move the mean of every field by 2^-r / 2 in every forward transform.  (From r = 32 on, where ties are
+// one value in 2^32, the bit that breaks them is another one.)
+__host__ __device__ inline long long fx_align(long long v, int r) {
+  const int one = r > 0;
+  const int odd = (int)((unsigned)v >> (r < 31 ? r : 31)) & one;
+  return (v + (((1LL << r) >> 1) - one) + odd) >> r;
+}
+
 // Shared memory of a CTA of the block fixed-point kernels: the twiddles, two exchange buffers of
 // fx_buffer(N) values and one pair of words per warp (at most 16).
 __host__ __device__ constexpr int fx_buffer(int N) { return N + N / 8; }

@@ -189,11 +189,7 @@ __device__ __forceinline__ double2 spread_leave(fxc y, int h, int places) {
   return x;
 }
 
-// v >> r, rounded
-__device__ __forceinline__ fxc spread_align(fxc v, int r) {
-  const long long half = (1LL << r) >> 1;
-  return fxc{(v.x + half) >> r, (v.y + half) >> r};
-}
+__device__ __forceinline__ fxc spread_align(fxc v, int r) { return fxc{fx_align(v.x, r), fx_align(v.y, r)}; }
 
 // Output r of the P-point DFT of v: sum_c W_P^(r c) v_c.  r is the same for the whole warp.
 template <int P>
