@@ -1025,14 +1025,17 @@ struct Medium {
     ck(cudaMemsetAsync(d.p + h.size(), 0, kTablePad * sizeof(double2), stream), "upload");
   }
   // A table for the block fixed-point transforms, relative to the smallest power of two (*et) that no modulus
-  // exceeds by more than its rounding; left empty when a value is not finite (or all are zero).
+  // exceeds by more than its rounding; left empty when a value is not finite, or when the squares of all that are not
+  // zero underflow.
   void uploadFx(DevBuf<int4>& d, int* et, const std::vector<double2>& h) {
     double big = 0;
+    bool zero = true;   // a medium without self-steepening or nonlinearity has a table of zeros
     for (const double2& v : h) {
       if (!std::isfinite(v.x) || !std::isfinite(v.y)) return;
       big = std::max(big, v.x * v.x + v.y * v.y);
+      zero = zero && v.x == 0 && v.y == 0;
     }
-    if (!(big > 0) || !std::isfinite(big)) return;
+    if ((!(big > 0) && !zero) || !std::isfinite(big)) return;
     std::frexp(std::sqrt(big) * (1 - 1e-15), et);
     std::vector<int4> q;
     q.reserve(h.size() + kTablePad);

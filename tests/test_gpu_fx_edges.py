@@ -218,3 +218,19 @@ def test_mixed_radices_round_like_fp64(nlm, n):
     med.runSignalSimulation(x, True)
     for row in (100, 399):
         assert cases.rel_l2(med.signalTime[row], x) < 3.6e-16 * row
+
+
+# ---- tables of zeros ----------------------------------------------------------------------------------------------
+
+@pytest.mark.parametrize("n", [128, 512, 600, 2048])
+def test_gnlse_without_nonlinearity(nlm, oracle, n):
+    """Infinite nonlinear and self-steepening lengths: a steepening table of zeros is a table, and few rows keep their
+    one-point-per-thread clusters.  40 steps: tolerance as in test_gpu_fx.py."""
+    kw = dict(GNLSE, nlLength=cases.INF, selfSteepLength=cases.INF, relativeLength=1, tMax=10, tPrecision=n,
+              zPrecision=40)
+    med, ref = nlm.Chi3GNLSE(**kw), oracle.Chi3GNLSE(**kw)
+    x = cases.noise(np.random.default_rng(n), 3 * n, 1.0).reshape(3, n)
+    out = med.batchSignalSimulation(x)
+    if n in (512, 2048):
+        assert med._last_schedule()["R"] == 1
+    assert cases.rel_l2(out, ref.batch_signal_simulation(x, False)) < 1e-12
