@@ -287,6 +287,11 @@ nlm_status nlm_last_schedule(const nlm_medium* m, int* values);
  * each medium's form among those its mode allows (1: one, four, eight or sixteen CTAs; 3: one, four
  * or eight).  Other values: NLM_ERR_VALUE.  No counterpart in the reference. */
 nlm_status nlm_set_cluster(nlm_medium* m, int enable);
+/* Polls after which a cluster kernel of this handle stops waiting for an exchange between its CTAs
+ * (negative: the default, 65536).  The kernel then runs to its end without the exchange, and the call
+ * returns NLM_ERR_RUNTIME with results that are not valid; the handle stays usable.  0 gives up at
+ * once: the failure path without a failure.  No counterpart in the reference. */
+nlm_status nlm_set_exchange_limit(nlm_medium* m, int polls);
 /* Arithmetic of the single-mode precomputed-propagator kernel (Chi3, Chi2PDC Green's functions
  * and batches on power-of-two grids up to 4096 points): 0 = FP64 (default), 1 = double-float
  * (pairs of FP32 values, ~48-bit significand, on the FP32 units).  Other paths stay FP64, among

@@ -18,7 +18,7 @@ __global__ void __launch_bounds__(C == 16 ? 256 : kMaxThreads) k_adjoint_gnlse_s
   SpreadFFT f;
   const int rank = (int)cl.block_rank();
   const int M = a.plan.N;
-  spread_init<C>(f, smem, a.fx.twN, M, rank, a.fx.err);
+  spread_init<C>(f, smem, a.fx.twN, M, rank, a.fx.wait);
   cl.sync();
   const int N = M * C;
   const int tn = rank + C * f.t, fk = f.j + M * rank;
@@ -61,6 +61,7 @@ __global__ void __launch_bounds__(C == 16 ? 256 : kMaxThreads) k_adjoint_gnlse_s
     d.gin[inst * (long long)N + fk] = cmulc(g, __ldg(a.half + fk));
   }
   cl.sync();
+  spread_drain(f);
 }
 
 void add_kernels_adjoint_gnlse_spread(std::vector<KernelEntry>& t) {

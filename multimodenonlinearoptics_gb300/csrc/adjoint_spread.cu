@@ -27,7 +27,7 @@ __global__ void __launch_bounds__(kMaxThreads) k_adjoint_pdc_spread(const PropAr
   SpreadFFT f;
   const int rank = (int)cl.block_rank();
   const int M = a.plan.N;
-  spread_init(f, smem, a.fx.twN, M, rank, a.fx.err);
+  spread_init(f, smem, a.fx.twN, M, rank, a.fx.wait);
   cl.sync();
   const int N = M * kSpreadC;
   const int tn = rank + kSpreadC * f.t, fk = f.j + M * rank;
@@ -70,6 +70,7 @@ __global__ void __launch_bounds__(kMaxThreads) k_adjoint_pdc_spread(const PropAr
     d.gin[inst * (long long)N + fk] = cmulc(g, __ldg(a.half + fk));
   }
   cl.sync();
+  spread_drain(f);
 }
 
 // Pipelined form for checkpoint intervals K > 1 on clusters of eight CTAs (two groups of four, as in
@@ -84,7 +85,7 @@ __global__ void __launch_bounds__(kMaxThreads) k_adjoint_pdc_spread_pipe(const P
   const int role = crank / kSpreadC;   // 0: reverse sweep, 1: recomputation
   SpreadFFT f;
   const int M = a.plan.N;
-  spread_init(f, smem, a.fx.twN, M, crank - role * kSpreadC, a.fx.err);
+  spread_init(f, smem, a.fx.twN, M, crank - role * kSpreadC, a.fx.wait);
   f.base = role * kSpreadC;
   cl.sync();
   const int N = M * kSpreadC;
@@ -138,6 +139,7 @@ __global__ void __launch_bounds__(kMaxThreads) k_adjoint_pdc_spread_pipe(const P
     }
   }
   cl.sync();
+  spread_drain(f);
 }
 
 // Stage-factor gradient groups beside the pipelined sweep, on clusters of 4 (2 + G) CTAs, for
@@ -167,7 +169,7 @@ __global__ void __launch_bounds__(kMaxThreads) k_adjoint_pdc_spread_stage(const 
   const int N = M * kSpreadC;
   SpreadFFT f;
   if (role < 2) {
-    spread_init(f, smem, a.fx.twN, M, lr, a.fx.err);
+    spread_init(f, smem, a.fx.twN, M, lr, a.fx.wait);
     f.base = role * kSpreadC;
   }
   cl.sync();
@@ -263,6 +265,7 @@ __global__ void __launch_bounds__(kMaxThreads) k_adjoint_pdc_spread_stage(const 
     }
     cl.sync();
   }
+  if (role < 2) spread_drain(f);
 }
 
 void add_kernels_adjoint_spread(std::vector<KernelEntry>& t) {

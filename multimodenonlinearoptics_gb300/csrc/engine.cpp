@@ -679,6 +679,14 @@ nlm_status nlm_set_cluster(nlm_medium* h, int enable) {
   });
 }
 
+nlm_status nlm_set_exchange_limit(nlm_medium* h, int polls) {
+  return guarded([&] {
+    Medium* m = M(h);
+    m->exchangePolls = polls < 0 ? nlm::kExchangePolls : polls;
+    for (Medium* c : m->media) c->exchangePolls = m->exchangePolls;
+  });
+}
+
 nlm_status nlm_set_precision(nlm_medium* h, int precision) {
   return guarded([&] {
     if (precision != 0 && precision != 1) throw std::invalid_argument("precision must be 0 (FP64) or 1 (double-float)");

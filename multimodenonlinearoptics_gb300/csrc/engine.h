@@ -198,7 +198,7 @@ inline void add_prop_key(GraphKey& k, const PropArgs& a) {
   k.add(a.out).add(a.outStride).add(a.tw).add(a.dstep).add(a.dlast).add(a.half).add(a.back).add(a.prop);
   k.add(a.pump).add(a.pumpStride).add(a.nPumps).add(a.coef).add(a.nCoef).add(a.gridF).add(a.gridT);
   k.add(a.ckpt).add(a.ckK).add(a.ckN).add(a.stages).add(a.raman).add(a.steep).add(a.relInt);
-  k.add(a.fx.tw).add(a.fx.L).add(a.fx.chirp).add(a.fx.conv).add(a.fx.root).add(a.fx.twN).add(a.fx.tab).add(a.fx.et).add(a.fx.raman).add(a.fx.steep).add(a.fx.etRaman).add(a.fx.etSteep).add(a.fx.A0).add(a.fx.sh).add(a.fx.ls);
+  k.add(a.fx.tw).add(a.fx.L).add(a.fx.chirp).add(a.fx.conv).add(a.fx.root).add(a.fx.twN).add(a.fx.tab).add(a.fx.et).add(a.fx.raman).add(a.fx.steep).add(a.fx.etRaman).add(a.fx.etSteep).add(a.fx.A0).add(a.fx.sh).add(a.fx.ls).add(a.fx.wait.err).add(a.fx.wait.polls);
 }
 
 struct GraphCache {
@@ -845,6 +845,10 @@ struct Medium {
     if (ownStream && stream) cudaStreamDestroy(stream);
   }
 
+  // How this medium's cluster kernels wait for their exchanges (nlm_set_exchange_limit).
+  int exchangePolls = kExchangePolls;
+  ExchangeWait exchangeWait() const { return ExchangeWait{g_exchange.flag(), exchangePolls}; }
+
   // Waits for the medium's stream.
   void sync(const char* what) {
     ck(cudaStreamSynchronize(stream), what);
@@ -1442,7 +1446,7 @@ struct Medium {
     upload(dr, rel);
     if (spreadGrid() || wideGrid()) {
       // the march on four (up to 1024 points) or eight SMs with one point per thread (prop_spread.cu)
-      ck(launch_pump_chi3_spread(pumpFreq.p, pumpTime.p, de.p, dh.p, dd.p, db.p, dr.p, (int)nZP, (int)N, spreadTw(), g_exchange.flag(), stream),
+      ck(launch_pump_chi3_spread(pumpFreq.p, pumpTime.p, de.p, dh.p, dd.p, db.p, dr.p, (int)nZP, (int)N, spreadTw(), exchangeWait(), stream),
          "chi3 pump (spread)");
     } else if (useCluster && is_pow2((int)N) && N >= 1024) {
       // 1024..8192 points: the march on four SMs (prop_cluster_pump.cu), four points per thread
@@ -1494,15 +1498,15 @@ struct Medium {
   }
 
   // Runs a deferred pump march alone (four CTAs, k_pump_chi3_spread) and waits for it.  The march stays
-  // deferred if its launch fails, so the next reader tries again rather than reading stale grids.
+  // deferred if it fails, so the next reader tries again rather than reading stale grids.
   void flushPump() {
     if (!deferredPump.pending) return;
     const PumpMarchArgs p = deferredPumpArgs();
-    ck(launch_pump_chi3_spread(p.pf, p.pt, p.env, p.halfP, p.dstepP, p.backP, p.rel, p.nRows, (int)N, spreadTw(), g_exchange.flag(), stream),
+    ck(launch_pump_chi3_spread(p.pf, p.pt, p.env, p.halfP, p.dstepP, p.backP, p.rel, p.nRows, (int)N, spreadTw(), exchangeWait(), stream),
        "chi3 pump (spread)");
-    deferredPump.pending = false;
     launches++;
     sync("chi3 pump");
+    deferredPump.pending = false;
   }
 
   // src/_NonlinearMedium.cpp:506-534
@@ -1798,7 +1802,7 @@ struct Medium {
     a.fx.steep = fxSteep.p;
     a.fx.etRaman = fxEtRaman;
     a.fx.etSteep = fxEtSteep;
-    a.fx.err = g_exchange.flag();
+    a.fx.wait = exchangeWait();
     a.dstep = dstep.p;
     a.dlast = dlast.p;
     a.half = half.p;
@@ -1863,7 +1867,7 @@ struct Medium {
     f.steep = fxSteep.p;
     f.etRaman = fxEtRaman;
     f.etSteep = fxEtSteep;
-    f.err = g_exchange.flag();
+    f.wait = exchangeWait();
     f.root = fxRoots;
     const int bit = p.gen ? 16 : 2;
     int level = 0;   // 1 / bit of a bit
@@ -2471,6 +2475,7 @@ struct Medium {
     checkGrid(R);
     const size_t steps = nZ - 1;
     adjStored = false;
+    adjRows = 0;   // nothing to differentiate until this forward has succeeded
     if (interval <= 0 && storeStages(rows)) {
       // Chi3GNLSE with few rows on a cluster grid: the forward on 4-CTA clusters stores the stage values
       // of every step, and the reverse sweep reads them (nothing recomputed)
@@ -2987,6 +2992,7 @@ struct Medium {
     if (pipe) launchPumpSignal(a);
     else propagate(a, 1, true);
     sync("signal simulation");
+    if (pipe) deferredPump.pending = false;   // only now: a march that failed stays deferred
     signalVersion++;
   }
 
@@ -3011,7 +3017,6 @@ struct Medium {
       ck(cudaEventRecord(ev0, stream), "event");
     }
     ck(launch_chi3_pump_signal_spread(a, p, stream, &lastRegs), "chi3 pump + signal (cluster of eight)");
-    deferredPump.pending = false;   // only once launched: a failed launch leaves the march deferred
     launches++;
     if (timeKernels) {
       ck(cudaEventRecord(ev1, stream), "event");

@@ -23,6 +23,13 @@ struct FFTPlanH {
   int R;   // points per thread the plan was made for
 };
 
+// How a cluster kernel waits for an exchange between its CTAs (nlm_spread.cuh).
+constexpr int kExchangePolls = 1 << 16;
+struct ExchangeWait {
+  int* err;    // host memory, raised when an exchange does not arrive
+  int polls;   // polls before a wait gives up
+};
+
 // Block fixed-point transforms (nlm_fx.cuh): the twiddles and dispersion tables as Q62 integers, each complex
 // value as balanced 32-bit halves {re high, re low, im high, im low} with value (h 2^32 + l) 2^(et - 62).
 struct FxArgs {
@@ -41,7 +48,7 @@ struct FxArgs {
   int etRaman, etSteep;
   int A0;            // log2 bound of the field's 2-norm on entry
   int sh;            // places a transform shifts right in all
-  int* err;          // host memory: raised when an exchange between the CTAs of a cluster does not arrive
+  ExchangeWait wait; // cluster kernels
   int ls;            // places the table product after a forward transform is shifted left
 };
 
@@ -219,7 +226,7 @@ constexpr int kSpreadW16Key = 900;
 // two from 32 to 1024.
 cudaError_t launch_pump_chi3_spread(double2* pumpFreq, double2* pumpTime, const double2* env, const double2* halfP,
                                     const double2* dstepP, const double2* backP, const double2* rel, int nRows, int N,
-                                    const int4* tw, int* err, cudaStream_t s);
+                                    const int4* tw, ExchangeWait wait, cudaStream_t s);
 
 // The Chi3 pump march's grids and per-point tables (k_pump_chi3_spread's arguments).
 struct PumpMarchArgs {

@@ -30,7 +30,10 @@
 // of earlier global stores: with cluster barriers those were a third of a step.  Two mbarriers per warp and two
 // halves of the receive buffer serve the exchanges in turn: a thread writes half n again only after it has
 // received exchange n + 1 from the thread that reads that column, which pushed it after reading half n.
-// Waits give up after kSpreadWait polls and raise *err; every CTA then still runs to the closing cluster barrier.
+// Waits give up after wait.polls polls (kExchangePolls unless the caller limits them) and raise *wait.err.  The thread
+// then neither waits nor sends any more (an mbarrier whose phase is open takes no further arrival), so its peers give
+// up too, and every CTA runs to the closing cluster barrier.  After it spread_drain waits, again with a limit, for what
+// is still on its way into this CTA's memory.
 // Shared memory: M twiddles, two M-point exchange buffers (alternating: a thread writes a buffer only after
 // the barrier that every reader of that buffer's previous contents has passed), the two halves of C x M values.
 // M is a power of two of at least 32, N = C M at most 4096.
@@ -52,7 +55,6 @@ constexpr int kSpreadA0 = 59;      // log2 bound of a warp's 2-norm on entry
 constexpr int kSpreadPeak = 5;     // half bits the norm may stand above it
 constexpr int kSpreadZero = -(1 << 20), kSpreadBad = 1 << 20;   // codes of a zero warp, of one with Inf or NaN
 constexpr int kSpreadMaxCodes = 4096 / 32 * 4;                  // warps of a cluster times fields
-constexpr int kSpreadWait = 1 << 16;                            // polls of an exchange before it gives up
 
 struct SpreadFFT {
   const int4* twM;      // [M] exp(-2 pi i m / M) in Q62, shared memory
@@ -66,8 +68,8 @@ struct SpreadFFT {
   int ephase;           // the next of the two
   unsigned bar;         // shared address of this warp's two mbarriers
   unsigned parity;      // bits 0, 1: the phases that the warp's mbarriers complete next; 2, 3: the codes'
-  int* err;             // raised (host memory) when an exchange does not arrive
-  bool dead;            // an exchange has timed out: no more waiting
+  ExchangeWait wait;
+  int dead;             // not 0: the exchange of bit dead - 1 of parity has timed out; no more waiting, no more sending
   int M, rank, j;
   int l, g, t;          // lane, warp and local time index g + (M / 32) l of this thread
   int sel, phase;       // next exchange buffer / receive half
@@ -82,7 +84,7 @@ __device__ __forceinline__ unsigned spread_saddr(const void* p) { return (unsign
 // together (the _k forms), which sizes the exchange and receive buffers.
 template <int C = kSpreadC, int K = 1>
 __device__ __forceinline__ void spread_init(SpreadFFT& f, double2* smem, const int4* __restrict__ tw, int M, int rank,
-                                            int* err) {
+                                            ExchangeWait wait) {
   __shared__ int s_ecode[2 * kSpreadMaxCodes];
   __shared__ unsigned long long s_bar[2 * 16 + 2];
   f.M = M;
@@ -99,8 +101,8 @@ __device__ __forceinline__ void spread_init(SpreadFFT& f, double2* smem, const i
   f.bar = spread_saddr(s_bar + 2 * f.g);
   f.ebar = spread_saddr(s_bar + 2 * 16);
   f.parity = 0;
-  f.err = err;
-  f.dead = false;
+  f.wait = wait;
+  f.dead = 0;
   int4* twM = reinterpret_cast<int4*>(smem);
   f.buf = twM + M;
   f.recv = twM + (1 + 2 * K) * M;
@@ -121,22 +123,39 @@ __device__ __forceinline__ void spread_init(SpreadFFT& f, double2* smem, const i
   f.wgl = twM[f.g * f.l];
 }
 
-// Waits for the phase of an mbarrier that bit `bit` of f.parity names, and moves on to the next one.
-__device__ __forceinline__ void spread_wait(SpreadFFT& f, unsigned bar, int bit) {
-  const unsigned par = (f.parity >> bit) & 1;
-  f.parity ^= 1u << bit;
-  if (f.dead) return;
-  for (int n = 0; n < kSpreadWait; n++) {
+// Whether the mbarrier's phase `par` completes within `polls` polls.
+__device__ __forceinline__ bool spread_poll(unsigned bar, unsigned par, int polls) {
+  for (int n = 0; n < polls; n++) {
     unsigned ok;
     asm volatile(
         "{\n.reg .pred p;\nmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}"
         : "=r"(ok)
         : "r"(bar), "r"(par)
         : "memory");
-    if (ok) return;
+    if (ok) return true;
   }
-  f.dead = true;
-  if (f.err) *(volatile int*)f.err = 1;
+  return false;
+}
+
+// Waits for the phase of an mbarrier that bit `bit` of f.parity names, and moves on to the next one.
+__device__ __forceinline__ void spread_wait(SpreadFFT& f, unsigned bar, int bit) {
+  if (f.dead) return;
+  if (spread_poll(bar, (f.parity >> bit) & 1, f.wait.polls)) {
+    f.parity ^= 1u << bit;
+    return;
+  }
+  f.dead = 1 + bit;
+  if (f.wait.err) *(volatile int*)f.wait.err = 1;
+}
+
+// After the closing cluster barrier: all that the cluster sends has been sent.  A thread that has waited for every
+// exchange has received all of it; one that gave up waits for that exchange, and 64 us for any that a peer sent after
+// it, before its CTA's memory is given up.
+__device__ __forceinline__ void spread_drain(const SpreadFFT& f) {
+  if (!f.dead) return;
+  const int bit = f.dead - 1;
+  spread_poll(bit < 2 ? f.bar + 8 * bit : f.ebar + 8 * (bit - 2), (f.parity >> bit) & 1, kExchangePolls);
+  for (int n = 0; n < 64; n++) __nanosleep(1000);
 }
 
 // Local time index of thread j of a CTA of M threads (the time ownership above).
@@ -282,6 +301,7 @@ __device__ __forceinline__ void spread_cross(SpreadFFT& f, fxc (&x)[K]) {
 template <int C, int K>
 __device__ __forceinline__ void spread_push(SpreadFFT& f, const fxc (&y)[K]) {
   static_assert(C == 4 || C == 8 || C == 16, "four, eight or sixteen CTAs");
+  if (f.dead) return;
   const int M = f.M;
   const unsigned bar = f.bar + 8 * f.phase;
   const unsigned dst = spread_saddr(f.recv + ((long long)f.phase * C + f.rank) * K * M + f.j);
@@ -321,6 +341,7 @@ __device__ __forceinline__ fxc spread_mul(fxc a, int4 w, int s) { return fx_cmul
 // every warp of the cluster has read half n.
 template <int C, int K>
 __device__ __forceinline__ void spread_push_codes(SpreadFFT& f, const int (&h)[K]) {
+  if (f.dead) return;
   const int G = f.M >> 5;
   const unsigned bar = f.ebar + 8 * f.ephase;
   if (f.j == 0)

@@ -24,7 +24,7 @@ __global__ void __launch_bounds__(kMaxThreads) k_chi3_pump_signal_spread(const P
   const int role = crank / kSpreadC;   // 0: pump march, 1: signal
   SpreadFFT f;
   const int M = a.plan.N;
-  spread_init(f, smem, a.fx.twN, M, crank - role * kSpreadC, a.fx.err);
+  spread_init(f, smem, a.fx.twN, M, crank - role * kSpreadC, a.fx.wait);
   f.base = role * kSpreadC;
   const int N = M * kSpreadC;
   const int tn = f.rank + kSpreadC * f.t, fk = f.j + M * f.rank;
@@ -54,6 +54,7 @@ __global__ void __launch_bounds__(kMaxThreads) k_chi3_pump_signal_spread(const P
     p.pt[last + tn] = cscale(spread_inv_end(f, x), invN);
     cl.sync();
     cl.sync();
+    spread_drain(f);
     return;
   }
   const long long inst = a.instBase;
@@ -85,6 +86,7 @@ __global__ void __launch_bounds__(kMaxThreads) k_chi3_pump_signal_spread(const P
     }
   }
   cl.sync();
+  spread_drain(f);
 }
 
 cudaError_t launch_chi3_pump_signal_spread(const PropArgs& a, const PumpMarchArgs& p, cudaStream_t s, int* regs) {

@@ -22,7 +22,7 @@ __global__ void __launch_bounds__(C == 16 ? 256 : kMaxThreads) k_propagate_gnlse
   SpreadFFT f;
   const int rank = (int)cl.block_rank();
   const int M = a.plan.N;
-  spread_init<C>(f, smem, a.fx.twN, M, rank, a.fx.err);
+  spread_init<C>(f, smem, a.fx.twN, M, rank, a.fx.wait);
   cl.sync();
   const int N = M * C;
   const int tn = rank + C * f.t;   // time-domain point of this thread
@@ -97,6 +97,7 @@ __global__ void __launch_bounds__(C == 16 ? 256 : kMaxThreads) k_propagate_gnlse
     }
   }
   cl.sync();
+  spread_drain(f);
 }
 
 // kind kKindCluster, R = 1 (one point per thread): key Chi3GNLSE (four CTAs), + kSpreadWideKey (eight),

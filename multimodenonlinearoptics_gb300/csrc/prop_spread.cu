@@ -11,7 +11,7 @@ namespace nlm {
 
 cudaError_t launch_pump_chi3_spread(double2* pumpFreq, double2* pumpTime, const double2* env, const double2* halfP,
                                     const double2* dstepP, const double2* backP, const double2* rel, int nRows, int N,
-                                    const int4* tw, int* err, cudaStream_t s) {
+                                    const int4* tw, ExchangeWait wait, cudaStream_t s) {
   // four CTAs up to 1024 points, eight above (M = N / C threads per CTA)
   const int C = N <= 1024 ? 4 : 8;
   int M = N / C;
@@ -23,7 +23,7 @@ cudaError_t launch_pump_chi3_spread(double2* pumpFreq, double2* pumpTime, const 
   if (e != cudaSuccess) return e;
   if (smem == 0) return cudaErrorInvalidValue;
   void* args[] = {(void*)&pumpFreq, (void*)&pumpTime, (void*)&env, (void*)&halfP, (void*)&dstepP, (void*)&backP,
-                  (void*)&rel, (void*)&nRows, (void*)&M, (void*)&tw, (void*)&err};
+                  (void*)&rel, (void*)&nRows, (void*)&M, (void*)&tw, (void*)&wait};
   return launch_clustered(fn, C, M, smem, s, C, args);
 }
 

@@ -17,12 +17,12 @@ __global__ void __launch_bounds__(kMaxThreads) k_pump_chi3_spread(double2* __res
                                                                   const double2* __restrict__ dstepP,
                                                                   const double2* __restrict__ backP,
                                                                   const double2* __restrict__ rel, int nRows, int M,
-                                                                  const int4* __restrict__ tw, int* err) {
+                                                                  const int4* __restrict__ tw, ExchangeWait wait) {
   extern __shared__ double2 smem[];
   cg::cluster_group cl = cg::this_cluster();
   SpreadFFT f;
   const int rank = (int)cl.block_rank();
-  spread_init<C>(f, smem, tw, M, rank, err);
+  spread_init<C>(f, smem, tw, M, rank, wait);
   cl.sync();
   const int N = M * C;
   const int tn = rank + C * f.t;          // time-domain point of this thread
@@ -49,6 +49,7 @@ __global__ void __launch_bounds__(kMaxThreads) k_pump_chi3_spread(double2* __res
   pf[last + fk] = x;
   pt[last + tn] = cscale(spread_inv_end<C>(f, x), invN);
   cl.sync();
+  spread_drain(f);
 }
 
 // The modes one place on, the first one last.
@@ -109,7 +110,7 @@ __global__ void __launch_bounds__(kMaxThreads) k_propagate_spread(const PropArgs
   SpreadFFT f;
   const int rank = (int)cl.block_rank();
   const int M = a.plan.N;
-  spread_init<C, K>(f, smem, a.fx.twN, M, rank, a.fx.err);
+  spread_init<C, K>(f, smem, a.fx.twN, M, rank, a.fx.wait);
   cl.sync();
   const int N = M * C;
   const int tn = rank + C * f.t;
@@ -268,6 +269,7 @@ __global__ void __launch_bounds__(kMaxThreads) k_propagate_spread(const PropArgs
     }
   }
   cl.sync();
+  spread_drain(f);
 }
 
 }  // namespace nlm

@@ -76,6 +76,7 @@ def _load():
         "nlm_set_schedule": (i, [vp, i, i, i]),
         "nlm_set_precision": (i, [vp, i]),
         "nlm_set_cluster": (i, [vp, i]),
+        "nlm_set_exchange_limit": (i, [vp, i]),
         "nlm_graph_stats": (i, [vp, P(ctypes.c_long), P(ctypes.c_long)]),
         "nlm_last_schedule": (i, [vp, P(i)]),
         "nlm_last_launch_count": (i, [vp, P(ctypes.c_long)]),
@@ -397,6 +398,11 @@ class _NonlinearMedium:
         eight above) and with the two Chi3 marches one after the other; 2 four
         points per thread only (grids of 1024 points and more); 0 one CTA per propagation."""
         _check(_lib.nlm_set_cluster(self._h(), int(enable)))
+
+    def _set_exchange_limit(self, polls=-1):
+        """Polls after which a cluster kernel stops waiting for an exchange between its CTAs (negative: the
+        default); the call then raises RuntimeError."""
+        _check(_lib.nlm_set_exchange_limit(self._h(), int(polls)))
 
     def _set_precision(self, precision):
         """"f64" (default) or "ff": double-float arithmetic (FP32 pairs, ~48-bit significand) for the
