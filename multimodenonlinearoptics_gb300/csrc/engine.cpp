@@ -323,7 +323,7 @@ static void cascade_green(Medium* c, int inTime, int runPump, unsigned nThreads,
     Ct.alloc(ri * cc);
     St.alloc(ri * cc);
     nlm::ck(nlm::launch_cgemm_compose(Ci.p, Si.p, C.p, S.p, (int)ri, (int)ci, (int)cc, Ct.p, St.p, mi->stream), "compose");
-    nlm::ck(cudaStreamSynchronize(mi->stream), "compose");
+    mi->sync("compose");
     std::swap(C.p, Ct.p);
     std::swap(C.n, Ct.n);
     std::swap(S.p, St.p);
@@ -655,7 +655,7 @@ nlm_status nlm_set_stream(nlm_medium* h, void* cuda_stream) {
 nlm_status nlm_synchronize(nlm_medium* h) {
   return guarded([&] {
     Medium* m = M(h);
-    if (m->stream) nlm::ck(cudaStreamSynchronize(m->stream), "synchronize");
+    if (m->stream) m->sync("synchronize");
   });
 }
 

@@ -433,27 +433,37 @@ struct FxConvolutionCache {
 };
 inline FxConvolutionCache g_fxConvolutions;
 
-// Host memory that a cluster kernel raises when an exchange between its CTAs does not arrive in time (nlm_spread.cuh);
-// read after every wait for a stream.
-struct ExchangeFlag {
+// Words of host memory that cluster kernels raise when an exchange between their CTAs does not arrive in time
+// (nlm_spread.cuh).  Every medium takes one with its device tables and gives it back when it is destroyed, so that media
+// on different threads and streams each see their own; a page of words is kept for the process.
+struct ExchangeFlags {
+  static constexpr int kPage = 1024;
   std::mutex mu;
-  int* p = nullptr;
-  int* flag() {
+  std::vector<int*> idle;
+  size_t words = 0;
+  int* take() {
     std::lock_guard<std::mutex> lock(mu);
-    if (!p) {
-      ck(cudaHostAlloc((void**)&p, sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped), "exchange flag");
-      *p = 0;
+    if (idle.empty()) {
+      int* p = nullptr;
+      ck(cudaHostAlloc((void**)&p, kPage * sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped), "exchange flags");
+      idle.reserve(words += kPage);   // give() then never allocates
+      for (int k = kPage - 1; k >= 0; k--) idle.push_back(p + k);
     }
+    int* p = idle.back();
+    idle.pop_back();
+    *p = 0;
     return p;
   }
-  void check() {
-    if (p && *(volatile int*)p) {
-      *(volatile int*)p = 0;
-      throw std::runtime_error("an exchange between the CTAs of a cluster did not arrive; the results are not valid");
-    }
+  void give(int* p) {
+    std::lock_guard<std::mutex> lock(mu);
+    idle.push_back(p);
   }
 };
-inline ExchangeFlag g_exchange;
+// (never destroyed: media may outlive the library's static objects)
+inline ExchangeFlags& exchange_flags() {
+  static ExchangeFlags* flags = new ExchangeFlags;
+  return *flags;
+}
 
 inline bool is_pow2(int n) { return n > 0 && (n & (n - 1)) == 0; }
 
@@ -843,16 +853,28 @@ struct Medium {
     if (ev0) cudaEventDestroy(ev0);
     if (ev1) cudaEventDestroy(ev1);
     if (ownStream && stream) cudaStreamDestroy(stream);
+    if (exchangeFlag) exchange_flags().give(exchangeFlag);
   }
 
   // How this medium's cluster kernels wait for their exchanges (nlm_set_exchange_limit).
   int exchangePolls = kExchangePolls;
-  ExchangeWait exchangeWait() const { return ExchangeWait{g_exchange.flag(), exchangePolls}; }
+  int* exchangeFlag = nullptr;
+  ExchangeWait exchangeWait() const { return ExchangeWait{exchangeFlag, exchangePolls}; }
+  // Whether a launch of this medium has given up an exchange since the last time this was asked; asked after every wait
+  // for its launches, so that none is in flight.
+  bool exchangeFailed() {
+    if (!exchangeFlag || *(volatile int*)exchangeFlag == 0) return false;
+    *(volatile int*)exchangeFlag = 0;
+    return true;
+  }
+  [[noreturn]] static void throwExchange() {
+    throw std::runtime_error("an exchange between the CTAs of a cluster did not arrive; the results are not valid");
+  }
 
   // Waits for the medium's stream.
   void sync(const char* what) {
     ck(cudaStreamSynchronize(stream), what);
-    g_exchange.check();
+    if (exchangeFailed()) throwExchange();
   }
 
   // -- set-up, src/_NonlinearMedium.cpp:43-102 -------------------------------------------
@@ -962,6 +984,7 @@ struct Medium {
       ck(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking), "cudaStreamCreate");
       ownStream = true;
     }
+    if (!exchangeFlag) exchangeFlag = exchange_flags().take();
     tw = g_twiddles.get((int)N, stream);
     const size_t n = N;
     if (nPump > 0 && nZP > 0) {
@@ -1522,7 +1545,7 @@ struct Medium {
     if (modeIndex >= other.nSignal) throw std::invalid_argument("Mode index larger than number of modes in medium");
     ensureDevice();
     other.ensureDevice();
-    ck(cudaStreamSynchronize(other.stream), "other medium");
+    other.sync("other medium");
     const double ratio = static_cast<double>(other.nZ - 1) / (nZP - 1);
     double2* pf = pumpFreq.p + (size_t)idx * nZP * N;
     double2* pt = pumpTime.p + (size_t)idx * nZP * N;

@@ -569,7 +569,9 @@ nlm_status nlm_ragged_batch(nlm_medium* const* media, size_t n_media, const doub
     ck(cudaEventRecord(g_ragged.t1, origin), "ragged timing");
     g_ragged.lastKey = key.bytes;
     ck(cudaStreamSynchronize(origin), "ragged batch");
-    g_exchange.check();
+    bool failed = false;
+    for (size_t k : fused) failed = ms[k]->exchangeFailed() || failed;
+    if (failed) Medium::throwExchange();
     float gpuMs = 0;
     ck(cudaEventElapsedTime(&gpuMs, g_ragged.t0, g_ragged.t1), "ragged timing");
     // host-side state of what ran: the matrices built; one launch per propagation, build and ragged

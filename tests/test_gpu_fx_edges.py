@@ -374,3 +374,50 @@ def test_ragged_set_whose_exchange_gives_up(nlm):
     media[2]._set_exchange_limit()
     for a, b in zip(nlm.ragged_batch(media, xs), want):
         assert cases.rel_l2(a, b) < 1e-12   # a repeated call may run with its matrices (test_gpu_ragged.py)
+
+
+def test_each_medium_sees_its_own_failed_exchange(nlm):
+    """Media on threads of their own, one of which gives up its exchanges: it raises on every call, and the others never
+    do and keep their results bit by bit."""
+    import threading
+    media = [_signal(nlm, "Chi2PDC", n) for n in (512, 512, 128, 1024)]
+    want = [call() for _, call in media]
+    media[0][0]._set_exchange_limit(0)
+    raised, wrong = [0] * len(media), []
+    start = threading.Barrier(len(media))
+
+    def work(k):
+        start.wait()
+        for _ in range(100):
+            try:
+                if not np.array_equal(media[k][1](), want[k]):
+                    wrong.append(k)
+            except RuntimeError:
+                raised[k] += 1
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(len(media))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert raised == [100, 0, 0, 0] and not wrong
+    media[0][0]._set_exchange_limit()
+    assert np.array_equal(media[0][1](), want[0])
+
+
+def test_failed_exchange_of_a_ragged_set_stays_with_it(nlm):
+    """The flag of a set's medium is read and cleared by the set's call; a call of another medium after it succeeds, and
+    so does the medium's own next call."""
+    media = [_medium(nlm, "Chi2SFG", 512), _medium(nlm, "Chi2SFG", 512)]
+    other, call = _signal(nlm, "Chi2PDC", 512)
+    want = call()
+    x = cases.noise(np.random.default_rng(0), 512, 0.1)
+    for m in media:
+        m.runPumpSimulation()
+        m._set_exchange_limit(0)
+    with pytest.raises(RuntimeError, match="exchange"):
+        nlm.ragged_batch(media, [x, x])
+    assert np.array_equal(call(), want, equal_nan=True)
+    for m in media:
+        m._set_exchange_limit()
+        m.runSignalSimulation(x)
