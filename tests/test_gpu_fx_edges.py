@@ -421,3 +421,41 @@ def test_failed_exchange_of_a_ragged_set_stays_with_it(nlm):
     for m in media:
         m._set_exchange_limit()
         m.runSignalSimulation(x)
+
+
+# ---- four modes in one transform ----------------------------------------------------------------------------------
+
+@pytest.mark.parametrize("n", [128, 256, 512, 1024])
+@pytest.mark.parametrize("name", ["Chi2SFGII", "Chi2SHGOPA"])
+def test_four_modes_in_one_transform(nlm, oracle, name, n):
+    """Clusters that transform four modes together, two at a time (four CTAs, and eight for full grids of 1024 points),
+    with norms ten decades apart: every mode's field stays in its place and keeps its own exponent.  At most 111
+    steps of two evaluations that round by about 1e-15 of the norm a step, times a growth of a few: 1e-12, per mode at
+    the scale of the largest, which feeds the others."""
+    kw = dict(cases.CASES[name], tPrecision=n, tMax=20)
+    if name != "Chi2SFGII":   # whose keyword zPrecision binds to another slot (solvers/Chi2SFGII.cpp:98-106)
+        kw["zPrecision"] = 10
+    med, ref = getattr(nlm, name)(**kw), getattr(oracle, name)(**kw)
+    fnl = name in cases.FULLY_NONLINEAR
+    if not fnl:
+        med.runPumpSimulation()
+        ref.run_pump_simulation()
+    assert med._dims["nSignalModes"] == 4 and med._dims["nZSteps"] == ref.n_z_steps
+    x = cases.noise(np.random.default_rng(n), 8 * n, 0.3).reshape(2, 4, n)
+    x[0, 1] *= 1e-5
+    x[0, 3] *= 1e-10
+    x[1, :2] *= 1e-10
+    x = x.reshape(2, -1)
+    for in_time in (False, True):
+        args = (in_time,) if fnl else (in_time, False)
+        out = med.batchSignalSimulation(x, *args)
+        assert med._last_schedule()["R"] == 1 and med._last_schedule()["grid"] == 8
+        want = ref.batch_signal_simulation(x, *args)
+        for k in range(2):
+            assert cases.rel_l2(out[k], want[k]) < 1e-12
+        med.runSignalSimulation(x[0], in_time)
+        ref.run_signal_simulation(x[0], in_time)
+        assert med._last_schedule()["grid"] == (8 if n == 1024 else 4)
+        size = max(np.linalg.norm(f) for f in ref.signal_freq)
+        for m in range(4):
+            assert np.linalg.norm(med.signalFreqs(m) - ref.signal_freq[m]) < 1e-12 * size
