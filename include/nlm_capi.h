@@ -153,11 +153,13 @@ nlm_status nlm_batch_device(nlm_medium* m, const void* inputs_dev, size_t rows, 
  * batchSignalSimulation one row at a time, src/_NonlinearMedium.cpp:378-444).
  * inputs[k] is an N_k complex row for media[k]; outputs[k] receives the last row of all
  * signal modes (nSignalModes_k*N_k complex).  Pumps must have been run.  The call plans
- * each medium's form (one SM in a ragged launch, or a cluster of 4 or 8 SMs) for the
+ * each medium's form (one SM in a ragged launch, or a cluster of 4, 8 or 16 SMs) for the
  * shortest makespan and runs as one CUDA graph, replayed while the plan stays the same. */
 nlm_status nlm_ragged_batch(nlm_medium* const* media, size_t n_media, const double* const* inputs,
                             int in_time_domain, double* const* outputs);
-/* nlm_ragged_batch's makespan planner alone, with no device work: n_media media given by their grid
+/* The planning procedure of nlm_ragged_batch, with no device work, on a step-cost table of its own (that of the
+ * kernels with FP64 transforms; the call plans with the costs of the kernels it runs, so the two give other
+ * plans for the same media): n_media media given by their grid
  * (n_freqs), signal mode count, nZSteps, whether the RK4 propagator matrices are used (propagator),
  * ragged-launch class (media of one class share a launch: one solver and one grid) and available
  * forms (bit 0: one SM in a ragged launch, bits 1-3: clusters of 4, 8 and 16 SMs); the SMs that
@@ -166,8 +168,7 @@ nlm_status nlm_ragged_batch(nlm_medium* const* media, size_t n_media, const doub
  * makespan the plan was made for (microseconds; -1 when no plan fits the SMs at once, the slots then
  * queueing), per medium its form (0-3) and cluster slot (-1: a ragged launch; a slot's media run one
  * after another), the ragged launches' CTAs, and (times_us, n_media x 4) each medium's estimated
- * march time in each form (microseconds, -1 where the form is not available), from the engine's
- * GB300 per-step table.  No counterpart in the reference (scheduling support). */
+ * march time in each form (microseconds, -1 where the form is not available), from that table.  No counterpart in the reference (scheduling support). */
 nlm_status nlm_ragged_plan(size_t n_media, const unsigned* n_freqs, const unsigned* n_modes,
                            const unsigned* n_z_steps, const int* propagator, const int* launch_class,
                            const unsigned* forms, int cluster_sms, int w16_slots, int pool_sms,

@@ -178,7 +178,8 @@ def ragged_last_plan():
 
 def ragged_plan(n_freqs, n_modes, n_z_steps, propagator, launch_class, forms, cluster_sms=128, w16_slots=7,
                 pool_sms=152, pool_granularity=1):
-    """ragged_batch's makespan planner alone, with no device work (no counterpart in the reference).
+    """ragged_batch's planning procedure with no device work, on a step-cost table of its own: that of the kernels
+    with FP64 transforms (ragged_batch plans with the costs of the kernels it runs).  No counterpart in the reference.
 
     Per medium: its grid, signal mode count, nZSteps, whether its RK4 matrices are used, its
     ragged-launch class (one solver and one grid) and a mask of its available forms (bit 0 one SM,
