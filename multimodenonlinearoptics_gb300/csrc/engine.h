@@ -2299,8 +2299,8 @@ struct Medium {
         a.fx = fxArgs(a.plan);
       }
       // more rows than SMs (one row per thread group would take a second wave): two rows per thread
-      // group, sharing their Raman transforms (k_propagate_gnlse_pair: 14 transforms per row and step
-      // instead of 18, so a pair takes 1.56 rows' time)
+      // group, sharing their Raman transforms (12 transforms per row and step instead of 16 in k_fx_gnlse_pair and
+      // k_propagate_gnlse_pair; the rule is that of the FP64 kernels, whose pairs took 1.56 rows' time)
       if (!plainOne && nInst > smCount() && !a.gridF && !a.gridT) {
         if (const KernelEntry* kp = fx ? findKernel(kKindFxGnlse, fxKey + 400, a.R) : findKernel(kKindGnlse, solver + 400, R)) {
           k = kp;
@@ -2372,7 +2372,7 @@ struct Medium {
     if (!lastTuned) s = schedule(k, units, a.R, ctaPerSM < 0 ? 0 : ctaPerSM);
     // Paired rows run in waves of one pair per resident thread group.  When the last wave would leave
     // groups idle, the pairs fill whole waves and the rows left over run one per thread group in one
-    // more wave of the single-row kernel (a pair takes about 1.56 rows' time): 1024 rows of 4096
+    // more wave of the single-row kernel (with FP64 transforms a pair took about 1.56 rows' time): 1024 rows of 4096
     // points on 152 SMs take 3 pair waves and one single wave (5.7 row times) instead of 4 pair waves
     // (6.2).
     const KernelEntry* kTail = nullptr;
